@@ -24,6 +24,21 @@ __device__ __forceinline__ double rsqrt_f64(double s) {
     return fma(y * e, p, y);
 }
 
+// m s^(-3/2), the weight of a softened pair.  From the same seed y, t = y^2 and e = 1 - s t,
+// s^(-3/2) = y t (1 - e)^(-3/2) = y t (1 + 3e/2 + 15e^2/8 + O(e^3)), so the correction is
+// applied to the product m y t itself: 7 FP64 pipe operations after the seed, where refining
+// y first (5) and cubing it (3) took 8, and three roundings of the result instead of six.
+// The truncated term is about (35/16) e^3 < 2^-55.  s == 0 as in rsqrt_f64.
+__device__ __forceinline__ double inv_cube_f64(double s, double m) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
+    const double t = y * y;
+    const double e = fma(-s, t, 1.0);
+    const double p = fma(1.875, e, 1.5);
+    const double w = (m * y) * t;
+    return fma(w * e, p, w);
+}
+
 __device__ __forceinline__ float rsqrt_f32(float s) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
