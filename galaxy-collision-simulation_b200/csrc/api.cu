@@ -774,6 +774,7 @@ extern "C" int gx_diagnostics_compute(int64_t n, const double* x, const double* 
     GX_TRY(scratch.alloc(diagnostics_scratch_bytes(n) + 16 * sizeof(double), st));
     double* res = scratch.d();
     double* work = res + 16;
+    GX_CUDA(cudaMemsetAsync(work, 0, kDiagTicketBytes, st));
     GX_CUDA(launch_diagnostics(n, d[0], d[1], d[2], d[3], d[4], d[5], d[6], phys.G,
                                phys.softening * phys.softening, work, res, st));
     double h[13];
@@ -802,9 +803,9 @@ struct gx_session {
     double *x, *y, *z, *vx, *vy, *vz, *ax, *ay, *az, *m;
     double* part = nullptr;
     size_t part_cap = 0;
-    double* diag = nullptr;  // device: 16 result slots + diagnostics scratch
+    double* diag = nullptr;  // device: diagnostics scratch (ticket zeroed once, then by each launch)
     size_t diag_cap = 0;
-    double* host_diag = nullptr;  // pinned, 16 doubles
+    double* host_diag = nullptr;  // pinned, 16 doubles: written by the diagnostics kernel
     Choice cfg[3];
     std::map<std::tuple<int64_t, uint64_t, int, int, int>, cudaGraphExec_t> graphs;
     bool timing = false;
@@ -1040,12 +1041,13 @@ extern "C" int gx_session_create(int64_t n, gx_physics phys, int device, gx_sess
     s->buf = (double*)p;
     double** arr[10] = {&s->x, &s->y, &s->z, &s->vx, &s->vy, &s->vz, &s->ax, &s->ay, &s->az, &s->m};
     for (int k = 0; k < 10; ++k) *arr[k] = s->buf + (size_t)k * (size_t)n;
-    s->diag_cap = diagnostics_scratch_bytes(n) + 16 * sizeof(double);
+    s->diag_cap = diagnostics_scratch_bytes(n);
     e = dev_alloc(&p, s->diag_cap);
     if (e == cudaSuccess) s->diag = (double*)p;
     if (e == cudaSuccess) e = cudaMallocHost((void**)&s->host_diag, 16 * sizeof(double));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->buf, 0, (size_t)n * 10 * sizeof(double), s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->diag, 0, kDiagTicketBytes, s->stream);
     if (e != cudaSuccess) {
         const int r = fail_cuda(e, "gx_session_create");
         if (s->diag) cudaFree(s->diag);
@@ -1206,8 +1208,7 @@ extern "C" int gx_session_diagnostics(gx_session* s, gx_diagnostics* out) {
     if (!out) return fail(GX_ERR_INVALID_ARGUMENT, "gx_session_diagnostics: null");
     DeviceGuard g(s->device);
     GX_CUDA(launch_diagnostics(s->n, s->x, s->y, s->z, s->vx, s->vy, s->vz, s->m, s->phys.G,
-                               s->phys.softening * s->phys.softening, s->diag + 16, s->diag, s->stream));
-    GX_CUDA(cudaMemcpyAsync(s->host_diag, s->diag, 13 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+                               s->phys.softening * s->phys.softening, s->diag, s->host_diag, s->stream));
     GX_CUDA(cudaStreamSynchronize(s->stream));
     fill_diag(s->host_diag, out);
     return session_small_status(s);

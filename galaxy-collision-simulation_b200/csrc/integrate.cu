@@ -4,13 +4,15 @@
 // (v = v + a*dt, x = x + v*dt, no FMA contraction), so a device step reproduces the
 // reference's rounding given the same accelerations.
 //
-// Diagnostics follow cpp/core/diagnostics.cpp:7-37 in FP64: the O(N) moments are block
-// partial sums reduced in block order (deterministic); the potential energy
+// Diagnostics follow cpp/core/diagnostics.cpp:7-37 in FP64: the O(N) moments and the potential
 //     PE = -G sum_{i<j} m_i m_j / sqrt(|x_j - x_i|^2 + eps^2)
-// is evaluated as -G/2 sum_i m_i sum_{j != i} m_j / s_ij with the same tiling as the force
-// kernel (self pairs skipped by index, s == 0 pairs skipped as in the reference).
+// over every unordered pair once (s == 0 pairs skipped as in the reference), as block sums
+// added in a fixed order.
 #include "gx_device.cuh"
 #include "integrate.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace gx {
 namespace {
@@ -53,21 +55,53 @@ __global__ void kick_drift_kernel(int64_t n, double* x, double* y, double* z, do
     }
 }
 
-constexpr int kMomBlock = 256;
+// ---------------------------------------------------------------------------------------
+// Diagnostics in one launch.  Blocks [0, n_mom) add the 11 O(N) moments
+// [M, KE, Px, Py, Pz, Cx, Cy, Cz, Lx, Ly, Lz] (C = sum m x before the division by M); the
+// others the potential, every unordered pair once.  Bodies form tiles of BLOCK * IPT; tile row I
+// holds the tile pairs (I, J) with J >= I, and rows p and nt - 1 - p together always hold
+// nt + 1 tile pairs, so a work item is `run` consecutive tile pairs of one such double row and
+// all items cost the same.  The diagonal tile takes the pairs j > i only.  Every block leaves
+// its sums in `part`; the block that takes the last ticket adds them in a fixed order (so
+// results do not depend on scheduling) and writes the 13 values.  No block waits.
+//
+// Bound by the FP64 pipe: 12 operations per pair (3 subtractions, 3 FMA, 5 for the rsqrt, 1
+// FMA) over n^2 / 2 pairs.  N = 65,536: 1.69 ms a call (90% of the measured pipe rate) against
+// 5.37 ms for the sum over all ordered pairs with one target per thread; N = 1000: 52 us less
+// per call (136 blocks in place of 8, one launch and no copy in place of three and one).
+// ---------------------------------------------------------------------------------------
+struct DiagArgs {
+    int64_t n;
+    const double *x, *y, *z, *vx, *vy, *vz, *m;
+    double G, eps2;
+    int n_mom;        // moment blocks
+    int n_items;      // potential items (blocks)
+    int64_t tiles;    // nt
+    int chunks;       // items per double row
+    int64_t run;      // tile pairs per item
+    double* part;     // 11 * n_mom moment sums, then n_items potential sums
+    unsigned* ticket; // zero before the launch, zero after it
+    double* out;      // 13 values in diagnostics.csv order
+};
 
-// Block partial sums of the 11 O(N) moments:
-// [M, KE, Px, Py, Pz, Cx, Cy, Cz, Lx, Ly, Lz] (C = sum m x before the division by M).
-__global__ void __launch_bounds__(kMomBlock) moments_kernel(int64_t n, const double* x,
-                                                            const double* y, const double* z,
-                                                            const double* vx, const double* vy,
-                                                            const double* vz, const double* m,
-                                                            double* part) {
+template <int BLOCK>
+__device__ __forceinline__ double block_sum(double v, double* red) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    for (int w = 0; w < BLOCK / 32; ++w) s += red[w];
+    __syncthreads();
+    return s;
+}
+
+template <int BLOCK>
+__device__ void diag_moments(const DiagArgs& a, double* red) {
     double acc[11];
 #pragma unroll
     for (int c = 0; c < 11; ++c) acc[c] = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * kMomBlock + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * kMomBlock) {
-        const double mi = m[i], X = x[i], Y = y[i], Z = z[i], U = vx[i], V = vy[i], W = vz[i];
+    for (int64_t i = (int64_t)blockIdx.x * BLOCK + threadIdx.x; i < a.n; i += (int64_t)a.n_mom * BLOCK) {
+        const double mi = a.m[i], X = a.x[i], Y = a.y[i], Z = a.z[i], U = a.vx[i], V = a.vy[i], W = a.vz[i];
         acc[0] += mi;
         acc[1] += 0.5 * mi * (U * U + V * V + W * W);
         acc[2] += U * mi;
@@ -80,110 +114,140 @@ __global__ void __launch_bounds__(kMomBlock) moments_kernel(int64_t n, const dou
         acc[9] += (Z * U - X * W) * mi;
         acc[10] += (X * V - Y * U) * mi;
     }
-    __shared__ double red[11][kMomBlock / 32];
 #pragma unroll
     for (int c = 0; c < 11; ++c) {
-        const double v = warp_sum(acc[c]);
-        if ((threadIdx.x & 31) == 0) red[c][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 11) {
-        double s = 0.0;
-        for (int w = 0; w < kMomBlock / 32; ++w) s += red[threadIdx.x][w];
-        part[(size_t)blockIdx.x * 11 + threadIdx.x] = s;
+        const double s = block_sum<BLOCK>(acc[c], red);
+        if (threadIdx.x == 0) a.part[(size_t)c * a.n_mom + blockIdx.x] = s;
     }
 }
 
-// Potential: per target body i, pot_i = sum_{j != i} m_j / sqrt(s_ij); block partial of
-// m_i * pot_i.  FP64 with the refined rsqrt.
-template <int BLOCK, int JT, bool EPS0>
-__global__ void __launch_bounds__(BLOCK) potential_kernel(int64_t n, const double* x,
-                                                          const double* y, const double* z,
-                                                          const double* m, double eps2,
-                                                          double* part) {
-    __shared__ __align__(16) double sx[JT];
-    __shared__ __align__(16) double sy[JT];
-    __shared__ __align__(16) double sz[JT];
-    __shared__ __align__(16) double sm[JT];
+// Tile pairs (I, [j0, j1)) of one tile row: this thread's share of sum_i m_i sum_{j > i} m_j / s_ij.
+template <int BLOCK, int IPT, bool EPS0>
+__device__ __forceinline__ double diag_row(const DiagArgs& a, int64_t I, int64_t j0, int64_t j1, double2* sxy,
+                                           double2* szm) {
+    constexpr int T = BLOCK * IPT;
     const int tid = threadIdx.x;
-    const int64_t i = (int64_t)blockIdx.x * BLOCK + tid;
-    const bool ok = i < n;
-    const int64_t bi = ok ? i : 0;
-    const double xi = x[bi], yi = y[bi], zi = z[bi];
-    double pot = 0.0;
-    for (int64_t j0 = 0; j0 < n; j0 += JT) {
+    double xi[IPT], yi[IPT], zi[IPT], mi[IPT], pot[IPT];
 #pragma unroll
-        for (int r = 0; r < JT / BLOCK; ++r) {
+    for (int k = 0; k < IPT; ++k) {
+        const int64_t i = I * T + k * BLOCK + tid;
+        const bool in = i < a.n;
+        xi[k] = in ? a.x[i] : 0.0;
+        yi[k] = in ? a.y[i] : 0.0;
+        zi[k] = in ? a.z[i] : 0.0;
+        mi[k] = in ? a.m[i] : 0.0;
+        pot[k] = 0.0;
+    }
+    for (int64_t J = j0; J < j1; ++J) {
+#pragma unroll
+        for (int r = 0; r < IPT; ++r) {
             const int jj = r * BLOCK + tid;
-            const int64_t j = j0 + jj;
-            const bool in = j < n;
-            sx[jj] = in ? x[j] : 0.0;
-            sy[jj] = in ? y[j] : 0.0;
-            sz[jj] = in ? z[j] : 0.0;
-            sm[jj] = in ? m[j] : 0.0;
+            const int64_t j = J * T + jj;
+            const bool in = j < a.n;
+            sxy[jj] = in ? make_double2(a.x[j], a.y[j]) : make_double2(0.0, 0.0);
+            szm[jj] = in ? make_double2(a.z[j], a.m[j]) : make_double2(0.0, 0.0);
         }
         __syncthreads();
+        auto pairs = [&](auto diag) {
 #pragma unroll 4
-        for (int jj = 0; jj < JT; ++jj) {
-            const double dx = sx[jj] - xi, dy = sy[jj] - yi, dz = sz[jj] - zi;
-            double r = fma(dx, dx, eps2);
-            r = fma(dy, dy, r);
-            r = fma(dz, dz, r);
-            double w = sm[jj] * rsqrt_f64(r);
-            if (EPS0) w = (r == 0.0) ? 0.0 : w;
-            w = (j0 + jj == i) ? 0.0 : w;
-            pot += w;
-        }
+            for (int jj = 0; jj < T; ++jj) {
+                const double2 xy = sxy[jj], zm = szm[jj];
+#pragma unroll
+                for (int k = 0; k < IPT; ++k) {
+                    const double dx = xy.x - xi[k], dy = xy.y - yi[k], dz = zm.x - zi[k];
+                    double r = fma(dx, dx, a.eps2);
+                    r = fma(dy, dy, r);
+                    r = fma(dz, dz, r);
+                    double w = rsqrt_f64(r);
+                    if (EPS0) w = (r == 0.0) ? 0.0 : w;
+                    if (decltype(diag)::value) w = (jj > k * BLOCK + tid) ? w : 0.0;
+                    pot[k] = fma(zm.y, w, pot[k]);
+                }
+            }
+        };
+        if (J == I) pairs(std::true_type{});
+        else pairs(std::false_type{});
         __syncthreads();
     }
-    double v = ok ? m[i] * pot : 0.0;
+    double v = 0.0;
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) v = fma(mi[k], pot[k], v);
+    return v;
+}
+
+template <int BLOCK, int IPT, bool EPS0>
+__global__ void __launch_bounds__(BLOCK) diagnostics_kernel(const DiagArgs a) {
+    constexpr int T = BLOCK * IPT;
+    __shared__ __align__(16) double2 sxy[T];
+    __shared__ __align__(16) double2 szm[T];
     __shared__ double red[BLOCK / 32];
-    v = warp_sum(v);
-    if ((tid & 31) == 0) red[tid >> 5] = v;
-    __syncthreads();
-    if (tid == 0) {
-        double s = 0.0;
-        for (int w = 0; w < BLOCK / 32; ++w) s += red[w];
-        part[blockIdx.x] = s;
+    __shared__ unsigned s_last;
+    const int tid = threadIdx.x;
+    if ((int)blockIdx.x < a.n_mom) {
+        diag_moments<BLOCK>(a, red);
+    } else {
+        const int item = (int)blockIdx.x - a.n_mom;
+        const int64_t p = item / a.chunks, c0 = (item % a.chunks) * a.run;
+        const int64_t A = p, B = a.tiles - 1 - p, la = a.tiles - A;
+        const int64_t len = A == B ? la : a.tiles + 1, c1 = min(c0 + a.run, len);
+        double v = 0.0;
+        if (c0 < la) v += diag_row<BLOCK, IPT, EPS0>(a, A, A + c0, A + min(c1, la), sxy, szm);
+        if (c1 > la) v += diag_row<BLOCK, IPT, EPS0>(a, B, B + max(c0, la) - la, B + c1 - la, sxy, szm);
+        v = block_sum<BLOCK>(v, red);
+        if (tid == 0) a.part[(size_t)11 * a.n_mom + item] = v;
     }
+    __threadfence();  // this thread's partial sums before the ticket
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(a.ticket, 1u) == gridDim.x - 1u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double sums[12];
+#pragma unroll
+    for (int c = 0; c < 12; ++c) {
+        const double* q = a.part + (size_t)c * a.n_mom;
+        const int cnt = c < 11 ? a.n_mom : a.n_items;
+        double v = 0.0;
+#pragma unroll 8
+        for (int b = tid; b < cnt; b += BLOCK) v += __ldcg(q + b);
+        sums[c] = block_sum<BLOCK>(v, red);
+    }
+    if (tid != 0) return;
+    const double M = sums[0], pe = -a.G * sums[11];
+    double* out = a.out;
+    out[0] = M;
+    out[1] = sums[1];
+    out[2] = pe;
+    out[3] = sums[1] + pe;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        out[4 + c] = sums[2 + c];
+        out[7 + c] = M > 0.0 ? sums[5 + c] / M : sums[5 + c];
+        out[10 + c] = sums[8 + c];
+    }
+    __threadfence_system();  // out may be pinned host memory
+    *a.ticket = 0u;
 }
 
-// Final, single-block and ordered: out[13] in diagnostics.csv order.
-__global__ void diagnostics_final_kernel(int n_mom, const double* mom_part, int n_pot,
-                                         const double* pot_part, double G, double* out) {
-    __shared__ double sums[12];
-    const int c = threadIdx.x;
-    if (c < 11) {
-        double s = 0.0;
-        for (int b = 0; b < n_mom; ++b) s += mom_part[(size_t)b * 11 + c];
-        sums[c] = s;
-    } else if (c == 11) {
-        double s = 0.0;
-        for (int b = 0; b < n_pot; ++b) s += pot_part[b];
-        sums[11] = s;
-    }
-    __syncthreads();
-    if (c == 0) {
-        const double M = sums[0];
-        const double pe = -0.5 * G * sums[11];
-        out[0] = M;
-        out[1] = sums[1];
-        out[2] = pe;
-        out[3] = sums[1] + pe;
-        out[4] = sums[2];
-        out[5] = sums[3];
-        out[6] = sums[4];
-        out[7] = M > 0.0 ? sums[5] / M : sums[5];
-        out[8] = M > 0.0 ? sums[6] / M : sums[6];
-        out[9] = M > 0.0 ? sums[7] / M : sums[7];
-        out[10] = sums[8];
-        out[11] = sums[9];
-        out[12] = sums[10];
-    }
-}
+// Tile shape and items for n bodies.  Up to kDiagSmall bodies: 64-body tiles of one-target
+// threads, so that even a thousand bodies spread over all SMs; above: 256-body tiles, two
+// targets per thread (each staged source read once for two pairs).  Items hold as many tile
+// pairs as keeps their number at most kDiagMaxItems, several waves of resident blocks.
+constexpr int kDiagSmall = 8192;
+constexpr int64_t kDiagMaxItems = 16384;
+constexpr int kDiagMoments = 148;
+constexpr size_t kDiagHeader = 256;  // the ticket, then the block sums
 
-constexpr int kPotBlock = 128;
-constexpr int kPotJT = 256;
+void diag_shape(int64_t n, DiagArgs* a) {
+    const int64_t T = n <= kDiagSmall ? 64 : 256, block = n <= kDiagSmall ? 64 : 128;
+    a->tiles = (n + T - 1) / T;
+    const int64_t rows = (a->tiles + 1) / 2;
+    const int64_t most = std::max<int64_t>(1, kDiagMaxItems / rows);  // items per double row
+    a->run = (a->tiles + 1 + most - 1) / most;
+    a->chunks = (int)((a->tiles + 1 + a->run - 1) / a->run);
+    a->n_items = (int)(rows * a->chunks);
+    a->n_mom = (int)std::min<int64_t>(kDiagMoments, (n + block - 1) / block);
+}
 
 int grid_for(int64_t n, int block, int cap) {
     int64_t g = (n + block - 1) / block;
@@ -217,29 +281,36 @@ cudaError_t launch_kick_drift(int64_t n, double* x, double* y, double* z, double
 }
 
 size_t diagnostics_scratch_bytes(int64_t n) {
-    const int nm = grid_for(n, kMomBlock, 148 * 4);
-    const int np = grid_for(n, kPotBlock, 1 << 30);
-    return ((size_t)nm * 11 + (size_t)np + 16) * sizeof(double);
+    DiagArgs a;
+    diag_shape(std::max<int64_t>(n, 1), &a);
+    return kDiagHeader + ((size_t)11 * a.n_mom + (size_t)a.n_items) * sizeof(double);
 }
 
 cudaError_t launch_diagnostics(int64_t n, const double* x, const double* y, const double* z,
                                const double* vx, const double* vy, const double* vz,
-                               const double* m, double G, double eps2, double* scratch,
+                               const double* m, double G, double eps2, void* scratch,
                                double* out13, cudaStream_t st) {
-    const int nm = grid_for(n, kMomBlock, 148 * 4);
-    const int np = grid_for(n, kPotBlock, 1 << 30);
-    double* mom = scratch;
-    double* pot = scratch + (size_t)nm * 11;
-    if (n <= 0) {
-        cudaError_t e = cudaMemsetAsync(out13, 0, 13 * sizeof(double), st);
-        return e;
+    if (n <= 0) return cudaMemsetAsync(out13, 0, 13 * sizeof(double), st);
+    DiagArgs a;
+    diag_shape(n, &a);
+    a.n = n;
+    a.x = x; a.y = y; a.z = z;
+    a.vx = vx; a.vy = vy; a.vz = vz;
+    a.m = m;
+    a.G = G;
+    a.eps2 = eps2;
+    a.ticket = (unsigned*)scratch;
+    a.part = (double*)((char*)scratch + kDiagHeader);
+    a.out = out13;
+    const unsigned grid = (unsigned)(a.n_mom + a.n_items);
+    const bool eps0 = eps2 < 1e-200;
+    if (n <= kDiagSmall) {
+        if (eps0) diagnostics_kernel<64, 1, true><<<grid, 64, 0, st>>>(a);
+        else diagnostics_kernel<64, 1, false><<<grid, 64, 0, st>>>(a);
+    } else {
+        if (eps0) diagnostics_kernel<128, 2, true><<<grid, 128, 0, st>>>(a);
+        else diagnostics_kernel<128, 2, false><<<grid, 128, 0, st>>>(a);
     }
-    moments_kernel<<<nm, kMomBlock, 0, st>>>(n, x, y, z, vx, vy, vz, m, mom);
-    if (eps2 < 1e-200)
-        potential_kernel<kPotBlock, kPotJT, true><<<np, kPotBlock, 0, st>>>(n, x, y, z, m, eps2, pot);
-    else
-        potential_kernel<kPotBlock, kPotJT, false><<<np, kPotBlock, 0, st>>>(n, x, y, z, m, eps2, pot);
-    diagnostics_final_kernel<<<1, 32, 0, st>>>(nm, mom, np, pot, G, out13);
     return cudaGetLastError();
 }
 
