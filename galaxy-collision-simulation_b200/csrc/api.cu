@@ -341,6 +341,11 @@ Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_
         auto it = g_tuned.find(std::make_tuple(dev, precision, (int)eps0, n_src));
         if (it != g_tuned.end() && n_tgt == n_src) return it->second;
     }
+    if (precision == kF64Exact) {
+        Choice ch;
+        ch.variant = force_exact_variant(n_tgt);
+        return ch;
+    }
     int ids[32];
     const int c = std::min(32, force_variant_ids(precision, eps0 ? 1 : 0, ids, 32));
     int cnt;
@@ -387,7 +392,7 @@ ForceArgs make_args(const ForceJob& j, const gx_physics& ph, const ForceVariant&
     a.t_begin = j.t_begin;
     a.n_tgt = j.n_tgt;
     int ns = nsplit;
-    split_layout(j.n_src, v.jt, nsplit, &a.j_chunk, &ns);
+    split_layout(j.n_src, v.jt, v.precision == kF64Exact ? 1 : nsplit, &a.j_chunk, &ns);
     a.nsplit = ns;
     a.ax = j.ax;
     a.ay = j.ay;
@@ -429,6 +434,7 @@ int run_force(const ForceJob& j, const gx_physics& ph, int precision, Choice ch,
     const bool eps0 = eps0_of(precision, ph);
     if (ch.variant < 0) ch = heuristic_choice(dev, precision, eps0, j.n_tgt, j.n_src);
     const ForceVariant& v = all[ch.variant];
+    if (precision == kF64Exact) ch.nsplit = 1;  // its sums run over the sources in order
     const size_t need = part_bytes(v, j.n_src, j.n_tgt, ch.nsplit);
     const size_t tb = ticket_bytes(std::max(j.n_src, j.n_tgt));
     AsyncBuf tmp;

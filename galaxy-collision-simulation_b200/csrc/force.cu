@@ -75,16 +75,24 @@ __global__ void __launch_bounds__(BLOCK) force_f64_kernel(const ForceArgs a) {
     finish_tile<BLOCK, IPT>(a, tile, tile * (BLOCK * IPT));
 }
 
-template <int BLOCK, int JT>
-__global__ void __launch_bounds__(BLOCK) force_exact_kernel(const ForceArgs a) {
-    exact_tile<BLOCK, JT>(a, (int64_t)blockIdx.x * BLOCK);
+template <int TG, int PW, int U>
+__global__ void __launch_bounds__(ExactShape<TG, PW, U>::BLOCK) force_exact_kernel(const ForceArgs a) {
+    exact_tile<TG, PW, U>(a, (int64_t)blockIdx.x * TG);
+}
+
+template <int BLOCK, int JT, int U>
+__global__ void __launch_bounds__(BLOCK) force_exact_serial_kernel(const ForceArgs a) {
+    exact_serial_tile<BLOCK, JT, U>(a, (int64_t)blockIdx.x * BLOCK);
 }
 
 #define MIXED(B, I, J, P, E) {kMixed, B, I, J, P, E, (const void*)&force_mixed_kernel<B, I, J, P, E>}
 #define MIXTP(B, I, J, E, MB) {kMixed, B, I, J, 2, E, (const void*)&force_mixed_tp_kernel<B, I, J, E, MB>}
 #define MIXTPU(B, I, J, MB, U) {kMixed, B, I, J, 2, 0, (const void*)&force_mixed_tp_kernel<B, I, J, false, MB, U>}
 #define F64(B, I, J, E) {kF64, B, I, J, 0, E, (const void*)&force_f64_kernel<B, I, J, E>}
-#define EXACT(B, J) {kF64Exact, B, 1, J, 0, 1, (const void*)&force_exact_kernel<B, J>}
+#define EXSER(B, J, U) {kF64Exact, B, 1, J, 0, 1, (const void*)&force_exact_serial_kernel<B, J, U>}
+#define EXACT(T, W, U)                                                                             \
+    {kF64Exact, ExactShape<T, W, U>::BLOCK, 1, ExactShape<T, W, U>::JT, 0, 1,                      \
+     (const void*)&force_exact_kernel<T, W, U>, T}
 
 const ForceVariant kVariants[] = {
     // mixed, targets packed (fastest at N = 2^20; the first entry is the untuned default)
@@ -108,9 +116,17 @@ const ForceVariant kVariants[] = {
     F64(64, 2, 128, false),
     F64(256, 2, 256, true),
     F64(64, 2, 128, true),
-    EXACT(128, 256),
-    EXACT(64, 128),
+    EXACT(16, 8, 2),
+    EXSER(64, 128, 8),
 };
+// Which exact variant (the last two above, in that order) for n_tgt targets.  The serial kernel
+// needs one thread per target and fills the SMs from 592 warps of targets up; below, and until
+// its second round of warps is well filled, the cooperative one is faster in spite of the terms
+// it passes through shared memory.  Measured with n targets and n sources, cooperative /
+// serial: n = 1000 20 / 71 us, 4000 73 / 231, 16,384 821 / 886, 19,000 1195 / 1574, 30,000
+// 2682 / 2483 us, 65,536 12.3 / 10.2 ms.
+constexpr int64_t kExactCoopTargets = 27000;
+
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
 }  // namespace
@@ -133,8 +149,17 @@ int force_variant_ids(int precision, int eps0, int* ids, int max_ids) {
 }
 
 int64_t force_tiles(const ForceVariant& v, int64_t n_tgt) {
-    const int64_t tile = (int64_t)v.block * v.ipt;
+    const int64_t tile = v.targets ? v.targets : (int64_t)v.block * v.ipt;
     return (n_tgt + tile - 1) / tile;
+}
+
+int force_exact_variant(int64_t n_tgt) {
+    static const int first = [] {
+        int i = 0;
+        while (kVariants[i].precision != kF64Exact) ++i;
+        return i;
+    }();
+    return first + (n_tgt <= kExactCoopTargets ? 0 : 1);
 }
 
 cudaError_t force_launch(const ForceVariant& v, const ForceArgs& args, cudaStream_t stream) {

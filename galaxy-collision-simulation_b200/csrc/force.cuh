@@ -52,12 +52,16 @@ struct ForceVariant {
     int packed;  // 0 scalar FP32, 1 two sources per f32x2, 2 two targets per f32x2
     int eps0;  // guards s == 0 pairs (softening 0)
     const void* fn;
+    int targets = 0;  // targets per CTA where that is not block * ipt (the exact form)
 };
 
 // All compiled variants; eps0 variants are separate entries.
 const ForceVariant* force_variants(int* count);
 // Variants usable for (precision, eps0) in the order of gx_variant_* ids.
 int force_variant_ids(int precision, int eps0, int* ids, int max_ids);
+
+// The exact-form variant for n_tgt targets (an index into force_variants).
+int force_exact_variant(int64_t n_tgt);
 
 // Launches variant `v` over args (ceil(n_tgt / (block*ipt)) * nsplit CTAs) and, when
 // nsplit > 1 without tile tickets, the ordered partial-sum reduction with the epilogue.

@@ -39,6 +39,40 @@ __device__ __forceinline__ double inv_cube_f64(double s, double m) {
     return fma(w * e, p, w);
 }
 
+// RN(1 / RN(sqrt(s))), the value IEEE square root and division give, without their branches.
+// The method is Markstein's (IBM J. Res. Dev. 34, 1990), the argument that of Cornea, Harrison
+// and Tang: a bound, and a look at the exceptions.
+//   y = s^-1/2 within 1.6 x 2^-53; g = s y; the residual r = s - g^2 makes g + r y/2 agree
+//   with sqrt(s) to 10 x 2^-106 before its one rounding, so q could be wrong only for
+//   s = M^2 - d with an odd 54-bit M and |d| <= 80.  These are the square roots of d modulo
+//   2^54; q is right for all of them (|d| < 128; tests/test_exact_form_gpu.py meets each).
+//   e = 1 - q y is exact and |e| <= 2.6 x 2^-53, so y + y e agrees with 1/q to 7 x 2^-106, and
+//   inv could be wrong only where 1/q lies that close to the middle between two doubles.
+//   Then the exact e1 = 1 - q inv is q times half an ulp of inv, a power of two, to 2^-51:
+//   the mantissas of e1 and q agree, which the high words tell.  (Some sixty mantissas q,
+//   divisors of 2^106 + d with small d, do round the wrong way and are caught so.)
+// 12 FP64 operations and one MUFU; the checks are integer work.  A batch of arguments shares
+// one ExactGuard: when it is not clean() -- an argument outside [2^-894, 2^897) (zero, infinity
+// and NaN among them) or a rounding this cannot settle, about one argument in 2^18 -- the batch
+// takes IEEE root and division instead.
+struct ExactGuard {
+    unsigned near = 0xffffffffu, range = 0u;
+    __device__ __forceinline__ bool clean() const { return near > 2u && range < (1791u << 20); }
+};
+__device__ __forceinline__ double exact_inv(double s, ExactGuard& guard) {
+    const double y = rsqrt_f64(s);
+    const double g = __dmul_rn(s, y);
+    const double r = __fma_rn(-g, g, s);
+    const double q = __fma_rn(r, __dmul_rn(0.5, y), g);
+    const double e = __fma_rn(-q, y, 1.0);
+    const double inv = __fma_rn(e, y, y);
+    const double e1 = __fma_rn(-q, inv, 1.0);
+    guard.near = min(guard.near, (unsigned)(__double2hiint(e1) - __double2hiint(q) + 1) & 0xfffffu);
+    guard.range = max(guard.range, (unsigned)__double2hiint(s) - (129u << 20));
+    return inv;
+}
+__device__ __forceinline__ double ieee_inv(double s) { return __ddiv_rn(1.0, __dsqrt_rn(s)); }
+
 __device__ __forceinline__ float rsqrt_f32(float s) {
     float y;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
