@@ -1659,6 +1659,7 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
     GX_TRY(dev_copy(hs, T.near_leaf, &P.near_leaf));
     GX_TRY(mark(tm, 1, hs.st));
     GX_TRY(dev_array(hs, (int64_t)P.n_nodes * kFmmRec, &fa.rec));
+    GX_TRY(dev_array(hs, (int64_t)fmm_octets(P.n_nodes), &fa.octet_parent));
     GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), T.n_levels(), hs.st));
     GX_TRY(mark(tm, 2, hs.st));
     // far-field work items for the leaves that hold a target in [begin, end)
@@ -1772,7 +1773,14 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     fa.node_cz = t.cz;
     fa.perm = t.perm;
     GX_TRY(dev_array(hs, (int64_t)P.n_nodes * kFmmRec, &fa.rec));
-    GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), hdr[1], st));
+    GX_TRY(dev_array(hs, (int64_t)fmm_octets(P.n_nodes), &fa.octet_parent));
+    // flags of the one-launch upward pass: {error words (2), ticket, ready[]}
+    int* m2m;
+    GX_TRY(dev_array(hs, 3 + (int64_t)fmm_octets(P.n_nodes), &m2m));
+    GX_CUDA(cudaMemsetAsync(m2m, 0, 2 * sizeof(int), st));
+    int dev = 0;
+    GX_CUDA(cudaGetDevice(&dev));
+    GX_CUDA(launch_fmm_moments_tree(fa, m2m + 2, m2m + 3, m2m, sm_count(dev), st));
     GX_TRY(mark(tm, 2, st));
 
     TreeListArgs la{};
@@ -1810,9 +1818,18 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     GX_CUDA(launch_tree_lists_count(la, list_temp, list_bytes, st));
     int32_t nl = 0;
     unsigned long long tot[6];
-    GX_CUDA(cudaMemcpyAsync(&nl, la.start_ord + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GX_CUDA(cudaMemcpyAsync(tot, la.totals, sizeof(tot), cudaMemcpyDeviceToHost, st));
-    GX_CUDA(cudaStreamSynchronize(st));
+    for (int attempt = 0;; ++attempt) {
+        int m2m_err = 0;
+        GX_CUDA(cudaMemcpyAsync(&nl, la.start_ord + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GX_CUDA(cudaMemcpyAsync(tot, la.totals, sizeof(tot), cudaMemcpyDeviceToHost, st));
+        GX_CUDA(cudaMemcpyAsync(&m2m_err, m2m, sizeof(int), cudaMemcpyDeviceToHost, st));
+        GX_CUDA(cudaStreamSynchronize(st));
+        if (m2m_err == 0 || attempt == 1) break;
+        // a bounded wait of the one-launch upward pass gave up: the passes again, level by level
+        GX_CUDA(cudaMemsetAsync(m2m, 0, sizeof(int), st));
+        GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), hdr[1], st));
+        GX_CUDA(launch_tree_lists_count(la, list_temp, list_bytes, st));
+    }
     for (int k = 0; k < 4; ++k)
         if (tot[k] > (unsigned long long)std::numeric_limits<int32_t>::max())
             return fail(GX_ERR_UNSUPPORTED, "FMM: interaction lists exceed the int32 range");
@@ -2038,7 +2055,7 @@ struct FmmWork {
     size_t order_bytes = 0;
     void* p2p_scratch = nullptr;
     int* flags = nullptr;                // device: [0] per-evaluation overflow, [1] sticky (bit 1: too deep)
-    int* m2m_ready = nullptr;            // device: per-node flags and a ticket of the one-launch M2M
+    int* m2m_ready = nullptr;            // device: per-octet flags and a ticket of the one-launch M2M
     int* m2m_ticket = nullptr;
     // Second stream of the evaluation (moments, far field) and the events that fork and join
     // it; the near field of the FP64 and mixed forms goes to near[0..3n) and is added after.
@@ -2115,7 +2132,7 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     GX_TRY(w.grab((int64_t)w.tree_bytes, (char**)&w.tree_temp));
     GX_TRY(w.grab(2, &w.flags));
     GX_TRY(w.grab(6, &w.need));
-    GX_TRY(w.grab(NC, &w.m2m_ready));
+    GX_TRY(w.grab((int64_t)fmm_octets(NC), &w.m2m_ready));
     GX_TRY(w.grab(1, &w.m2m_ticket));
     GX_TRY(w.grab(3 * n, &w.near));
     GX_CUDA(cudaStreamCreateWithFlags(&w.aux, cudaStreamNonBlocking));
@@ -2135,6 +2152,7 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     fa.perm = t.perm;
     fa.cnt_nodes = t.hdr;
     GX_TRY(w.grab((int64_t)NC * kFmmRec, &fa.rec));
+    GX_TRY(w.grab((int64_t)fmm_octets(NC), &fa.octet_parent));
     GX_TRY(w.grab((int64_t)NC * kRec32, &fa.rec32));
 
     TreeListArgs& la = w.la;

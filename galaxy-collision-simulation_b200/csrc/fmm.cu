@@ -5,9 +5,9 @@
 // (cpp/fmm/fmm_solver.cpp:157-208) with add_multipole_point / add_multipole_shifted_child
 // (cpp/fmm/multipole.cpp:218-252) are restated with the reference's operations in the
 // reference's order and no contraction (dadd/dmul), so masses, centres of mass and the 31
-// moments of every node are bit-identical to the reference's (for masses >= 0).  One warp
-// per node; lane k owns moment 4 + k.  Leaves first, then one launch per tree level,
-// deepest first.
+// moments of every node are bit-identical to the reference's (for masses >= 0).  Leaves first
+// (one warp per leaf; lane k owns moment 4 + k), then the internal nodes, deepest first (a block
+// per node, a warp per child).
 //
 // M2P.  multipole_acceleration (multipole.cpp:254-296) builds the degree-4 Taylor
 // polynomial of (d + u)_c |d + u|_eps^-3 in the source offset u by truncated polynomial
@@ -91,54 +91,56 @@ constexpr MomentTables make_moment_tables() {
 
 __device__ const MomentTables kTab = make_moment_tables();
 
-// Traces of the moments (record slots 35..45) from slots 4..34.
-__device__ __forceinline__ void write_traces(double* r) {
-    r[kRecTrQ] = r[4] + r[7] + r[9];
-    r[kRecW + 0] = r[10] + r[13] + r[15];
-    r[kRecW + 1] = r[11] + r[16] + r[18];
-    r[kRecW + 2] = r[12] + r[17] + r[19];
-    const double txx = r[20] + r[23] + r[25], tyy = r[23] + r[30] + r[32], tzz = r[25] + r[32] + r[34];
-    r[kRecT2 + 0] = txx;
-    r[kRecT2 + 1] = r[21] + r[26] + r[28];
-    r[kRecT2 + 2] = r[22] + r[27] + r[29];
-    r[kRecT2 + 3] = tyy;
-    r[kRecT2 + 4] = r[24] + r[31] + r[33];
-    r[kRecT2 + 5] = tzz;
-    r[kRecTr2] = txx + tyy + tzz;
+// Traces of the moments (record slots 35..45), one lane each: slot 35 + t of the record from
+// mom[k] = moment 4 + k (shared memory).
+__device__ const signed char kTrace[11][3] = {{0, 3, 5},    {6, 9, 11},   {7, 12, 14},  {8, 13, 15},
+                                              {16, 19, 21}, {17, 22, 24}, {18, 23, 25}, {19, 26, 28},
+                                              {20, 27, 29}, {21, 28, 30}, {0, 0, 0}};
+__device__ __forceinline__ double trace_of(const double* mom, int t) {
+    auto sum3 = [&](int k) { return mom[kTrace[k][0]] + mom[kTrace[k][1]] + mom[kTrace[k][2]]; };
+    return t < 10 ? sum3(t) : sum3(4) + sum3(7) + sum3(9);
 }
 
-// v^e for e in 0..4 as pow_int (multipole.cpp:43-49) computes it: 1.0 times v, e times
-// (the first product is exact).
-struct Pow4 {
-    double p1, p2, p3, p4;
-    __device__ __forceinline__ explicit Pow4(double v) : p1(v), p2(dmul(v, v)), p3(dmul(p2, v)), p4(dmul(p3, v)) {}
-    __device__ __forceinline__ double operator()(int e) const {
-        return e == 0 ? 1.0 : (e == 1 ? p1 : (e == 2 ? p2 : (e == 3 ? p3 : p4)));
-    }
-};
-
 // Leaf moments: p2m_m2m leaf branch (fmm_solver.cpp:162-167, 180-181) and
-// compute_multipole_moments leaf branch (:187-193).  One warp per node; internal nodes
-// return.  The leaf's bodies are staged 32 at a time in shared memory; every lane then
-// runs the reference's sequential sums over them (lane k for moment 4 + k).  A massless
-// leaf gets its cell centre as centre of mass, as in the reference.
+// compute_multipole_moments leaf branch (:187-193).  One warp per node; the warp of an
+// internal node only enters it as its octet's parent (the children of the o-th split node are
+// nodes 1 + 8 o ..).  The leaf's bodies are staged 32 at a time in shared memory and every lane
+// runs the reference's sequential sums over them.  For the moments (lane k for moment 4 + k),
+// lane q first puts the powers of body q's offset, as pow_int (multipole.cpp:43-49) computes
+// them, beside one another (rows of 33: the lanes of a warp read up to five rows at one body
+// without a bank conflict).  A massless leaf gets its cell centre as centre of mass, as in the
+// reference.  Bound by latency (dependent loads, the sums, three divisions): N = 65,536 leaf 64
+// 13 us, N = 2^20 leaf 16 205 us; with every lane computing and selecting the powers of
+// every body 40 and 346 us.
+constexpr int kPowRow = 33;
 __global__ void __launch_bounds__(kMomBlock) fmm_leaf_kernel(const FmmArgs a) {
-    __shared__ double s_b[kMomBlock / 32][4][32];
+    __shared__ double s_pow[kMomBlock / 32][15 * kPowRow];  // rows 5 c + e; first x, y, z, m in rows 1, 6, 11, 14
+    __shared__ double s_m[kMomBlock / 32][32];
     const int wl = threadIdx.x >> 5;
     const int w = (int)((blockIdx.x * (unsigned)kMomBlock + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    if (w >= fmm_nodes(a) || a.node_child[w] >= 0) return;
+    if (w >= fmm_nodes(a)) return;
+    const int c0 = a.node_child[w];
+    if (c0 >= 0) {
+        if (lane == 0) a.octet_parent[(c0 - 1) >> 3] = w;
+        return;
+    }
     const int b = a.node_beg[w], e = a.node_end[w];
     double* r = a.rec + (size_t)w * kFmmRec;
-    double(*sb)[32] = s_b[wl];
+    double* const pw = s_pow[wl];
+    double* const sm = s_m[wl];
+    double x = 0.0, y = 0.0, z = 0.0;  // this lane's body of the staged chunk
     auto stage = [&](int k0) {
         __syncwarp();
         if (k0 + lane < e) {
             const int i = a.perm[k0 + lane];
-            sb[0][lane] = a.x[i];
-            sb[1][lane] = a.y[i];
-            sb[2][lane] = a.z[i];
-            sb[3][lane] = a.m[i];
+            x = a.x[i];
+            y = a.y[i];
+            z = a.z[i];
+            pw[1 * kPowRow + lane] = x;
+            pw[6 * kPowRow + lane] = y;
+            pw[11 * kPowRow + lane] = z;
+            sm[lane] = a.m[i];
         }
         __syncwarp();
         return min(32, e - k0);
@@ -148,165 +150,214 @@ __global__ void __launch_bounds__(kMomBlock) fmm_leaf_kernel(const FmmArgs a) {
         const int cnt = stage(k0);
 #pragma unroll 4
         for (int q = 0; q < cnt; ++q) {
-            const double mi = sb[3][q];
+            const double mi = sm[q];
             mass = dadd(mass, mi);
-            wx = dadd(wx, dmul(sb[0][q], mi));
-            wy = dadd(wy, dmul(sb[1][q], mi));
-            wz = dadd(wz, dmul(sb[2][q], mi));
+            wx = dadd(wx, dmul(pw[1 * kPowRow + q], mi));
+            wy = dadd(wy, dmul(pw[6 * kPowRow + q], mi));
+            wz = dadd(wz, dmul(pw[11 * kPowRow + q], mi));
         }
     }
-    const bool pos = mass > 0.0;
-    const double cx = pos ? __ddiv_rn(wx, mass) : a.node_cx[w];
-    const double cy = pos ? __ddiv_rn(wy, mass) : a.node_cy[w];
-    const double cz = pos ? __ddiv_rn(wz, mass) : a.node_cz[w];
+    // lanes 0..2 divide one component each
+    double com = 0.0;
+    if (lane < 3) {
+        const double num = lane == 0 ? wx : lane == 1 ? wy : wz;
+        const double* cell = lane == 0 ? a.node_cx : lane == 1 ? a.node_cy : a.node_cz;
+        com = mass > 0.0 ? __ddiv_rn(num, mass) : cell[w];
+    }
+    const double cx = __shfl_sync(0xffffffffu, com, 0), cy = __shfl_sync(0xffffffffu, com, 1);
+    const double cz = __shfl_sync(0xffffffffu, com, 2);
     const int ks = lane < 31 ? 4 + lane : 0;
-    const int ex = kTab.ex[ks], ey = kTab.ey[ks], ez = kTab.ez[ks];
+    const double* rx = pw + kTab.ex[ks] * kPowRow;
+    const double* ry = pw + (5 + kTab.ey[ks]) * kPowRow;
+    const double* rz = pw + (10 + kTab.ez[ks]) * kPowRow;
     double v = 0.0;
     for (int k0 = b; k0 < e; k0 += 32) {
-        const int cnt = stage(k0);
-#pragma unroll 4
-        for (int q = 0; q < cnt; ++q) {
-            const Pow4 px(dsub(sb[0][q], cx)), py(dsub(sb[1][q], cy)), pz(dsub(sb[2][q], cz));
-            const double mono = dmul(dmul(px(ex), py(ey)), pz(ez));
-            v = dadd(v, dmul(sb[3][q], mono));
+        const int cnt = e - b > 32 ? stage(k0) : e - b;
+        __syncwarp();
+        if (lane < cnt) {
+            auto powers = [&](double u, double* p) {
+                const double u2 = dmul(u, u), u3 = dmul(u2, u);
+                p[0] = 1.0;
+                p[kPowRow] = u;
+                p[2 * kPowRow] = u2;
+                p[3 * kPowRow] = u3;
+                p[4 * kPowRow] = dmul(u3, u);
+            };
+            powers(dsub(x, cx), pw + lane);
+            powers(dsub(y, cy), pw + 5 * kPowRow + lane);
+            powers(dsub(z, cz), pw + 10 * kPowRow + lane);
         }
-    }
-    if (lane < 31) {
-        r[4 + lane] = v;
-    } else {
-        r[0] = cx;
-        r[1] = cy;
-        r[2] = cz;
-        r[kRecMass] = mass;
+        __syncwarp();
+#pragma unroll 4
+        for (int q = 0; q < cnt; ++q) v = dadd(v, dmul(sm[q], dmul(dmul(rx[q], ry[q]), rz[q])));
     }
     __syncwarp();
-    if (lane == 0) write_traces(r);
+    pw[lane] = v;
+    if (lane < 31) r[4 + lane] = v;
+    else r[kRecMass] = mass;
+    if (lane < 3) r[lane] = com;
+    __syncwarp();
+    if (lane < 11) r[kRecTrQ + lane] = trace_of(pw, lane);
 }
 
 // Internal node: p2m_m2m (fmm_solver.cpp:168-181) over the children in octant order, then
-// add_multipole_shifted_child per child (multipole.cpp:227-252).  One CTA per node: the 8
-// children's records are staged in shared memory, warp c computes child c's shifted
-// contribution to every moment (lane a for moment 4 + a), and warp 0 adds the 8
-// contributions in child order, as the reference does.  A massless child adds exact zeros
-// to every sum in the reference and is skipped here (masses are >= 0).
-// All threads of the CTA call it for the same node w (it holds CTA barriers).
-__device__ __forceinline__ void m2m_node(const FmmArgs& a, const int w, double (*s_child)[kRecTrQ],
-                                         double (*s_val)[32]) {
-    const int c0 = a.node_child[w];
-    if (c0 < 0) return;
+// add_multipole_shifted_child per child (multipole.cpp:227-252), with the reference's operations
+// in its order.  One block per node at a time: the 8 children's records are staged in shared
+// memory, warp c computes child c's shifted contribution to every moment (lane a for moment
+// 4 + a), and warp 0 adds the 8 contributions in child order, as the reference does.  A massless
+// child adds exact zeros to every sum in the reference and is skipped here (masses are >= 0).
+// The terms of a moment (binomial product, slot of the child's moment, powers of the shift) differ
+// from lane to lane, so they are read from tables: in shared memory, term by term across the
+// lanes, and the powers of a child's shift beside them, all free of bank conflicts (in global
+// memory they cost some 1800 L1 wavefronts per child: N = 2^20 leaf 16 750 us).
+constexpr int kM2MBlock = 256;
+struct M2MShared {
+    double bin[kMaxShiftTerms][32];
+    int term[kMaxShiftTerms][32];  // kb | dx << 8 | dy << 12 | dz << 16
+    double child[8][kRecTrQ];
+    double pow[8][3][6];
+    double val[8][32];
+    double mom[32];
+    int node;
+};
+
+__device__ __forceinline__ void m2m_tables(M2MShared& s) {
+    for (int i = threadIdx.x; i < kMaxShiftTerms * 32; i += kM2MBlock) {
+        const int q = i >> 5, l = i & 31;
+        const bool in = l < 31 && q < kTab.nterm[l];
+        s.bin[q][l] = in ? kTab.bin[l][q] : 0.0;
+        // slot of the child's moment: the mass for moment 0
+        const int kb = in ? (kTab.kb[l][q] == 0 ? kRecMass : kTab.kb[l][q]) : kRecMass;
+        s.term[q][l] = in ? kb | kTab.dx[l][q] << 8 | kTab.dy[l][q] << 12 | kTab.dz[l][q] << 16 : kb;
+    }
+}
+
+// All threads of the block, for the same internal node w with children c0 .. c0 + 7; tables filled
+// (before a barrier).  Ends with a barrier.
+__device__ __forceinline__ void m2m_node(const FmmArgs& a, const int w, const int c0, M2MShared& s) {
     const int tid = threadIdx.x, c = tid >> 5, lane = tid & 31;
-    for (int k = tid; k < 8 * kRecTrQ; k += 256)
-        s_child[k / kRecTrQ][k % kRecTrQ] = __ldcg(&a.rec[(size_t)(c0 + k / kRecTrQ) * kFmmRec + k % kRecTrQ]);
+    for (int k = tid; k < 8 * kRecTrQ; k += kM2MBlock)
+        s.child[k / kRecTrQ][k % kRecTrQ] = __ldcg(&a.rec[(size_t)(c0 + k / kRecTrQ) * kFmmRec + k % kRecTrQ]);
     __syncthreads();
     double mass = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
+#pragma unroll
     for (int q = 0; q < 8; ++q) {
-        const double cm = s_child[q][kRecMass];
+        const double cm = s.child[q][kRecMass];
         if (!(cm > 0.0)) continue;
         mass = dadd(mass, cm);
-        wx = dadd(wx, dmul(s_child[q][0], cm));
-        wy = dadd(wy, dmul(s_child[q][1], cm));
-        wz = dadd(wz, dmul(s_child[q][2], cm));
+        wx = dadd(wx, dmul(s.child[q][0], cm));
+        wy = dadd(wy, dmul(s.child[q][1], cm));
+        wz = dadd(wz, dmul(s.child[q][2], cm));
     }
-    const bool pos = mass > 0.0;
-    const double cx = pos ? __ddiv_rn(wx, mass) : a.node_cx[w];
-    const double cy = pos ? __ddiv_rn(wy, mass) : a.node_cy[w];
-    const double cz = pos ? __ddiv_rn(wz, mass) : a.node_cz[w];
-    const double* cr = s_child[c];
-    const double cm = cr[kRecMass];
-    if (lane < 31 && cm > 0.0) {
-        const Pow4 px(dsub(cr[0], cx)), py(dsub(cr[1], cy)), pz(dsub(cr[2], cz));
-        // The terms are independent until the sum: the loop runs to the table's bound with the
-        // lane's own count as a predicate, so the loads and products of later terms overlap the
-        // additions, which stay in the reference's order.
-        const int nt = kTab.nterm[lane];
+    // lane 0..2 of every warp divides its component
+    const double num = lane == 0 ? wx : lane == 1 ? wy : wz;
+    const double* cell = lane == 0 ? a.node_cx : lane == 1 ? a.node_cy : a.node_cz;
+    double com = 0.0;
+    const double* cr = s.child[c];
+    if (lane < 3) {
+        com = mass > 0.0 ? __ddiv_rn(num, mass) : cell[w];
+        // powers 0..4 of the child's shift, as pow_int computes them
+        const double v = dsub(cr[lane], com);
+        double* pw = s.pow[c][lane];
+        const double v2 = dmul(v, v), v3 = dmul(v2, v);
+        pw[0] = 1.0;
+        pw[1] = v;
+        pw[2] = v2;
+        pw[3] = v3;
+        pw[4] = dmul(v3, v);
+    }
+    __syncwarp();
+    if (cr[kRecMass] > 0.0) {
+        const int nt = lane < 31 ? kTab.nterm[lane] : 0;
         double value = 0.0;
 #pragma unroll
         for (int q = 0; q < kMaxShiftTerms; ++q) {
-            if (q < nt) {
-                const double sf = dmul(dmul(dmul(kTab.bin[lane][q], px(kTab.dx[lane][q])), py(kTab.dy[lane][q])),
-                                       pz(kTab.dz[lane][q]));
-                if (sf != 0.0) {
-                    const int kb = kTab.kb[lane][q];
-                    value = dadd(value, dmul(sf, kb == 0 ? cm : cr[kb]));
-                }
-            }
+            const int t = s.term[q][lane];
+            const double sf = dmul(dmul(dmul(s.bin[q][lane], s.pow[c][0][t >> 8 & 15]), s.pow[c][1][t >> 12 & 15]),
+                                   s.pow[c][2][t >> 16]);
+            const double next = dadd(value, dmul(sf, cr[t & 255]));
+            if (q < nt && sf != 0.0) value = next;
         }
-        s_val[c][lane] = value;
+        s.val[c][lane] = value;
     }
     __syncthreads();
     if (c == 0) {
         double* r = a.rec + (size_t)w * kFmmRec;
-        if (lane < 31) {
-            double total = 0.0;
-            for (int q = 0; q < 8; ++q)
-                if (s_child[q][kRecMass] > 0.0) total = dadd(total, s_val[q][lane]);
-            r[4 + lane] = total;
-        } else {
-            r[0] = cx;
-            r[1] = cy;
-            r[2] = cz;
-            r[kRecMass] = mass;
-        }
+        double total = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (s.child[q][kRecMass] > 0.0) total = dadd(total, s.val[q][lane]);
+        s.mom[lane] = total;
+        if (lane < 31) r[4 + lane] = total;
+        if (lane < 3) r[lane] = com;
+        if (lane == 3) r[kRecMass] = mass;
         __syncwarp();
-        if (lane == 0) write_traces(r);
+        if (lane < 11) r[kRecTrQ + lane] = trace_of(s.mom, lane);
     }
     __syncthreads();  // the staging arrays are free for the next node
 }
 
-__global__ void __launch_bounds__(256) fmm_m2m_kernel(const FmmArgs a, int lb) {
-    __shared__ double s_child[8][kRecTrQ];
-    __shared__ double s_val[8][32];
-    m2m_node(a, lb + blockIdx.x, s_child, s_val);
+// The octets [ob, oe) (one level's split nodes), level by level.
+__global__ void __launch_bounds__(kM2MBlock) fmm_m2m_kernel(const FmmArgs a, int ob, int oe) {
+    __shared__ M2MShared s;
+    m2m_tables(s);
+    for (int o = ob + blockIdx.x; o < oe; o += gridDim.x) m2m_node(a, a.octet_parent[o], 1 + 8 * o, s);
 }
 
-// Every internal node in one launch, without a barrier per level.  Blocks take the nodes
-// from a ticket counter in decreasing index order; levels are numbered top down, so a node
-// comes after all its children.  A block waits (thread c for child c) until the flag of each
-// internal child is set, computes the node as above and sets its own flag.  A block only
-// waits for nodes whose tickets were taken before its own, by blocks already running, so the
-// wait always ends; it is bounded all the same (timeout_ns of the global timer), and a wait
-// that gives up sets bit 0 of err[0] and err[1] (the evaluation is then redone).  Child
-// records are read through L2 (__ldcg), since another SM wrote them in this launch.
+// Every internal node in one launch, without a barrier per level.  Blocks take the octets from
+// a ticket counter in decreasing order; levels are numbered top down, so a node comes after all
+// its children.  A block waits (thread c for child c) until the flag of each internal child's
+// octet is set, computes the node and sets its own flag.  A block only waits for nodes whose
+// tickets were taken before its own, by blocks already running, so the wait always ends; it is
+// bounded all the same (timeout_ns of the global timer), and a wait that gives up sets bit 0 of
+// err[0] and err[1] (the evaluation is then redone).  Child records are read through L2
+// (__ldcg), since another SM wrote them in this launch.
+// Bound by the latency of one node per level: N = 65,536 leaf 64 (9 levels) 40 us, N = 2^20 leaf 16
+// 235 us, against 79 and 750 us with the tables in global memory (and a ticket per node, or a
+// launch per level).  (Eight lanes per node with the shift terms as straight-line code:
+// 110 and 156 us; its 80 KB of instructions are fetched anew on every level.)
 __device__ __forceinline__ unsigned long long m2m_clock() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
 
-__global__ void __launch_bounds__(256) fmm_m2m_tree_kernel(const FmmArgs a, int* ticket, int* ready, int* err,
-                                                           unsigned long long timeout_ns) {
-    __shared__ double s_child[8][kRecTrQ];
-    __shared__ double s_val[8][32];
-    __shared__ int s_t;
-    const int nn = fmm_nodes(a);
+__global__ void __launch_bounds__(kM2MBlock) fmm_m2m_tree_kernel(const FmmArgs a, int* ticket, int* ready, int* err,
+                                                                 unsigned long long timeout_ns) {
+    __shared__ M2MShared s;
+    m2m_tables(s);
+    const int octets = (fmm_nodes(a) - 1) >> 3;  // -1 >> 3 = -1 when there are no nodes
     for (;;) {
-        if (threadIdx.x == 0) s_t = atomicAdd(ticket, 1);
+        if (threadIdx.x == 0) s.node = atomicAdd(ticket, 1);
         __syncthreads();
-        const int t = s_t;
-        __syncthreads();
-        if (t >= nn) return;
-        const int w = nn - 1 - t;
-        const int c0 = a.node_child[w];
-        if (c0 < 0) continue;  // a leaf: fmm_leaf_kernel wrote it
-        if (threadIdx.x < 8 && a.node_child[c0 + threadIdx.x] >= 0) {
-            const int* f = ready + c0 + threadIdx.x;
-            const unsigned long long t0 = m2m_clock();
-            int v = 0;
-            for (unsigned it = 0;; ++it) {
-                asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
-                if (v) break;
-                if ((it & 255) == 255 && m2m_clock() - t0 > timeout_ns) {
-                    atomicOr(err, 1);
-                    atomicOr(err + 1, 1);
-                    break;
+        const int o = octets - 1 - s.node;
+        if (o < 0) return;
+        const int c0 = 1 + 8 * o;
+        if (threadIdx.x < 8) {
+            const int gc = a.node_child[c0 + threadIdx.x];
+            if (gc >= 0) {
+                const int* f = ready + ((gc - 1) >> 3);
+                const unsigned long long t0 = m2m_clock();
+                int v = 0;
+                for (unsigned it = 0;; ++it) {
+                    asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+                    if (v) break;
+                    if ((it & 255) == 255 && m2m_clock() - t0 > timeout_ns) {
+                        atomicOr(err, 1);
+                        atomicOr(err + 1, 1);
+                        break;
+                    }
                 }
             }
         }
         __syncthreads();
-        m2m_node(a, w, s_child, s_val);  // ends with a block barrier
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(ready + w), "r"(1) : "memory");
+        m2m_node(a, a.octet_parent[o], c0, s);  // ends with a block barrier; warp 0 wrote the record
+        if (threadIdx.x < 32) {
+            __threadfence();
+            __syncwarp();
+            if (threadIdx.x == 0)
+                asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(ready + o), "r"(1) : "memory");
+        }
     }
 }
 
@@ -391,18 +442,29 @@ __device__ __forceinline__ void m2p_one(const float* __restrict__ r, double tx, 
     m2p_terms<P, float>(r + 3, (float)(com[0] - tx), (float)(com[1] - ty), (float)(com[2] - tz), eps2, fx, fy, fz);
 }
 
-// The mixed-precision records (kRec32) from the FP64 ones, one thread per node.
+// The mixed-precision records (kRec32) from the FP64 ones, one thread per 16 bytes (13 per
+// node) so that both sides are read and written in whole sectors.  Bound by HBM: N = 2^20 leaf 16
+// (282,000 nodes, 158 MB) 25 us, against 155 us with one thread per node.
+constexpr int kRec32Pieces = kRec32 / 4;
 __global__ void __launch_bounds__(256) fmm_rec32_kernel(const FmmArgs a) {
-    const int k = blockIdx.x * 256 + threadIdx.x;
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    const int64_t k = i / kRec32Pieces;
+    const int p = (int)(i - k * kRec32Pieces);
     if (k >= fmm_nodes(a)) return;
     const double* r = a.rec + (size_t)k * kFmmRec;
-    float* o = a.rec32 + (size_t)k * kRec32;
-    double* oc = reinterpret_cast<double*>(o);
-    oc[0] = r[0];
-    oc[1] = r[1];
-    oc[2] = r[2];
-    for (int q = kRecMass; q <= kRecTr2; ++q) o[q + 3] = __double2float_rn(r[q]);
-    for (int q = kRecTr2 + 4; q < kRec32; ++q) o[q] = 0.0f;
+    float4 v;
+    float* f = reinterpret_cast<float*>(&v);
+    if (p == 0) {
+        reinterpret_cast<double2*>(&v)[0] = make_double2(r[0], r[1]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int slot = 4 * p + q - 3;  // float 4 p + q holds slot 4 p + q - 3 of the record
+            f[q] = slot <= kRecTr2 ? __double2float_rn(r[slot]) : 0.0f;
+        }
+        if (p == 1) reinterpret_cast<double*>(&v)[0] = r[2];  // floats 4 and 5: the third coordinate
+    }
+    reinterpret_cast<float4*>(a.rec32 + (size_t)k * kRec32)[p] = v;
 }
 
 // Shared-memory stride of a staged node record, in elements: slots 0..45 of an FP64 record
@@ -588,13 +650,13 @@ int fmm_effective_order(int expansion_order) {
 cudaError_t launch_fmm_moments_tree(const FmmArgs& a, int* ticket, int* ready, int* err, int sms, cudaStream_t st) {
     constexpr int wpb = kMomBlock / 32;
     if (a.n_nodes == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(ready, 0, (size_t)a.n_nodes * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(ready, 0, fmm_octets(a.n_nodes) * sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(ticket, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     fmm_leaf_kernel<<<(a.n_nodes + wpb - 1) / wpb, kMomBlock, 0, st>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int grid = std::min(a.n_nodes, sms * 8);
-    fmm_m2m_tree_kernel<<<grid, 256, 0, st>>>(a, ticket, ready, err, 1000000000ull);
+    const int grid = (int)std::min<int64_t>((int64_t)fmm_octets(a.n_nodes), (int64_t)sms * 8);
+    fmm_m2m_tree_kernel<<<grid, kM2MBlock, 0, st>>>(a, ticket, ready, err, 1000000000ull);
     return cudaGetLastError();
 }
 
@@ -623,10 +685,10 @@ cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, 
     fmm_leaf_kernel<<<(a.n_nodes + wpb - 1) / wpb, kMomBlock, 0, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    for (int d = n_levels - 1; d >= 0; --d) {
-        const int lb = level_off_host[d], le = level_off_host[d + 1];
-        if (le <= lb) continue;
-        fmm_m2m_kernel<<<le - lb, 256, 0, st>>>(a, lb);
+    for (int d = n_levels - 2; d >= 0; --d) {  // octets whose children are level d + 1
+        const int ob = (level_off_host[d + 1] - 1) >> 3, oe = (level_off_host[d + 2] - 1) >> 3;
+        if (oe <= ob) continue;
+        fmm_m2m_kernel<<<std::min(oe - ob, 148 * 8), kM2MBlock, 0, st>>>(a, ob, oe);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -636,7 +698,7 @@ cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, 
 cudaError_t launch_fmm_m2p(const FmmArgs& a, bool mixed, cudaStream_t st) {
     if (a.n_items == 0) return cudaSuccess;
     if (!mixed) return launch_m2p_type<double>(a, st);
-    fmm_rec32_kernel<<<(a.n_nodes + 255) / 256, 256, 0, st>>>(a);
+    fmm_rec32_kernel<<<(unsigned)(((int64_t)a.n_nodes * kRec32Pieces + 255) / 256), 256, 0, st>>>(a);
     const cudaError_t e = cudaGetLastError();
     return e != cudaSuccess ? e : launch_m2p_type<float>(a, st);
 }

@@ -47,6 +47,7 @@ struct FmmArgs {
     const double* node_cx;
     const double* node_cy;
     const double* node_cz;
+    int32_t* octet_parent;  // node whose children are 1 + 8 o ..; fmm_octets(n_nodes), filled with the leaf moments
     const int32_t* perm;
     // leaves with mass > 0, depth-first
     int32_t n_leaves;
@@ -86,17 +87,20 @@ __device__ __forceinline__ int fmm_items(const FmmArgs& a) {
     return a.cnt_items ? (int)min(*a.cnt_items, (unsigned long long)a.n_items) : a.n_items;
 }
 
+// Sets of 8 children a tree of n_nodes nodes has (rounded up).
+constexpr size_t fmm_octets(int32_t n_nodes) { return (size_t)n_nodes / 8 + 1; }
+
 constexpr int kMaxLevels = 22;  // levels an octree of 63-bit path keys can have
 
 // Effective expansion order of multipole_acceleration (multipole.cpp:261-265).
 int fmm_effective_order(int expansion_order);
 constexpr int kM2PChunk = 512;  // far nodes per work item
 
-// Stream-ordered: leaf moments, then one launch per level (deepest first), then M2P.
+// Stream-ordered: leaf moments, then one launch per level (deepest first).
 cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, int n_levels, cudaStream_t st);
 // The same with every internal node in one launch (blocks wait on their children's flags):
-// ticket (1 int) and ready (n_nodes ints) are scratch; a wait that times out sets bit 0 of
-// err[0] and err[1].
+// ticket (1 int) and ready (fmm_octets(n_nodes) ints) are scratch; a wait that times out sets
+// bit 0 of err[0] and err[1].
 cudaError_t launch_fmm_moments_tree(const FmmArgs& a, int* ticket, int* ready, int* err, int sms, cudaStream_t st);
 // ax += nx etc. for i < n (the near field added to the far field).
 cudaError_t launch_fmm_add_near(int64_t n, double* ax, double* ay, double* az, const double* nx, const double* ny,
