@@ -543,7 +543,7 @@ extern "C" int gx_debug_small_warps_per_target(int wpt) {
 }
 
 extern "C" int gx_debug_fmm_tight_pools(int enable) {
-    g_fmm_tight_pools.store(enable ? 1 : 0);
+    g_fmm_tight_pools.store(enable < 0 || enable > 2 ? 1 : enable);
     return GX_OK;
 }
 
@@ -1508,7 +1508,7 @@ extern "C" int gx_p2p_leaves(int64_t n, const double* x, const double* y, const 
     GX_TRY(scratch.alloc(p2p_scratch_bytes(n, n_leaves), st));
     if (device) {
         a.x = x; a.y = y; a.z = z; a.m = m;
-        a.leaf_off = leaf_offsets; a.leaf_part = leaf_particles; a.near_off = near_offsets; a.near_leaf = near_leaves;
+        a.leaf_off = leaf_offsets; a.leaf_part = leaf_particles; a.near_beg = near_offsets; a.near_end = near_offsets + 1; a.near_leaf = near_leaves;
         a.ax = ax; a.ay = ay; a.az = az;
         GX_CUDA(launch_p2p(a, n, precision, scratch.p, sm_count(dev), st));
         return GX_OK;
@@ -1546,7 +1546,7 @@ extern "C" int gx_p2p_leaves(int64_t n, const double* x, const double* y, const 
     GX_TRY(hs.in_any(near_offsets, (int64_t)n_leaves + 1, &dno));
     GX_TRY(hs.in_any(near_leaves ? near_leaves : leaf_offsets, (int64_t)std::max<int32_t>(n_nl, 1), &dnl));
     a.x = dx; a.y = dy; a.z = dz; a.m = dm;
-    a.leaf_off = dlo; a.leaf_part = dlp; a.near_off = dno; a.near_leaf = dnl;
+    a.leaf_off = dlo; a.leaf_part = dlp; a.near_beg = dno; a.near_end = dno + 1; a.near_leaf = dnl;
     a.ax = dax; a.ay = day; a.az = daz;
     GX_CUDA(launch_p2p(a, n, precision, scratch.p, sm_count(dev), st));
     GX_TRY(copy_back(ax, dax, n, st));
@@ -1589,11 +1589,14 @@ struct FmmPlan {
     bool on_device = false;
     int32_t n_nodes = 0, n_leaves = 0;
     std::vector<int32_t> level_off;
-    int64_t n_far = 0, n_near = 0, n_slots = 0;
+    int64_t n_far = 0, n_near = 0, n_slots = 0, n_chunks = 0, n_segs = 0;
     int64_t far_pairs = 0, near_pairs = 0;
     FmmArgs fa{};
-    const int32_t* near_off = nullptr;
+    const int32_t* near_beg = nullptr;  // see P2PArgs
+    const int32_t* near_end = nullptr;
     const int32_t* near_leaf = nullptr;
+    const int32_t* near_src = nullptr;
+    int64_t near_len = 0;  // length of near_leaf
 };
 
 template <typename T>
@@ -1655,7 +1658,9 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
     GX_TRY(dev_copy(hs, T.leaf_off, &fa.leaf_off));
     GX_TRY(dev_copy(hs, T.leaf_part, &fa.leaf_part));
     GX_TRY(dev_copy(hs, T.far_node, &fa.far_node));
-    GX_TRY(dev_copy(hs, T.near_off, &P.near_off));
+    GX_TRY(dev_copy(hs, T.near_off, &P.near_beg));
+    P.near_end = P.near_beg + 1;
+    P.near_len = P.n_near;
     GX_TRY(dev_copy(hs, T.near_leaf, &P.near_leaf));
     GX_TRY(mark(tm, 1, hs.st));
     GX_TRY(dev_array(hs, (int64_t)P.n_nodes * kFmmRec, &fa.rec));
@@ -1679,10 +1684,9 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
             M2PItem it;
             it.leaf = l;
             it.fb = fb + c * kM2PChunk;
-            it.fe = std::min(fe, it.fb + kM2PChunk);
+            it.count = std::min(fe - (int32_t)it.fb, (int32_t)kM2PChunk);
             it.chunk = c;
             it.nchunks = nch;
-            it.pad = 0;
             it.scratch = base;
             items.push_back(it);
         }
@@ -1691,8 +1695,8 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
         return fail(GX_ERR_UNSUPPORTED, "FMM: too many far-field work items");
     // largest items first (targets x nodes), as the device builder orders them
     std::stable_sort(items.begin(), items.end(), [&](const M2PItem& u, const M2PItem& v) {
-        const int64_t cu = (int64_t)(T.leaf_off[u.leaf + 1] - T.leaf_off[u.leaf]) * (u.fe - u.fb);
-        const int64_t cv = (int64_t)(T.leaf_off[v.leaf + 1] - T.leaf_off[v.leaf]) * (v.fe - v.fb);
+        const int64_t cu = (int64_t)(T.leaf_off[u.leaf + 1] - T.leaf_off[u.leaf]) * u.count;
+        const int64_t cv = (int64_t)(T.leaf_off[v.leaf + 1] - T.leaf_off[v.leaf]) * v.count;
         return cu > cv;
     });
     fa.n_items = (int32_t)items.size();
@@ -1701,6 +1705,9 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
     GX_TRY(mark(tm, 3, hs.st));
     return GX_OK;
 }
+
+// The list walk's stack: with gx_debug_fmm_tight_pools(2) so short that ordinary trees overflow it.
+int fmm_walk_stack() { return g_fmm_tight_pools.load() == 2 ? 64 : kWalkStackSlots; }
 
 // Device builder; *deep is set (and nothing else is valid) when the tree needs a split
 // below the key depth, which the host builder handles.
@@ -1807,48 +1814,71 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     GX_TRY(dev_array(hs, n, &la.leaf_part));
     GX_TRY(dev_array(hs, lb, &la.leaf_node));
     GX_TRY(dev_array(hs, lb, &la.node_leaf));
-    for (int32_t** p : {&la.far_cnt, &la.near_cnt, &la.item_cnt, &la.slot_cnt, &la.far_off, &la.near_off, &la.item_off,
-                        &la.slot_off})
+    for (int32_t** p : {&la.near_beg, &la.near_end, &la.near_src, &la.far_nch, &la.long_leaf, &la.long_head, &la.long_near,
+                        &la.slow_leaf})
         GX_TRY(dev_array(hs, lb, p));
-    GX_TRY(dev_array(hs, 6, &la.totals));
+    GX_TRY(dev_array(hs, lb, &la.far_slot));
+    GX_TRY(dev_array(hs, 1, &la.counters));
     GX_TRY(dev_array(hs, (int64_t)P.n_nodes, &la.wn));
     const size_t list_bytes = tree_list_temp_bytes(la.n, la.n_nodes);
     void* list_temp;
     GX_TRY(dev_array(hs, (int64_t)list_bytes, (char**)&list_temp));
-    GX_CUDA(launch_tree_lists_count(la, list_temp, list_bytes, st));
+    // Pools for the lists: a guess from the number of leaves and theta (a leaf of a two-disk system
+    // has 300 to 600 far nodes and 80 to 150 near leaves at theta 0.6, growing as theta falls); when
+    // it is too small, the totals tell what is needed and the lists are made again.
+    const double wide = std::min(8.0, std::max(1.0, 0.36 / (la.theta * la.theta)));
+    const int64_t leaf_bound = P.n_nodes - P.n_nodes / 8 + 1;
+    la.far_cap = (int64_t)(2.0 * wide * (double)leaf_bound) + 64;
+    la.near_cap = std::min<int64_t>((int64_t)(256.0 * wide * (double)leaf_bound) + 4096,
+                                    std::numeric_limits<int32_t>::max());
+    la.seg_cap = (int64_t)(wide * (double)leaf_bound / 16.0) + 256;
+    la.slot_cap = std::numeric_limits<int64_t>::max();
+    if (g_fmm_tight_pools.load()) la.far_cap = la.near_cap = la.seg_cap = 1;
+    la.walk_stack = fmm_walk_stack();
+    M2PItem* items;
     int32_t nl = 0;
-    unsigned long long tot[6];
+    ListCounters tot;
     for (int attempt = 0;; ++attempt) {
+        GX_TRY(dev_array(hs, la.far_cap * kM2PChunk, &la.far_node));
+        GX_TRY(dev_array(hs, la.far_cap, &items));
+        la.items = items;
+        GX_TRY(dev_array(hs, la.near_cap, &la.near_leaf));
+        GX_TRY(dev_array(hs, la.seg_cap * kNearSeg, &la.seg_near));
+        GX_TRY(dev_array(hs, la.seg_cap, &la.seg_next));
+        GX_TRY(dev_array(hs, la.seg_cap, &la.seg_count));
+        GX_CUDA(launch_tree_lists(la, list_temp, list_bytes, sm_count(dev), st));
         int m2m_err = 0;
         GX_CUDA(cudaMemcpyAsync(&nl, la.start_ord + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        GX_CUDA(cudaMemcpyAsync(tot, la.totals, sizeof(tot), cudaMemcpyDeviceToHost, st));
+        GX_CUDA(cudaMemcpyAsync(&tot, la.counters, sizeof(tot), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaMemcpyAsync(&m2m_err, m2m, sizeof(int), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaStreamSynchronize(st));
-        if (m2m_err == 0 || attempt == 1) break;
-        // a bounded wait of the one-launch upward pass gave up: the passes again, level by level
-        GX_CUDA(cudaMemsetAsync(m2m, 0, sizeof(int), st));
-        GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), hdr[1], st));
-        GX_CUDA(launch_tree_lists_count(la, list_temp, list_bytes, st));
-    }
-    for (int k = 0; k < 4; ++k)
-        if (tot[k] > (unsigned long long)std::numeric_limits<int32_t>::max())
+        if (m2m_err != 0 && attempt < 3) {
+            // a bounded wait of the one-launch upward pass gave up: the passes again, level by level
+            GX_CUDA(cudaMemsetAsync(m2m, 0, sizeof(int), st));
+            GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), hdr[1], st));
+            continue;
+        }
+        if (tot.far > (unsigned long long)std::numeric_limits<int32_t>::max() ||
+            tot.near > (unsigned long long)std::numeric_limits<int32_t>::max() ||
+            tot.chunks > (unsigned long long)std::numeric_limits<int32_t>::max())
             return fail(GX_ERR_UNSUPPORTED, "FMM: interaction lists exceed the int32 range");
-    P.far_pairs = (int64_t)tot[4];
-    P.near_pairs = (int64_t)tot[5];
+        if (tot.chunks <= (unsigned long long)la.far_cap && tot.near <= (unsigned long long)la.near_cap &&
+            tot.segs <= (unsigned long long)la.seg_cap)
+            break;
+        if (attempt == 4) return fail(GX_ERR_CUDA, "FMM: interaction lists keep outgrowing their pools");
+        la.far_cap = std::max<int64_t>(la.far_cap, (int64_t)tot.chunks);
+        la.near_cap = std::max<int64_t>(la.near_cap, (int64_t)tot.near);
+        la.seg_cap = std::max<int64_t>(la.seg_cap, (int64_t)tot.segs);
+    }
+    P.far_pairs = (int64_t)tot.far_pairs;
+    P.near_pairs = (int64_t)tot.near_pairs;
     P.n_leaves = fa.n_leaves = nl;
-    P.n_far = (int64_t)tot[0];
-    P.n_near = (int64_t)tot[1];
-    fa.n_items = (int32_t)tot[2];
-    P.n_slots = (int64_t)tot[3];
-    GX_TRY(dev_array(hs, P.n_far, &la.far_node));
-    GX_TRY(dev_array(hs, P.n_near, &la.near_key));
-    GX_TRY(dev_array(hs, (int64_t)nl, &la.long_leaf));
-    GX_TRY(dev_array(hs, 1, &la.long_count));
-    GX_TRY(dev_array(hs, P.n_near, &la.near_leaf));
-    M2PItem* items;
-    GX_TRY(dev_array(hs, fa.n_items, &items));
-    la.items = items;
-    GX_CUDA(launch_tree_lists_fill(la, nl, st));
+    P.n_far = (int64_t)tot.far;
+    P.n_near = (int64_t)tot.near;
+    P.n_chunks = (int64_t)tot.chunks;
+    fa.n_items = (int32_t)tot.chunks;
+    P.n_slots = (int64_t)tot.slots;
+    P.n_segs = (int64_t)tot.segs;
     // far-field items, largest first
     M2PItem* sorted_items;
     uint32_t *cost, *cost_alt;
@@ -1861,7 +1891,7 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     const size_t order_bytes = item_order_temp_bytes(fa.n_items);
     void* order_temp;
     GX_TRY(dev_array(hs, (int64_t)order_bytes, (char**)&order_temp));
-    GX_CUDA(launch_item_order(items, la.leaf_off, fa.n_items, nullptr, nullptr, cost, cost_alt, idx, idx_alt, order_temp, order_bytes,
+    GX_CUDA(launch_item_order(la, fa.n_items, nullptr, nullptr, cost, cost_alt, idx, idx_alt, order_temp, order_bytes,
                               sorted_items, st));
     items = sorted_items;
     GX_TRY(mark(tm, 3, st));
@@ -1869,8 +1899,11 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     fa.leaf_part = la.leaf_part;
     fa.far_node = la.far_node;
     fa.items = items;
-    P.near_off = la.near_off;
+    P.near_beg = la.near_beg;
+    P.near_end = la.near_end;
     P.near_leaf = la.near_leaf;
+    P.near_src = la.near_src;
+    P.near_len = la.near_cap;
     return GX_OK;
 }
 
@@ -1992,7 +2025,8 @@ int fmm_accel(const char* fn, int64_t n, const double* x, const double* y, const
 
         P2PArgs pa{};
         pa.x = dx; pa.y = dy; pa.z = dz; pa.m = dm;
-        pa.leaf_off = fa.leaf_off; pa.leaf_part = fa.leaf_part; pa.near_off = P->near_off; pa.near_leaf = P->near_leaf;
+        pa.leaf_off = fa.leaf_off; pa.leaf_part = fa.leaf_part; pa.near_beg = P->near_beg; pa.near_end = P->near_end; pa.near_leaf = P->near_leaf;
+        pa.near_src = P->near_src;
         pa.n_leaves = P->n_leaves;
         pa.ax = dax; pa.ay = day; pa.az = daz;
         pa.t_begin = begin;
@@ -2038,7 +2072,7 @@ struct FmmWork {
     gx_physics phys{};
     gx_fmm_options opt{};
     int32_t node_cap = 0;
-    int64_t far_cap = 0, near_cap = 0, item_cap = 0, slot_cap = 0;
+    int64_t far_cap = 0, near_cap = 0, seg_cap = 0, slot_cap = 0;  // chunks (= items), entries, segments, slots
     int32_t leaves_hint = 0;
     std::vector<void*> owned;
     TreeBuildArgs t{};
@@ -2062,7 +2096,7 @@ struct FmmWork {
     cudaStream_t aux = nullptr;
     cudaEvent_t fork0 = nullptr, fork = nullptr, join = nullptr;
     double* near = nullptr;
-    unsigned long long* need = nullptr;  // device: largest {nodes, far, near, items, slots, tree levels} seen
+    unsigned long long* need = nullptr;  // device: largest needs seen (TreeListArgs::need)
     int key_levels = 0;                  // levels of the path keys the tree sort orders
     ~FmmWork() {
         if (aux) {
@@ -2094,7 +2128,7 @@ int64_t with_headroom(int64_t v) { return g_fmm_tight_pools.load() ? std::max<in
 // so a tree two levels deeper still builds; a deeper one sets the overflow flag and the
 // chunk is redone with all levels.
 int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_fmm_options opt, int64_t nodes,
-                    int64_t leaves, int64_t far, int64_t near, int64_t items, int64_t slots, int key_levels,
+                    int64_t leaves, int64_t chunks, int64_t near, int64_t segs, int64_t slots, int key_levels,
                     cudaStream_t st) {
     W.reset(new FmmWork());
     FmmWork& w = *W;
@@ -2105,9 +2139,9 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     const int64_t cap = std::max<int64_t>(1, opt.leaf_capacity);
     const int64_t node_bound = 1 + 8 * (int64_t)kKeyLevels * (n / (cap + 1) + 1);
     w.node_cap = (int32_t)std::min<int64_t>({with_headroom(nodes), node_bound, (int64_t)0x7fff0000});
-    w.far_cap = with_headroom(far);
+    w.far_cap = std::min<int64_t>(with_headroom(chunks), 0x7fff0000);
     w.near_cap = with_headroom(near);
-    w.item_cap = std::min<int64_t>(with_headroom(items), 0x7fff0000);
+    w.seg_cap = with_headroom(segs);
     w.slot_cap = with_headroom(slots);
     w.leaves_hint = (int32_t)std::max<int64_t>(1, leaves);
     const int32_t NC = w.node_cap;
@@ -2131,7 +2165,7 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     w.tree_bytes = tree_build_temp_bytes(t.n, cap);
     GX_TRY(w.grab((int64_t)w.tree_bytes, (char**)&w.tree_temp));
     GX_TRY(w.grab(2, &w.flags));
-    GX_TRY(w.grab(6, &w.need));
+    GX_TRY(w.grab(kNeed, &w.need));
     GX_TRY(w.grab((int64_t)fmm_octets(NC), &w.m2m_ready));
     GX_TRY(w.grab(1, &w.m2m_ticket));
     GX_TRY(w.grab(3 * n, &w.near));
@@ -2177,33 +2211,35 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     la.far_cap = w.far_cap;
     la.near_cap = w.near_cap;
     GX_TRY(w.grab(n + 1, &la.mprefix));
-    la.item_cap = w.item_cap;
+    la.seg_cap = w.seg_cap;
+    la.walk_stack = fmm_walk_stack();
     la.slot_cap = w.slot_cap;
     for (int32_t** q : {&la.start_flag, &la.start_ord, &la.keep, &la.newpos}) GX_TRY(w.grab(n + 1, q));
     GX_TRY(w.grab((int64_t)NC + 1, &la.leaf_off));
     GX_TRY(w.grab(n, &la.leaf_part));
     GX_TRY(w.grab((int64_t)NC + 1, &la.leaf_node));
     GX_TRY(w.grab((int64_t)NC + 1, &la.node_leaf));
-    for (int32_t** q : {&la.far_cnt, &la.near_cnt, &la.item_cnt, &la.slot_cnt, &la.far_off, &la.near_off,
-                        &la.item_off, &la.slot_off})
+    for (int32_t** q : {&la.near_beg, &la.near_end, &la.near_src, &la.far_nch, &la.long_leaf, &la.long_head, &la.long_near,
+                        &la.slow_leaf})
         GX_TRY(w.grab((int64_t)NC + 1, q));
-    GX_TRY(w.grab(6, &la.totals));
+    GX_TRY(w.grab((int64_t)NC + 1, &la.far_slot));
+    GX_TRY(w.grab(1, &la.counters));
     GX_TRY(w.grab(NC, &la.wn));
     w.list_bytes = tree_list_temp_bytes(la.n, NC);
     GX_TRY(w.grab((int64_t)w.list_bytes, (char**)&w.list_temp));
-    GX_TRY(w.grab(w.far_cap, &la.far_node));
-    GX_TRY(w.grab(w.near_cap, &la.near_key));
+    GX_TRY(w.grab(w.far_cap * kM2PChunk, &la.far_node));
     GX_TRY(w.grab(w.near_cap, &la.near_leaf));
-    GX_TRY(w.grab((int64_t)NC, &la.long_leaf));
-    GX_TRY(w.grab(1, &la.long_count));
-    GX_TRY(w.grab(w.item_cap, &w.items));
+    GX_TRY(w.grab(w.seg_cap * kNearSeg, &la.seg_near));
+    GX_TRY(w.grab(w.seg_cap, &la.seg_next));
+    GX_TRY(w.grab(w.seg_cap, &la.seg_count));
+    GX_TRY(w.grab(w.far_cap, &w.items));
     la.items = w.items;
-    GX_TRY(w.grab(w.item_cap, &w.sorted));
-    GX_TRY(w.grab(w.item_cap, &w.cost));
-    GX_TRY(w.grab(w.item_cap, &w.cost_alt));
-    GX_TRY(w.grab(w.item_cap, &w.idx));
-    GX_TRY(w.grab(w.item_cap, &w.idx_alt));
-    w.order_bytes = item_order_temp_bytes((int32_t)w.item_cap);
+    GX_TRY(w.grab(w.far_cap, &w.sorted));
+    GX_TRY(w.grab(w.far_cap, &w.cost));
+    GX_TRY(w.grab(w.far_cap, &w.cost_alt));
+    GX_TRY(w.grab(w.far_cap, &w.idx));
+    GX_TRY(w.grab(w.far_cap, &w.idx_alt));
+    w.order_bytes = item_order_temp_bytes((int32_t)w.far_cap);
     GX_TRY(w.grab((int64_t)w.order_bytes, (char**)&w.order_temp));
 
     fa.n_leaves = NC;
@@ -2212,14 +2248,14 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     fa.leaf_part = la.leaf_part;
     fa.far_node = la.far_node;
     fa.items = w.sorted;
-    fa.n_items = (int32_t)w.item_cap;
-    fa.cnt_items = la.totals + 2;
+    fa.n_items = (int32_t)w.far_cap;
+    fa.cnt_items = &la.counters->chunks;
     fa.overflow = w.flags;
     GX_TRY(w.grab(w.slot_cap * 3, &fa.scratch));
     GX_TRY(w.grab(NC, &fa.done));
     GX_TRY(w.grab((int64_t)p2p_scratch_bytes(n, NC), (char**)&w.p2p_scratch));
     GX_CUDA(cudaMemsetAsync(w.flags, 0, 2 * sizeof(int), st));
-    GX_CUDA(cudaMemsetAsync(w.need, 0, 6 * sizeof(unsigned long long), st));
+    GX_CUDA(cudaMemsetAsync(w.need, 0, kNeed * sizeof(unsigned long long), st));
     return GX_OK;
 }
 
@@ -2252,11 +2288,10 @@ int fmm_work_enqueue(FmmWork& w, const double* x, const double* y, const double*
     TreeListArgs& la = w.la;
     la.m = m;
     GX_CUDA(launch_tree_massive(la, w.list_temp, w.list_bytes, st));
-    GX_CUDA(launch_tree_lists_count(la, w.list_temp, w.list_bytes, st));
+    GX_CUDA(launch_tree_lists(la, w.list_temp, w.list_bytes, sm_count(dev), st));
     GX_CUDA(launch_pool_check(la, t.hdr, st));
-    GX_CUDA(launch_tree_lists_fill(la, w.node_cap, st));
-    GX_CUDA(launch_item_order(w.items, la.leaf_off, (int32_t)w.item_cap, la.totals + 2, w.flags, w.cost, w.cost_alt,
-                              w.idx, w.idx_alt, w.order_temp, w.order_bytes, w.sorted, st));
+    GX_CUDA(launch_item_order(la, (int32_t)w.far_cap, &la.counters->chunks, w.flags, w.cost, w.cost_alt, w.idx, w.idx_alt,
+                              w.order_temp, w.order_bytes, w.sorted, st));
     GX_CUDA(cudaEventRecord(w.fork, st));
     GX_CUDA(cudaStreamWaitEvent(w.aux, w.fork, 0));
     for (double* p : {ax, ay, az}) GX_CUDA(cudaMemsetAsync(p, 0, (size_t)n * sizeof(double), w.aux));
@@ -2274,7 +2309,8 @@ int fmm_work_enqueue(FmmWork& w, const double* x, const double* y, const double*
     double* nz = side ? w.near + 2 * n : az;
     P2PArgs pa{};
     pa.x = x; pa.y = y; pa.z = z; pa.m = m;
-    pa.leaf_off = la.leaf_off; pa.leaf_part = la.leaf_part; pa.near_off = la.near_off; pa.near_leaf = la.near_leaf;
+    pa.leaf_off = la.leaf_off; pa.leaf_part = la.leaf_part; pa.near_beg = la.near_beg; pa.near_end = la.near_end; pa.near_leaf = la.near_leaf;
+    pa.near_src = la.near_src;
     pa.n_leaves = w.node_cap;
     pa.cnt_leaves = la.start_ord + n;
     pa.overflow = w.flags;
@@ -2305,8 +2341,8 @@ int session_fmm_size(gx_session* s, bool* device_ok) {
     *device_ok = !deep;
     if (deep) return GX_OK;
     std::unique_ptr<FmmWork> W;
-    GX_TRY(fmm_work_create(W, s->n, s->phys, s->fmm_opt, P->n_nodes, P->n_leaves, P->n_far, P->n_near,
-                           P->fa.n_items, P->n_slots,
+    GX_TRY(fmm_work_create(W, s->n, s->phys, s->fmm_opt, P->n_nodes, P->n_leaves, P->n_chunks, P->n_near,
+                           P->n_segs, P->n_slots,
                            g_fmm_tight_pools.load() ? 1 : (int)P->level_off.size() - 1 + 2, s->stream));
     fmm_work_release(s->fmm);
     s->fmm = W.release();
@@ -2318,15 +2354,15 @@ int session_fmm_size(gx_session* s, bool* device_ok) {
 // again larger than before.
 int session_fmm_regrow(gx_session* s) {
     FmmWork& w = *s->fmm;
-    unsigned long long need[6];
+    unsigned long long need[kNeed];
     GX_CUDA(cudaMemcpyAsync(need, w.need, sizeof(need), cudaMemcpyDeviceToHost, s->stream));
     GX_CUDA(cudaStreamSynchronize(s->stream));
     std::unique_ptr<FmmWork> W;
     GX_TRY(fmm_work_create(W, s->n, s->phys, s->fmm_opt, std::max<int64_t>((int64_t)need[0], w.node_cap),
                            w.leaves_hint, std::max<int64_t>((int64_t)need[1], w.far_cap),
-                           std::max<int64_t>((int64_t)need[2], w.near_cap), std::max<int64_t>((int64_t)need[3], w.item_cap),
-                           std::max<int64_t>((int64_t)need[4], w.slot_cap),
-                           std::max(w.key_levels, (int)std::min<unsigned long long>(need[5], kKeyLevels) + 2), s->stream));
+                           std::max<int64_t>((int64_t)need[2], w.near_cap), std::max<int64_t>((int64_t)need[5], w.seg_cap),
+                           std::max<int64_t>((int64_t)need[3], w.slot_cap),
+                           std::max(w.key_levels, (int)std::min<unsigned long long>(need[4], kKeyLevels) + 2), s->stream));
     fmm_work_release(s->fmm);
     s->fmm = W.release();
     s->clear_graphs();
@@ -2534,20 +2570,25 @@ extern "C" int gxi_leaf_lists_from_device(int64_t n, const double* x, const doub
     *on_device = P->on_device ? 1 : 0;
     const int32_t nl = P->n_leaves;
     T->leaf_off.resize((size_t)nl + 1);
-    T->near_off.resize((size_t)nl + 1);
-    GX_CUDA(cudaMemcpyAsync(T->leaf_off.data(), P->fa.leaf_off, T->leaf_off.size() * sizeof(int32_t),
-                            cudaMemcpyDeviceToHost, st));
-    GX_CUDA(cudaMemcpyAsync(T->near_off.data(), P->near_off, T->near_off.size() * sizeof(int32_t),
-                            cudaMemcpyDeviceToHost, st));
+    T->near_off.assign((size_t)nl + 1, 0);
+    std::vector<int32_t> beg((size_t)nl), end((size_t)nl), near((size_t)P->near_len);
+    auto fetch = [&](std::vector<int32_t>& v, const int32_t* d) -> int {
+        if (!v.empty()) GX_CUDA(cudaMemcpyAsync(v.data(), d, v.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        return GX_OK;
+    };
+    GX_TRY(fetch(T->leaf_off, P->fa.leaf_off));
+    GX_TRY(fetch(beg, P->near_beg));
+    GX_TRY(fetch(end, P->near_end));
+    GX_TRY(fetch(near, P->near_leaf));
     GX_CUDA(cudaStreamSynchronize(st));
     T->leaf_part.resize((size_t)T->leaf_off[nl]);
-    T->near_leaf.resize((size_t)P->n_near);
-    if (!T->leaf_part.empty())
-        GX_CUDA(cudaMemcpyAsync(T->leaf_part.data(), P->fa.leaf_part, T->leaf_part.size() * sizeof(int32_t),
-                                cudaMemcpyDeviceToHost, st));
-    if (!T->near_leaf.empty())
-        GX_CUDA(cudaMemcpyAsync(T->near_leaf.data(), P->near_leaf, T->near_leaf.size() * sizeof(int32_t),
-                                cudaMemcpyDeviceToHost, st));
+    GX_TRY(fetch(T->leaf_part, P->fa.leaf_part));
+    T->near_leaf.clear();
+    T->near_leaf.reserve((size_t)P->n_near);
+    for (int32_t l = 0; l < nl; ++l) {  // the device's lists lie in any order
+        T->near_leaf.insert(T->near_leaf.end(), near.begin() + beg[(size_t)l], near.begin() + end[(size_t)l]);
+        T->near_off[(size_t)l + 1] = (int32_t)T->near_leaf.size();
+    }
     GX_CUDA(cudaStreamSynchronize(st));
     T->n_far = P->n_far;
     T->n_pairs = 0;

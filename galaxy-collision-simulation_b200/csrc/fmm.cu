@@ -511,7 +511,8 @@ __global__ void __launch_bounds__(kM2PBlock) fmm_m2p_kernel(const FmmArgs a) {
     const int n_items = fmm_items(a);
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
         const M2PItem w = a.items[it];
-        const int cnt = w.fe - w.fb;
+        if (w.leaf < 0) continue;
+        const int cnt = w.count;
         const int tb = a.leaf_off[w.leaf], nt = a.leaf_off[w.leaf + 1] - tb;
         const int W = min(nt, kM2PBlock);
         const int S = kM2PBlock / W;

@@ -26,11 +26,11 @@ constexpr int kRec32 = 52;
 
 // Far-field work item: one target leaf and a chunk of its far list.
 struct M2PItem {
-    int32_t leaf;
-    int32_t fb, fe;   // far_node[fb .. fe)
+    int32_t leaf;     // -1: a chunk that was given up (skipped)
     int32_t chunk;    // index of this chunk among the leaf's chunks
     int32_t nchunks;
-    int32_t pad;
+    int32_t count;
+    int64_t fb;       // far_node[fb .. fb + count)
     int64_t scratch;  // first partial-sum slot of the leaf (targets), when nchunks > 1
 };
 

@@ -17,17 +17,16 @@
 // Nodes are numbered breadth-first.  Trees that need a split below level 21 (more than
 // leaf_capacity nearly coincident bodies) are reported back for the host builder.
 //
-// Lists: every leaf with mass > 0 is walked with the reference's tests (mass > 0,
-// well_separated, leaf) by one warp over a shared-memory stack; a count pass, exclusive
-// sums, and a fill pass (near lists sorted into the reference's depth-first order).
+// Lists: every leaf with mass > 0 is walked once with the reference's tests (mass > 0,
+// well_separated, leaf) by one warp over a shared-memory stack; far nodes go straight into
+// chunks of a pool (one far-field work item each), near leaves into a buffer that is sorted into the
+// reference's depth-first order.
 #include "fmm_build.cuh"
 #include "fmm.cuh"
 #include "gx_device.cuh"
 
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
-#include <thrust/iterator/zip_iterator.h>
-#include <thrust/tuple.h>
 
 #include <algorithm>
 #include <cfloat>
@@ -37,16 +36,16 @@ namespace {
 
 constexpr int kBboxThreads = 256;
 constexpr int kWalkThreads = 128;  // 4 warps, one leaf each
-// Shared stack slots per warp: 4 x 1024 x 4 B = 16 KiB per block, plus the 1 KiB the
-// runtime reserves per block: 8 blocks (32 warps, the count __launch_bounds__(kWalkThreads, 8)
-// sizes the registers for) take 136 KiB, inside the 60% shared-memory carveout walk_kernel
-// asks for; the rest of the SM's unified memory stays L1 for the node-record loads (measured
-// against 1760 slots at the largest carveout: lists phase 13% faster at N=2^20, leaf 16).
+// Slots of a warp's shared buffer: its stack grows from the bottom (up to kWalkStack), the near
+// leaves it has met from the top (up to kWalkNear).  4 x 1152 x 4 B = 18 KiB per block, plus the
+// 1 KiB the runtime reserves: 8 blocks (32 warps, the count __launch_bounds__(kWalkThreads, 8)
+// sizes the registers for) take 152 KiB, inside the 70% shared-memory carveout asked for; the
+// rest of the SM's unified memory stays L1 for the node-record loads.
+constexpr int kWalkSlots = 1152;
 constexpr int kWalkStack = 1024;
-// near lists up to this many entries are sorted in the warp's stack buffer (a bitonic network
-// pads to a power of two, so the largest power of two that fits kWalkStack / 2 keys)
-constexpr int pow2_floor(int v) { return v < 2 ? v : 2 * pow2_floor(v / 2); }
-constexpr int kSortCap = pow2_floor(kWalkStack / 2);
+constexpr int kWalkNear = 512;
+static_assert(kWalkNear == kNearSeg, "a full buffer is one segment");
+static_assert(kWalkStack == kWalkStackSlots, "the host's bound of the stack");
 constexpr int kStack = 7 * (kKeyLevels + 1) + 8;
 
 __global__ void __launch_bounds__(kBboxThreads) bbox_partial_kernel(const TreeBuildArgs t) {
@@ -392,10 +391,9 @@ __global__ void __launch_bounds__(256) walk_pack_kernel(const TreeListArgs a) {
     w.cy = a.cy[k];
     w.cz = a.cz[k];
     w.hw = a.hw[k];
-    w.mass = node_massive(a, k) ? 1.0 : 0.0;  // the walk only asks whether it is > 0
     w.child = a.child[k];
-    w.beg = a.beg[k];
-    w.end = a.end[k];
+    w.count = a.end[k] - a.beg[k];
+    w.leaf = w.child < 0 && node_massive(a, k) ? a.node_leaf[k] : -1;
     w.mask = 0;
     if (w.child >= 0)
         for (int c = 0; c < 8; ++c) w.mask |= (node_massive(a, w.child + c) ? 1 : 0) << c;
@@ -404,321 +402,548 @@ __global__ void __launch_bounds__(256) walk_pack_kernel(const TreeListArgs a) {
 
 // well_separated (fmm_solver.cpp:228-241): 2 (hw_t + hw_s) / dist < theta, dist != 0, with
 // the reference's operations.  The reference's quotient is within 1.5 ulp of the exact
-// num / sqrt(r2), so wherever num^2 and theta^2 r2 (each within a few ulp) differ by more
-// than 1e-12 relative the squares give the same answer without the square root and the
-// division; only near-ties, and magnitudes where the squares could overflow or underflow,
-// take the reference's own operations.
-__device__ __forceinline__ bool well_separated(const WalkNode& T, const WalkNode& S, double theta) {
-    const double dx = dsub(S.cx, T.cx), dy = dsub(S.cy, T.cy), dz = dsub(S.cz, T.cz);
-    const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-    if (r2 == 0.0) return false;  // dist == 0
-    const double num = dmul(2.0, dadd(T.hw, S.hw));
-    const double lhs = dmul(num, num), rhs = dmul(dmul(theta, theta), r2);
-    if (theta > 0.0 && rhs > 1e-290 && rhs < 1e290 && lhs < 1e290) {
-        if (lhs < dmul(rhs, 1.0 - 1e-12)) return true;
-        if (lhs > dmul(rhs, 1.0 + 1e-12)) return false;
+// num / sqrt(r2), so wherever (hw_t + hw_s)^2 and theta^2 r2 / 4 (each within a few ulp) differ by
+// more than 1e-12 relative the squares give the same answer without the square root and the
+// division; only near-ties take the reference's own operations.  So do all nodes of a tree whose
+// extent or theta could make the squares overflow or underflow (SeparationTest::squares).
+struct SeparationTest {
+    double theta, lo, hi;  // theta^2 / 4 times 1 -+ 1e-12
+    bool squares;
+    __device__ __forceinline__ SeparationTest(double th, double root_hw) : theta(th) {
+        const double q = dmul(dmul(th, th), 0.25);
+        lo = dmul(q, 1.0 - 1e-12);
+        hi = dmul(q, 1.0 + 1e-12);
+        // cells are at least root_hw 2^-32 wide (max_depth bounds the tree on the device at 21)
+        squares = th > 1e-50 && th < 1e50 && root_hw > 1e-60 && root_hw < 1e60;
     }
-    return __ddiv_rn(num, __dsqrt_rn(r2)) < theta;
+    __device__ __forceinline__ bool operator()(const WalkNode& T, const WalkNode& S) const {
+        const double dx = dsub(S.cx, T.cx), dy = dsub(S.cy, T.cy), dz = dsub(S.cz, T.cz);
+        const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+        const double w = dadd(T.hw, S.hw);
+        if (squares) {
+            const double w2 = dmul(w, w);
+            if (w2 < dmul(lo, r2)) return true;
+            if (w2 > dmul(hi, r2)) return false;
+        }
+        if (r2 == 0.0) return false;  // dist == 0
+        return __ddiv_rn(dmul(2.0, w), __dsqrt_rn(r2)) < theta;
+    }
+};
+
+__device__ __forceinline__ WalkNode load_walk_node(const WalkNode* wn, int s) {
+    WalkNode r;
+    const double2* q = reinterpret_cast<const double2*>(wn + s);
+    const double2 a0 = q[0], a1 = q[1];
+    const int4 a2 = *reinterpret_cast<const int4*>(q + 2);
+    r.cx = a0.x; r.cy = a0.y; r.cz = a1.x; r.hw = a1.y;
+    r.child = a2.x; r.mask = a2.y; r.leaf = a2.z; r.count = a2.w;
+    return r;
 }
 
-// One node of the walk (build_leaf_interactions, fmm_solver.cpp:254-277): 1 far, 2 near,
-// 3 expand, 0 massless.
-__device__ __forceinline__ int classify(const WalkNode& T, int t, const WalkNode& S, int s, double theta) {
-    if (!(S.mass > 0.0)) return 0;
-    if (s != t && well_separated(T, S, theta)) return 1;
-    return S.child < 0 ? 2 : 3;
-}
-
-// One warp sorts the distinct keys v[0 .. n) ascending and writes the low 32 bits of each to
-// out in that order: a bitonic sort in the shared buffer buf (kWalkStack / 2 slots) when the
-// list fits, else every key's rank (the number of smaller keys) computed from global memory.
-__device__ void sort_into(const uint64_t* v, int n, uint64_t* buf, int lane, int32_t* out) {
-    if (n <= kSortCap) {
-        int P = 1;
-        while (P < n) P <<= 1;
-        for (int i = lane; i < P; i += 32) buf[i] = i < n ? v[i] : ~0ull;
-        __syncwarp();
-        for (int k = 2; k <= P; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = lane; i < P; i += 32) {
-                    const int m = i ^ j;
-                    if (m > i) {
-                        const uint64_t x = buf[i], y = buf[m];
-                        if ((x > y) == ((i & k) == 0)) {
-                            buf[i] = y;
-                            buf[m] = x;
-                        }
-                    }
-                }
-                __syncwarp();
+// One warp sorts n <= 32 K distinct values of src (shared memory, any order) ascending into dst,
+// by way of the 32 K words of tmp (shared, apart from src): a bitonic network in registers, K
+// neighbours per lane, its compare-exchanges across lanes by shuffle.
+template <int K>
+__device__ __forceinline__ void warp_sort(const uint32_t* src, uint32_t* tmp, int n, int lane, int32_t* dst) {
+    uint32_t v[K];
+#pragma unroll
+    for (int r = 0; r < K; ++r) v[r] = r * 32 + lane < n ? src[r * 32 + lane] : 0xffffffffu;
+    auto exchange = [](uint32_t& x, uint32_t& y, bool up) {  // x before y
+        const uint32_t lo = min(x, y), hi = max(x, y);
+        x = up ? lo : hi;
+        y = up ? hi : lo;
+    };
+    // runs of up to K inside a lane
+    if constexpr (K > 1) {
+#pragma unroll
+        for (int k = 2; k <= K; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+                for (int r = 0; r < K; ++r)
+                    if ((r & j) == 0) exchange(v[r], v[r | j], k < K ? (r & k) == 0 : (lane & 1) == 0);
+    }
+    for (int k = 2; k <= 32; k <<= 1) {  // runs of k lanes
+        const bool up = (lane & k) == 0;
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const bool low = (lane & j) == 0;
+#pragma unroll
+            for (int r = 0; r < K; ++r) {
+                const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], j);
+                v[r] = low == up ? min(v[r], o) : max(v[r], o);
             }
-        for (int i = lane; i < n; i += 32) out[i] = (int32_t)(uint32_t)buf[i];
-        __syncwarp();
+        }
+        if constexpr (K > 1) {
+#pragma unroll
+            for (int j = K >> 1; j > 0; j >>= 1)
+#pragma unroll
+                for (int r = 0; r < K; ++r)
+                    if ((r & j) == 0) exchange(v[r], v[r | j], up);
+        }
+    }
+    if (K == 1) {
+        if (lane < n) dst[lane] = (int32_t)v[0];
         return;
     }
-    for (int i = lane; i < n; i += 32) {
-        const uint64_t key = v[i];
-        int r = 0;
-        for (int q = 0; q < n; ++q) r += v[q] < key;
-        out[r] = (int32_t)(uint32_t)key;
-    }
+#pragma unroll
+    for (int r = 0; r < K; ++r) tmp[lane * K + r] = v[r];
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) dst[i] = (int32_t)tmp[i];
+    __syncwarp();
 }
 
-// Every leaf with mass > 0, one warp each: the walk of build_leaf_interactions from the
-// root, with a shared-memory stack the warp pops 32 nodes at a time (each lane classifies
-// one node; expanded nodes push their children with mass > 0).  The fill pass writes each far node
-// where the walk meets it (the far list holds the reference's nodes in the walk's own,
-// deterministic order; only the summation order of the far field depends on it) and each
-// near leaf as its ordinal, then sorts the near list into the reference's depth-first order
-// (leaf ordinals are depth-first numbers), which the near field's exact form relies on.  When the stack would overflow, every lane finishes its share of
-// the pending nodes depth first with a private stack.
-template <bool FILL>
+// The far list of one leaf in the making (uniform over the warp): chunks are reserved as they are
+// needed, the full ones entered as work items.
+struct FarChunks {
+    int leaf;
+    bool wanted;               // the leaf has a target in range
+    int64_t chunk = -1;        // current chunk
+    int fill = kM2PChunk;      // entries in it (full: the next entry opens a chunk)
+    int nch = 0;
+    int count = 0;             // entries met
+
+    __device__ __forceinline__ void close(const TreeListArgs& a, int lane) {
+        if (chunk < 0) return;
+        if (lane == 0 && chunk < a.far_cap) {
+            M2PItem it;
+            it.leaf = leaf;
+            it.chunk = nch;
+            it.nchunks = 0;  // entered with the item order, like scratch
+            it.count = fill;
+            it.fb = chunk * kM2PChunk;
+            it.scratch = 0;
+            ((M2PItem*)a.items)[chunk] = it;
+        }
+        ++nch;
+    }
+    // Lanes of mask m append their node s, in lane order.
+    __device__ __forceinline__ void append(const TreeListArgs& a, unsigned m, int lane, int s) {
+        if (m == 0) return;
+        const int k = __popc(m), pos = fill + __popc(m & ((1u << lane) - 1u));
+        count += k;
+        if (!wanted) return;
+        int64_t next = chunk;
+        if (fill + k > kM2PChunk) {
+            unsigned long long c = 0;
+            if (lane == 0) c = atomicAdd(&a.counters->chunks, 1ull);
+            next = (int64_t)__shfl_sync(0xffffffffu, c, 0);
+        }
+        if (m >> lane & 1u) {
+            const int64_t c = pos < kM2PChunk ? chunk : next;
+            if (c < a.far_cap) a.far_node[c * kM2PChunk + (pos & (kM2PChunk - 1))] = s;
+        }
+        if (fill + k > kM2PChunk) {
+            const int left = fill + k - kM2PChunk;
+            fill = kM2PChunk;
+            close(a, lane);
+            chunk = next;
+            fill = left;
+        } else {
+            fill += k;
+        }
+    }
+};
+static_assert((kM2PChunk & (kM2PChunk - 1)) == 0, "positions wrap by mask");
+
+__device__ __forceinline__ bool leaf_in_range(const TreeListArgs& a, int tb, int te, int lane) {
+    if (a.t_begin <= 0 && a.t_end >= a.n) return true;
+    bool any = false;
+    for (int k = tb + lane; k < te; k += 32) any |= a.leaf_part[k] >= a.t_begin && a.leaf_part[k] < a.t_end;
+    return __any_sync(0xffffffffu, any);
+}
+
+// Totals a warp has met, added to the counters once at its end.
+struct WalkTotals {
+    unsigned long long far = 0, far_pairs = 0, near_pairs = 0;
+    __device__ __forceinline__ void flush(const TreeListArgs& a, int lane) const {
+        if (lane != 0 || far + near_pairs == 0) return;
+        atomicAdd(&a.counters->far, far);
+        atomicAdd(&a.counters->far_pairs, far_pairs);
+        atomicAdd(&a.counters->near_pairs, near_pairs);
+    }
+};
+
+// The leaf's list sizes, once its far chunks are closed (lane 0); those of slow_walk_kernel's leaves
+// carry a minus sign, as its items do: the chunks walk_kernel had begun for such a leaf are void.
+__device__ __forceinline__ void leaf_done(const TreeListArgs& a, int l, int targets, int nf, int nch, bool slow, int nsrc,
+                                          WalkTotals& tot) {
+    a.far_nch[l] = slow ? -nch : nch;
+    a.far_slot[l] = nch > 1 ? (int64_t)atomicAdd(&a.counters->slots, (unsigned long long)nch * targets) : 0;
+    a.near_src[l] = nsrc;
+    tot.far += nf;
+    tot.far_pairs += (unsigned long long)nf * targets;
+    tot.near_pairs += (unsigned long long)nsrc * targets;
+}
+
+// A place for the n near leaves of leaf l (lane 0); past the pool: an empty list.
+__device__ __forceinline__ int near_place(const TreeListArgs& a, int l, int n) {
+    const unsigned long long b = atomicAdd(&a.counters->near, (unsigned long long)n);
+    const bool ok = (int64_t)b + n <= a.near_cap;
+    a.near_beg[l] = ok ? (int32_t)b : 0;
+    a.near_end[l] = ok ? (int32_t)b + n : 0;
+    return ok ? (int)b : -1;
+}
+
+// Every leaf with mass > 0, one warp each (leaves taken from a ticket): the walk of
+// build_leaf_interactions (fmm_solver.cpp:254-277) from the root, with a shared-memory stack the
+// warp pops 32 nodes at a time (each lane classifies one node; expanded nodes push their children
+// with mass > 0; the massless ones would be skipped).  Far nodes are written where the walk meets
+// them (the far list holds the reference's nodes in the walk's own, deterministic order; only the
+// summation order of the far field depends on it).  Near leaves are collected as ordinals, then
+// sorted into the reference's depth-first order (leaf ordinals are depth-first numbers), which
+// the near field's exact form relies on; a list longer than the buffer goes to linked segments and
+// long_near_kernel.  A leaf whose stack would overflow is left to slow_walk_kernel.
+// Bound by the latency of a pop (its node records, the test, the pushes) and, for small trees, by
+// the few leaves with thousands of nodes to visit.  N = 65,536 leaf 64 86 us, N = 2^20 leaf 16
+// 2.2 ms, against 197 us and 5.0 ms for a count and a fill walk with 56-byte records, near lists
+// sorted in shared memory and each leaf's totals added by atomics.
 __global__ void __launch_bounds__(kWalkThreads, 8) walk_kernel(const TreeListArgs a) {
     constexpr int W = kWalkThreads / 32;
-    __shared__ __align__(16) int s_stk[W][kWalkStack];
-    if (FILL && a.overflow && *a.overflow) return;
+    __shared__ __align__(16) int s_buf[W][kWalkSlots];
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int l = blockIdx.x * W + wid;
     const int n_leaves = a.start_ord[a.n];
-    if (l >= n_leaves) return;
-    const int t = a.leaf_node[l];
-    const WalkNode T = a.wn[t];
-    const int fo = FILL ? a.far_off[l] : 0, no = FILL ? a.near_off[l] : 0;
     const unsigned lt = (1u << lane) - 1u;
-    int* stk = s_stk[wid];
-    int nf = 0, nn = 0, top = 1, pend = -1, pmask = 0, pchild = 0;
-    long long nsrc = 0;  // count pass: bodies of the near leaves found by this lane
+    int* const stk = s_buf[wid];
+    const SeparationTest separated(a.theta, n_leaves > 0 ? a.hw[0] : 0.0);
+    // consecutive leaves share most of their nodes: a warp takes four at a time when there are many
+    const int batch = n_leaves > 8 * W * (int)gridDim.x ? 4 : 1;
+    WalkTotals tot;
+    for (;;) {
+        int l0 = 0;
+        if (lane == 0) l0 = atomicAdd(&a.counters->ticket, batch);
+        l0 = __shfl_sync(0xffffffffu, l0, 0);
+        if (l0 >= n_leaves) break;
+        for (int l = l0; l < min(l0 + batch, n_leaves); ++l) {
+            const int t = a.leaf_node[l];
+            const WalkNode T = load_walk_node(a.wn, t);
+            const int tb = a.leaf_off[l], te = a.leaf_off[l + 1];
+            FarChunks far;
+            far.leaf = l;
+            far.wanted = leaf_in_range(a, tb, te, lane);
+            int nn = 0, nb = 0, head = -1, top = 1;  // near leaves met, of them in the buffer, segments
+            int nsrc = 0;  // bodies of the near leaves this lane met
+            bool slow = false;
+            // the nb near leaves of the buffer into a new segment
+            auto flush_near = [&] {
+                unsigned long long c = 0;
+                if (lane == 0) c = atomicAdd(&a.counters->segs, 1ull);
+                const int64_t seg = (int64_t)__shfl_sync(0xffffffffu, c, 0);
+                if (seg < a.seg_cap) {
+                    for (int i = lane; i < nb; i += 32) a.seg_near[seg * kNearSeg + i] = stk[kWalkSlots - 1 - i];
+                    if (lane == 0) {
+                        a.seg_next[seg] = head;
+                        a.seg_count[seg] = nb;
+                    }
+                    head = (int)seg;
+                }
+                __syncwarp();
+                nb = 0;
+            };
+            __syncwarp();
+            if (lane == 0) stk[0] = 0;
+            __syncwarp();
+            while (top > 0) {
+                const int take = min(32, top), base = top - take;
+                const bool in = lane < take;
+                const int s = in ? stk[base + lane] : t;
+                const WalkNode S = load_walk_node(a.wn, s);
+                const bool is_far = in && s != t && separated(T, S);
+                const bool is_near = in && !is_far && S.child < 0;
+                const int m = in && !is_far && !is_near ? S.mask : 0;
+                const unsigned mf = __ballot_sync(0xffffffffu, is_far);
+                const unsigned mn = __ballot_sync(0xffffffffu, is_near);
+                far.append(a, mf, lane, s);
+                // children to push: prefix sums of the lanes' counts (0..8) from four ballots
+                const int mine = __popc(m);
+                const unsigned b0 = __ballot_sync(0xffffffffu, mine & 1), b1 = __ballot_sync(0xffffffffu, mine & 2);
+                const unsigned b2 = __ballot_sync(0xffffffffu, mine & 4), b3 = __ballot_sync(0xffffffffu, mine & 8);
+                const int add = __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2) + 8 * __popc(b3);
+                const int at = base + __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt) + 8 * __popc(b3 & lt);
+                if (base + add > a.walk_stack) {
+                    slow = true;
+                    break;
+                }
+                top = base + add;
+                const int kn = __popc(mn);
+                if (kn > 0 && (nb + kn > kWalkNear || top + nb + kn > kWalkSlots)) flush_near();
+                else if (top + nb > kWalkSlots) flush_near();
+                if (is_near) {
+                    stk[kWalkSlots - 1 - nb - __popc(mn & lt)] = S.leaf;
+                    nsrc += S.count;
+                }
+                nb += kn;
+                nn += kn;
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if (m >> c & 1) stk[at + __popc(m >> (c + 1))] = S.child + c;
+                __syncwarp();
+            }
+            far.close(a, lane);
+            if (slow) {
+                if (lane == 0) a.slow_leaf[atomicAdd(&a.counters->n_slow, 1)] = l;
+                continue;
+            }
+            const int src = __reduce_add_sync(0xffffffffu, nsrc);
+            if (lane == 0) leaf_done(a, l, te - tb, far.count, far.nch, false, src, tot);
+            if (nn != nb) {
+                if (nb > 0) flush_near();
+                if (lane == 0) {
+                    const int k = atomicAdd(&a.counters->n_long, 1);
+                    a.long_leaf[k] = l;
+                    a.long_head[k] = head;
+                    a.long_near[k] = nn;
+                }
+                continue;
+            }
+            int nbase = 0;
+            if (lane == 0) nbase = near_place(a, l, nn);
+            nbase = __shfl_sync(0xffffffffu, nbase, 0);
+            if (nbase < 0) continue;
+            uint32_t* src_buf = reinterpret_cast<uint32_t*>(stk) + kWalkSlots - nn;  // stack is empty
+            int32_t* dst = a.near_leaf + nbase;
+            uint32_t* tmp = reinterpret_cast<uint32_t*>(stk);
+            if (nn <= 32) warp_sort<1>(src_buf, tmp, nn, lane, dst);
+            else if (nn <= 64) warp_sort<2>(src_buf, tmp, nn, lane, dst);
+            else if (nn <= 128) warp_sort<4>(src_buf, tmp, nn, lane, dst);
+            else if (nn <= 256) warp_sort<8>(src_buf, tmp, nn, lane, dst);
+            else warp_sort<16>(src_buf, tmp, nn, lane, dst);
+        }
+    }
+    tot.flush(a, lane);
+}
+
+// The leaves whose stack overflowed, one warp each, in two passes: the walk as above
+// until the stack would overflow, then every lane walks its pending children and its share of the
+// stack depth first with a private stack -- once to count, so that the lists' sizes and the lanes'
+// places (lanes in order) are known and the order is deterministic, and once to write.
+template <bool WRITE>
+__device__ void slow_walk(const TreeListArgs& a, const int t, const WalkNode& T, const SeparationTest& separated,
+                          int* stk, const int lane, int64_t fbase, int64_t nbase, int& nf, int& nn, int& nsrc) {
+    const unsigned lt = (1u << lane) - 1u;
+    nf = nn = nsrc = 0;
+    int top = 1, pmask = 0, pchild = 0;
+    // 1 far, 2 near, 3 expand
+    auto classify = [&](int s, const WalkNode& S) { return s != t && separated(T, S) ? 1 : S.child < 0 ? 2 : 3; };
+    __syncwarp();
     if (lane == 0) stk[0] = 0;
     __syncwarp();
     while (top > 0) {
         const int take = min(32, top), base = top - take;
-        int s = -1, cls = 0;
-        WalkNode S;
+        int s = 0, cls = 0;
+        WalkNode S = T;
         if (lane < take) {
             s = stk[base + lane];
-            S = a.wn[s];
-            cls = classify(T, t, S, s, a.theta);
+            S = load_walk_node(a.wn, s);
+            cls = classify(s, S);
         }
-        __syncwarp();
-        top = base;
         const unsigned mf = __ballot_sync(0xffffffffu, cls == 1);
         const unsigned mn = __ballot_sync(0xffffffffu, cls == 2);
-        const unsigned me = __ballot_sync(0xffffffffu, cls == 3);
-        if (FILL) {
-            if (cls == 1) {
-                const int pos = fo + nf + __popc(mf & lt);
-                a.far_node[pos] = s;
-            }
-            if (cls == 2) a.near_key[no + nn + __popc(mn & lt)] = (uint32_t)a.node_leaf[s];
-        } else if (cls == 2) {
-            nsrc += S.end - S.beg;
+        if (WRITE && cls == 1 && fbase >= 0) a.far_node[fbase + nf + __popc(mf & lt)] = s;
+        if (cls == 2) {
+            if (WRITE) a.seg_near[nbase + nn + __popc(mn & lt)] = S.leaf;
+            nsrc += S.count;
         }
         nf += __popc(mf);
         nn += __popc(mn);
-        // expanded nodes push their massive children (massless ones would be skipped anyway)
-        const int mine = cls == 3 ? __popc(S.mask) : 0;
+        const int m = cls == 3 ? S.mask : 0, mine = __popc(m);
         int at = mine;
         for (int o = 1; o < 32; o <<= 1) {
             const int u = __shfl_up_sync(0xffffffffu, at, o);
             if (lane >= o) at += u;
         }
         const int add = __shfl_sync(0xffffffffu, at, 31);
-        if (top + add > kWalkStack) {
-            pend = cls == 3 ? s : -1;
-            pmask = cls == 3 ? S.mask : 0;
-            pchild = cls == 3 ? S.child : 0;
+        top = base;
+        if (base + add > a.walk_stack) {
+            pmask = m;
+            pchild = S.child;
             break;
         }
-        if (cls == 3) {
-            at = top + at - mine;
-            for (int c = 7; c >= 0; --c)
-                if (S.mask >> c & 1) stk[at++] = S.child + c;
-        }
+        at += base - mine;
+        for (int c = 7; c >= 0; --c)
+            if (m >> c & 1) stk[at++] = S.child + c;
         top += add;
         __syncwarp();
     }
-    if (top > 0 || __any_sync(0xffffffffu, pend >= 0)) {
-        // overflow: each lane walks its pending children and its share of the stack depth
-        // first with a private stack -- once to count, and in the fill pass once more to
-        // write at the lane's place (lanes in order), so the list order is deterministic
-        int st[kStack];
-        auto lane_walk = [&](bool write, int fpos, int npos, int& lf, int& ln) {
-            lf = ln = 0;
-            for (int i = lane - 32; i < top; i += 32) {
-                int sp = 0;
-                if (i < 0) {
-                    if (pend < 0) continue;
-                    for (int c = 7; c >= 0; --c)
-                        if (pmask >> c & 1) st[sp++] = pchild + c;
-                } else {
-                    st[sp++] = stk[i];
-                }
-                while (sp > 0) {
-                    const int s = st[--sp];
-                    const WalkNode S = a.wn[s];
-                    const int cls = classify(T, t, S, s, a.theta);
-                    if (cls == 1) {
-                        if (write) a.far_node[fpos + lf] = s;
-                        ++lf;
-                    } else if (cls == 2) {
-                        if (write) a.near_key[npos + ln] = (uint32_t)a.node_leaf[s];
-                        else nsrc += S.end - S.beg;
-                        ++ln;
-                    } else if (cls == 3) {
-                        for (int c = 7; c >= 0; --c)
-                            if (S.mask >> c & 1) st[sp++] = S.child + c;
-                    }
-                }
-            }
-        };
-        int lf, ln;
-        lane_walk(false, 0, 0, lf, ln);
-        int ef = lf, en = ln;  // inclusive prefix sums over the lanes
-        for (int o = 1; o < 32; o <<= 1) {
-            const int uf = __shfl_up_sync(0xffffffffu, ef, o), un = __shfl_up_sync(0xffffffffu, en, o);
-            if (lane >= o) {
-                ef += uf;
-                en += un;
-            }
-        }
-        if (FILL) {
-            int lf2, ln2;
-            nsrc = 0;
-            lane_walk(true, fo + nf + ef - lf, no + nn + en - ln, lf2, ln2);
-        }
-        nf += __shfl_sync(0xffffffffu, ef, 31);
-        nn += __shfl_sync(0xffffffffu, en, 31);
-    }
-    if constexpr (FILL) {
-        // the near list into the reference's depth-first order (leaf ordinals are depth-first
-        // numbers)
-        __syncwarp();
-        if (nn <= kSortCap) {
-            sort_into(a.near_key + no, nn, reinterpret_cast<uint64_t*>(stk), lane, a.near_leaf + no);
-        } else if (lane == 0) {
-            a.long_leaf[atomicAdd(a.long_count, 1)] = l;  // sorted by long_sort_kernel
-        }
-    } else {
-        for (int o = 16; o > 0; o >>= 1) nsrc += __shfl_xor_sync(0xffffffffu, nsrc, o);
-        if (lane != 0) return;
-        a.far_cnt[l] = nf;
-        a.near_cnt[l] = nn;
-        // far-field work items: only leaves with a target in range
-        const int tb = a.leaf_off[l], te = a.leaf_off[l + 1];
-        bool any = false;
-        for (int k = tb; k < te && !any; ++k) any = a.leaf_part[k] >= a.t_begin && a.leaf_part[k] < a.t_end;
-        const int nch = (any && nf > 0) ? (nf + kM2PChunk - 1) / kM2PChunk : 0;
-        const int slots = nch > 1 ? nch * (te - tb) : 0;
-        a.item_cnt[l] = nch;
-        a.slot_cnt[l] = slots;
-        atomicAdd(&a.totals[0], (unsigned long long)nf);
-        atomicAdd(&a.totals[1], (unsigned long long)nn);
-        atomicAdd(&a.totals[2], (unsigned long long)nch);
-        atomicAdd(&a.totals[3], (unsigned long long)slots);
-        atomicAdd(&a.totals[4], (unsigned long long)nf * (unsigned long long)(te - tb));
-        atomicAdd(&a.totals[5], (unsigned long long)nsrc * (unsigned long long)(te - tb));
-    }
-}
-
-// Near lists longer than a warp's buffer: one CTA per list.  Runs of kLongSort ordinals
-// are sorted by a bitonic network in shared memory and written back in place; each ordinal's
-// final place is then the sum over the runs of the number of smaller ordinals in the run
-// (binary searches; the ordinals are distinct).
-constexpr int kLongSort = 8192;
-__global__ void __launch_bounds__(1024) long_sort_kernel(const TreeListArgs a) {
-    __shared__ uint32_t s_key[kLongSort];
-    const int n_long = *a.long_count;
-    for (int q = blockIdx.x; q < n_long; q += gridDim.x) {
-        const int l = a.long_leaf[q];
-        const int no = a.near_off[l], n = a.near_off[l + 1] - no;
-        uint64_t* v = a.near_key + no;
-        const int runs = (n + kLongSort - 1) / kLongSort;
-        for (int r = 0; r < runs; ++r) {
-            const int b = r * kLongSort, m = min(kLongSort, n - b);
-            int P = 1;
-            while (P < m) P <<= 1;
-            for (int i = threadIdx.x; i < P; i += 1024) s_key[i] = i < m ? (uint32_t)v[b + i] : 0xffffffffu;
-            __syncthreads();
-            for (int k = 2; k <= P; k <<= 1)
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    for (int i = threadIdx.x; i < P; i += 1024) {
-                        const int mm = i ^ j;
-                        if (mm > i) {
-                            const uint32_t x = s_key[i], y = s_key[mm];
-                            if ((x > y) == ((i & k) == 0)) {
-                                s_key[i] = y;
-                                s_key[mm] = x;
-                            }
-                        }
-                    }
-                    __syncthreads();
-                }
-            if (runs == 1) {
-                for (int i = threadIdx.x; i < m; i += 1024) a.near_leaf[no + i] = (int32_t)s_key[i];
+    int st[kStack];
+    auto lane_walk = [&](bool write, int64_t fpos, int64_t npos, int& lf, int& ln, int& lsrc) {
+        lf = ln = lsrc = 0;
+        for (int i = lane - 32; i < top; i += 32) {
+            int sp = 0;
+            if (i < 0) {
+                for (int c = 7; c >= 0; --c)
+                    if (pmask >> c & 1) st[sp++] = pchild + c;
             } else {
-                for (int i = threadIdx.x; i < m; i += 1024) v[b + i] = s_key[i];
+                st[sp++] = stk[i];
             }
-            __syncthreads();
-        }
-        if (runs == 1) continue;
-        __threadfence_block();
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += 1024) {
-            const uint64_t key = v[i];
-            int pos = 0;
-            for (int r = 0; r < runs; ++r) {
-                int lo = r * kLongSort, hi = min(n, lo + kLongSort);
-                const int base = lo;
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (v[mid] < key) lo = mid + 1;
-                    else hi = mid;
+            while (sp > 0) {
+                const int s = st[--sp];
+                const WalkNode S = load_walk_node(a.wn, s);
+                const int cls = classify(s, S);
+                if (cls == 1) {
+                    if (write && fbase >= 0) a.far_node[fpos + lf] = s;
+                    ++lf;
+                } else if (cls == 2) {
+                    if (write) a.seg_near[npos + ln] = S.leaf;
+                    ++ln;
+                    lsrc += S.count;
+                } else {
+                    for (int c = 7; c >= 0; --c)
+                        if (S.mask >> c & 1) st[sp++] = S.child + c;
                 }
-                pos += lo - base;
             }
-            a.near_leaf[no + pos] = (int32_t)(uint32_t)key;
         }
-        __syncthreads();
+    };
+    int lf, ln, lsrc;
+    lane_walk(false, 0, 0, lf, ln, lsrc);
+    nsrc += lsrc;
+    int ef = lf, en = ln;  // inclusive prefix sums over the lanes
+    for (int o = 1; o < 32; o <<= 1) {
+        const int uf = __shfl_up_sync(0xffffffffu, ef, o), un = __shfl_up_sync(0xffffffffu, en, o);
+        if (lane >= o) {
+            ef += uf;
+            en += un;
+        }
     }
+    if (WRITE) lane_walk(true, fbase + nf + ef - lf, nbase + nn + en - ln, lf, ln, lsrc);
+    nf += __shfl_sync(0xffffffffu, ef, 31);
+    nn += __shfl_sync(0xffffffffu, en, 31);
 }
 
-__global__ void __launch_bounds__(256) items_kernel(const TreeListArgs a, int n_leaves) {
-    const int l = blockIdx.x * 256 + threadIdx.x;
-    if (l >= min(n_leaves, a.start_ord[a.n]) || (a.overflow && *a.overflow)) return;
-    const int nch = a.item_cnt[l];
-    const int fb = a.far_off[l], fe = a.far_off[l + 1];
-    M2PItem* items = (M2PItem*)a.items;
-    for (int c = 0; c < nch; ++c) {
-        M2PItem it;
-        it.leaf = l;
-        it.fb = fb + c * kM2PChunk;
-        it.fe = min(fe, it.fb + kM2PChunk);
-        it.chunk = c;
-        it.nchunks = nch;
-        it.pad = 0;
-        it.scratch = nch > 1 ? a.slot_off[l] : 0;
-        items[a.item_off[l] + c] = it;
+__global__ void __launch_bounds__(kWalkThreads) slow_walk_kernel(const TreeListArgs a) {
+    constexpr int W = kWalkThreads / 32;
+    __shared__ int s_stk[W][kWalkStack];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_slow = a.counters->n_slow;
+    const SeparationTest separated(a.theta, n_slow > 0 ? a.hw[0] : 0.0);
+    WalkTotals tot;
+    for (int q = blockIdx.x * W + wid; q < n_slow; q += gridDim.x * W) {
+        const int l = a.slow_leaf[q], t = a.leaf_node[l];
+        const WalkNode T = load_walk_node(a.wn, t);
+        const int tb = a.leaf_off[l], te = a.leaf_off[l + 1];
+        int nf, nn, nsrc;
+        slow_walk<false>(a, t, T, separated, s_stk[wid], lane, 0, 0, nf, nn, nsrc);
+        const int src = __reduce_add_sync(0xffffffffu, nsrc);
+        const int nch = leaf_in_range(a, tb, te, lane) ? (nf + kM2PChunk - 1) / kM2PChunk : 0;
+        const int ns = (nn + kNearSeg - 1) / kNearSeg;
+        unsigned long long c0 = 0, s0 = 0;
+        if (lane == 0) {
+            c0 = atomicAdd(&a.counters->chunks, (unsigned long long)nch);
+            s0 = atomicAdd(&a.counters->segs, (unsigned long long)ns);
+            leaf_done(a, l, te - tb, nf, nch, true, src, tot);
+        }
+        c0 = __shfl_sync(0xffffffffu, c0, 0);
+        s0 = __shfl_sync(0xffffffffu, s0, 0);
+        if ((int64_t)c0 + nch > a.far_cap || (int64_t)s0 + ns > a.seg_cap) {
+            // the totals tell; the reserved chunks that do exist are void
+            for (int64_t c = (int64_t)c0 + lane; c < min((int64_t)c0 + nch, a.far_cap); c += 32)
+                ((M2PItem*)a.items)[c].leaf = -1;
+            continue;
+        }
+        // a leaf without a target in range keeps no far list (place -1)
+        slow_walk<true>(a, t, T, separated, s_stk[wid], lane, nch > 0 ? (int64_t)c0 * kM2PChunk : (int64_t)-1,
+                        (int64_t)s0 * kNearSeg, nf, nn, nsrc);
+        for (int c = lane; c < nch; c += 32) {
+            M2PItem it;
+            it.leaf = l;
+            it.chunk = c;
+            it.nchunks = -1;
+            it.count = min(kM2PChunk, nf - c * kM2PChunk);
+            it.fb = ((int64_t)c0 + c) * kM2PChunk;
+            it.scratch = 0;
+            ((M2PItem*)a.items)[c0 + c] = it;
+        }
+        for (int k = lane; k < ns; k += 32) {
+            a.seg_next[s0 + k] = k > 0 ? (int)(s0 + k - 1) : -1;
+            a.seg_count[s0 + k] = min(kNearSeg, nn - k * kNearSeg);
+        }
+        if (lane == 0) {
+            const int k = atomicAdd(&a.counters->n_long, 1);
+            a.long_leaf[k] = l;
+            a.long_head[k] = (int)(s0 + ns - 1);
+            a.long_near[k] = nn;
+        }
+    }
+    tot.flush(a, lane);
+}
+
+// Near lists that went to segments, one block each: the ordinals set bits in shared memory, and the
+// set bits in order are the sorted list (kLongBits leaves per round).  Replaces sorting networks
+// in shared memory and ranks by binary search: N = 65,536 leaf 64 (9 lists of 500 to 1200) 11 us, N = 2^20
+// leaf 16 (1100 lists) 69 us, against 42 and 310 us.
+constexpr int kLongThreads = 512;
+constexpr int kLongWords = 8192;
+__global__ void __launch_bounds__(kLongThreads) long_near_kernel(const TreeListArgs a) {
+    __shared__ unsigned s_bits[kLongWords];
+    __shared__ int s_warp[kLongThreads / 32];
+    __shared__ int s_base;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int n_long = a.counters->n_long, n_leaves = a.start_ord[a.n];
+    if ((int64_t)a.counters->segs > a.seg_cap) return;  // a list is incomplete: the totals tell
+    for (int q = blockIdx.x; q < n_long; q += gridDim.x) {
+        if (tid == 0) s_base = near_place(a, a.long_leaf[q], a.long_near[q]);
+        __syncthreads();
+        if (s_base >= 0) {
+            int out = s_base;
+            for (int r0 = 0; r0 < n_leaves; r0 += 32 * kLongWords) {
+                const int words = (min(32 * kLongWords, n_leaves - r0) + 31) / 32;
+                const int per = (words + kLongThreads - 1) / kLongThreads;  // consecutive words of a thread
+                for (int w = tid; w < words; w += kLongThreads) s_bits[w] = 0;
+                __syncthreads();
+                for (int seg = a.long_head[q]; seg >= 0; seg = a.seg_next[seg]) {
+                    if (tid < a.seg_count[seg]) {
+                        const int o = a.seg_near[(int64_t)seg * kNearSeg + tid] - r0;
+                        if (o >= 0 && o < 32 * kLongWords) atomicOr(&s_bits[o >> 5], 1u << (o & 31));
+                    }
+                }
+                __syncthreads();
+                const int wb = min(tid * per, words), we = min(wb + per, words);
+                int mine = 0;
+                for (int w = wb; w < we; ++w) mine += __popc(s_bits[w]);
+                int incl = mine;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += u;
+                }
+                if (lane == 31) s_warp[wid] = incl;
+                __syncthreads();
+                int pos = out + incl - mine, total = 0;
+                for (int w = 0; w < kLongThreads / 32; ++w) {
+                    if (w < wid) pos += s_warp[w];
+                    total += s_warp[w];
+                }
+                for (int w = wb; w < we; ++w)
+                    for (unsigned b = s_bits[w]; b != 0; b &= b - 1) a.near_leaf[pos++] = r0 + 32 * w + __ffs(b) - 1;
+                out += total;
+                __syncthreads();
+            }
+        }
+        __syncthreads();
     }
 }
+static_assert(kLongThreads == kNearSeg, "one thread per entry of a segment");
 
 // Far-field items, largest first (cost = targets x nodes): fewer long items at the tail.
 // Sort keys: the cost of the real items (n_real of them, from the device count when given) on
 // a log scale with four steps per octave (1..127, 7 bits: one radix pass), 0 for the rest of
 // the capacity, so that the real items come first, largest first.  The order only balances
 // the blocks' work: a leaf's partial sums are added in chunk order whatever it is.
-__global__ void __launch_bounds__(256) item_cost_kernel(const M2PItem* items, const int32_t* leaf_off, int n,
-                                                        const unsigned long long* n_real, const int* overflow,
-                                                        uint32_t* cost, int32_t* idx) {
+__device__ __forceinline__ bool item_valid(const TreeListArgs& a, const M2PItem& it) {
+    return it.leaf >= 0 && (a.far_nch[it.leaf] < 0) == (it.nchunks < 0);
+}
+__global__ void __launch_bounds__(256) item_cost_kernel(const TreeListArgs a, int n, const unsigned long long* n_real,
+                                                        const int* overflow, uint32_t* cost, int32_t* idx) {
     const int k = blockIdx.x * 256 + threadIdx.x;
     if (k >= n) return;
     const int real = (overflow && *overflow) ? 0 : n_real ? (int)min(*n_real, (unsigned long long)n) : n;
     uint32_t c = 0;
     if (k < real) {
-        const M2PItem it = items[k];
-        const uint32_t v = min((uint32_t)(leaf_off[it.leaf + 1] - leaf_off[it.leaf]) * (uint32_t)(it.fe - it.fb) + 1u,
-                               0x7fffffffu);
-        const int msb = 31 - __clz(v);
-        c = v < 4u ? v : (uint32_t)(msb * 4 + ((v >> (msb - 2)) & 3));
+        const M2PItem it = ((const M2PItem*)a.items)[k];
+        if (item_valid(a, it)) {
+            const uint32_t v = min((uint32_t)(a.leaf_off[it.leaf + 1] - a.leaf_off[it.leaf]) * (uint32_t)it.count + 1u,
+                                   0x7fffffffu);
+            const int msb = 31 - __clz(v);
+            c = v < 4u ? v : (uint32_t)(msb * 4 + ((v >> (msb - 2)) & 3));
+        }
     }
     cost[k] = c;
     idx[k] = k;
@@ -728,54 +953,40 @@ __global__ void __launch_bounds__(256) item_cost_kernel(const M2PItem* items, co
 // evaluation's totals, or the topology build could not complete on the device.
 __global__ void pool_check_kernel(const TreeListArgs a, const int32_t* tree_hdr) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const unsigned long long* t = a.totals;
+    const ListCounters& t = *a.counters;
     if (a.need) {
         atomicMax(&a.need[0], (unsigned long long)(tree_hdr[0] > 0 ? tree_hdr[0] : 0));
-        for (int k = 0; k < 4; ++k) atomicMax(&a.need[1 + k], t[k]);
+        atomicMax(&a.need[1], t.chunks);
+        atomicMax(&a.need[2], t.near);
+        atomicMax(&a.need[3], t.slots);
         // levels of the tree; a tree cut short by too few sorted key levels asks for all
-        atomicMax(&a.need[5], (unsigned long long)(tree_hdr[2] & 4 ? kKeyLevels : max(tree_hdr[1], 0)));
+        atomicMax(&a.need[4], (unsigned long long)(tree_hdr[2] & 4 ? kKeyLevels : max(tree_hdr[1], 0)));
+        atomicMax(&a.need[5], t.segs);
     }
-    if (t[0] > (unsigned long long)a.far_cap || t[1] > (unsigned long long)a.near_cap ||
-        t[2] > (unsigned long long)a.item_cap || t[3] > (unsigned long long)a.slot_cap || tree_hdr[2] != 0) {
+    if (t.chunks > (unsigned long long)a.far_cap || t.near > (unsigned long long)a.near_cap ||
+        t.segs > (unsigned long long)a.seg_cap || t.slots > (unsigned long long)a.slot_cap || tree_hdr[2] != 0) {
         *a.overflow = 1;
         if (a.overflow_sticky) atomicOr(a.overflow_sticky, tree_hdr[2] & 1 ? 3 : 1);  // bit 1: too deep
     }
 }
 
-__global__ void __launch_bounds__(256) item_gather_kernel(const M2PItem* items, const int32_t* idx, int n,
-                                                          M2PItem* out) {
+__global__ void __launch_bounds__(256) item_gather_kernel(const TreeListArgs a, const int32_t* idx, int n,
+                                                          const uint32_t* cost, M2PItem* out) {
     const int k = blockIdx.x * 256 + threadIdx.x;
-    if (k < n) out[k] = items[idx[k]];
+    if (k >= n) return;
+    M2PItem it;
+    it.leaf = -1;
+    if (cost[k] > 0) {  // real and valid
+        it = ((const M2PItem*)a.items)[idx[k]];
+        it.nchunks = abs(a.far_nch[it.leaf]);
+        it.scratch = a.far_slot[it.leaf];
+    }
+    out[k] = it;
 }
 
 size_t scan_bytes(int count) {
     size_t b = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, b, (const int32_t*)nullptr, (int32_t*)nullptr, count);
-    return b;
-}
-
-// The four per-leaf counts of the list pass (far, near, work items, partial-sum slots)
-// scanned together: one exclusive scan of 4-tuples, element-wise sums.
-using Count4 = thrust::tuple<int32_t, int32_t, int32_t, int32_t>;
-struct Sum4 {
-    __host__ __device__ Count4 operator()(const Count4& a, const Count4& b) const {
-        return Count4(thrust::get<0>(a) + thrust::get<0>(b), thrust::get<1>(a) + thrust::get<1>(b),
-                      thrust::get<2>(a) + thrust::get<2>(b), thrust::get<3>(a) + thrust::get<3>(b));
-    }
-};
-
-cudaError_t scan4(void* temp, size_t& bytes, const int32_t* const cnt[4], int32_t* const off[4], int count,
-                  cudaStream_t st) {
-    auto in = thrust::make_zip_iterator(thrust::make_tuple(cnt[0], cnt[1], cnt[2], cnt[3]));
-    auto out = thrust::make_zip_iterator(thrust::make_tuple(off[0], off[1], off[2], off[3]));
-    return cub::DeviceScan::ExclusiveScan(temp, bytes, in, out, Sum4{}, Count4(0, 0, 0, 0), count, st);
-}
-
-size_t scan4_bytes(int count) {
-    size_t b = 0;
-    const int32_t* cnt[4] = {nullptr, nullptr, nullptr, nullptr};
-    int32_t* off[4] = {nullptr, nullptr, nullptr, nullptr};
-    scan4(nullptr, b, cnt, off, count, nullptr);
     return b;
 }
 
@@ -847,28 +1058,23 @@ cudaError_t launch_tree_leaf_order(const TreeBuildArgs& t, int32_t n_nodes, void
 }
 
 size_t tree_list_temp_bytes(int32_t n, int32_t n_nodes) {
-    return std::max({scan_bytes(n + 1), scan_bytes(n_nodes + 1), scan4_bytes(n_nodes + 1)});
+    (void)n_nodes;
+    return scan_bytes(n + 1);
 }
 
-// Both walk kernels prefer a 60% shared-memory carveout (8 blocks of 17 KiB; the rest is L1).
+// The walk prefers a 70% shared-memory carveout (8 blocks of 19 KiB; the rest is L1).
 static cudaError_t walk_carveout() {
-    static cudaError_t once = [] {
-        cudaError_t e = cudaFuncSetAttribute(walk_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, 60);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(walk_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 60);
-        return e;
-    }();
+    static cudaError_t once =
+        cudaFuncSetAttribute(walk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 70);
     return once;
 }
 
-cudaError_t launch_tree_lists_count(const TreeListArgs& a, void* temp, size_t temp_bytes, cudaStream_t st) {
+cudaError_t launch_tree_lists(const TreeListArgs& a, void* temp, size_t temp_bytes, int sms, cudaStream_t st) {
     cudaError_t e;
-    const size_t nb = (size_t)(a.n + 1) * sizeof(int32_t), lb = (size_t)(a.n_nodes + 1) * sizeof(int32_t);
+    const size_t nb = (size_t)(a.n + 1) * sizeof(int32_t);
     if ((e = cudaMemsetAsync(a.start_flag, 0, nb, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(a.keep, 0, nb, st)) != cudaSuccess) return e;
-    for (int32_t* p : {a.far_cnt, a.near_cnt, a.item_cnt, a.slot_cnt})
-        if ((e = cudaMemsetAsync(p, 0, lb, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(a.totals, 0, 6 * sizeof(unsigned long long), st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(a.counters, 0, sizeof(ListCounters), st)) != cudaSuccess) return e;
     const int gn = (a.n_nodes + 255) / 256;
     leaf_mark_kernel<<<gn, 256, 0, st>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
@@ -879,12 +1085,11 @@ cudaError_t launch_tree_lists_count(const TreeListArgs& a, void* temp, size_t te
     leaf_emit_kernel<<<gn, 256, 0, st>>>(a);
     walk_pack_kernel<<<gn, 256, 0, st>>>(a);
     if ((e = walk_carveout()) != cudaSuccess) return e;
-    walk_kernel<false><<<(a.n_nodes + kWalkThreads / 32 - 1) / (kWalkThreads / 32), kWalkThreads, 0, st>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    const int32_t* const cnt[4] = {a.far_cnt, a.near_cnt, a.item_cnt, a.slot_cnt};
-    int32_t* const off[4] = {a.far_off, a.near_off, a.item_off, a.slot_off};
-    tb = temp_bytes;
-    return scan4(temp, tb, cnt, off, a.n_nodes + 1, st);
+    constexpr int W = kWalkThreads / 32;
+    walk_kernel<<<std::min((a.n_nodes + W - 1) / W, sms * 8), kWalkThreads, 0, st>>>(a);
+    slow_walk_kernel<<<sms, kWalkThreads, 0, st>>>(a);
+    long_near_kernel<<<sms * 4, kLongThreads, 0, st>>>(a);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_tree_massive(const TreeListArgs& a, void* temp, size_t temp_bytes, cudaStream_t st) {
@@ -901,16 +1106,6 @@ cudaError_t launch_pool_check(const TreeListArgs& a, const int32_t* tree_hdr, cu
     return cudaGetLastError();
 }
 
-cudaError_t launch_tree_lists_fill(const TreeListArgs& a, int32_t n_leaves, cudaStream_t st) {
-    if (n_leaves == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(a.long_count, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-    walk_kernel<true><<<(n_leaves + kWalkThreads / 32 - 1) / (kWalkThreads / 32), kWalkThreads, 0, st>>>(a);
-    long_sort_kernel<<<296, 1024, 0, st>>>(a);
-    items_kernel<<<(n_leaves + 255) / 256, 256, 0, st>>>(a, n_leaves);
-    return cudaGetLastError();
-}
-
 size_t item_order_temp_bytes(int32_t n_items) {
     size_t b = 0;
     cub::DoubleBuffer<uint32_t> k(nullptr, nullptr);
@@ -919,18 +1114,17 @@ size_t item_order_temp_bytes(int32_t n_items) {
     return b;
 }
 
-cudaError_t launch_item_order(const M2PItem* items, const int32_t* leaf_off, int32_t n_items,
-                              const unsigned long long* n_real, const int* overflow, uint32_t* cost,
-                              uint32_t* cost_alt, int32_t* idx, int32_t* idx_alt, void* temp, size_t temp_bytes,
-                              M2PItem* out, cudaStream_t st) {
+cudaError_t launch_item_order(const TreeListArgs& a, int32_t n_items, const unsigned long long* n_real,
+                              const int* overflow, uint32_t* cost, uint32_t* cost_alt, int32_t* idx, int32_t* idx_alt,
+                              void* temp, size_t temp_bytes, M2PItem* out, cudaStream_t st) {
     if (n_items == 0) return cudaSuccess;
     const int g = (n_items + 255) / 256;
-    item_cost_kernel<<<g, 256, 0, st>>>(items, leaf_off, n_items, n_real, overflow, cost, idx);
+    item_cost_kernel<<<g, 256, 0, st>>>(a, n_items, n_real, overflow, cost, idx);
     cub::DoubleBuffer<uint32_t> k(cost, cost_alt);
     cub::DoubleBuffer<int32_t> v(idx, idx_alt);
     cudaError_t e = cub::DeviceRadixSort::SortPairsDescending(temp, temp_bytes, k, v, n_items, 0, 7, st);
     if (e != cudaSuccess) return e;
-    item_gather_kernel<<<g, 256, 0, st>>>(items, v.Current(), n_items, out);
+    item_gather_kernel<<<g, 256, 0, st>>>(a, v.Current(), n_items, k.Current(), out);
     return cudaGetLastError();
 }
 

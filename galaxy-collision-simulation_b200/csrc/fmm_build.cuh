@@ -49,15 +49,26 @@ cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_by
 cudaError_t launch_tree_leaf_order(const TreeBuildArgs& t, int32_t n_nodes, void* temp, size_t temp_bytes,
                                    cudaStream_t st);
 
-// What the list walk reads of a node, packed (56 B); mask has bit c set when child c has
-// mass > 0.
-struct WalkNode {
+// What the list walk reads of a node, packed (48 B: three 16-byte loads).
+struct __align__(16) WalkNode {
     double cx, cy, cz, hw;
-    double mass;
-    int32_t child;
-    int32_t beg, end;
-    int32_t mask;
+    int32_t child;  // first child, -1 for a leaf
+    int32_t mask;   // bit c set when child c has mass > 0
+    int32_t leaf;   // ordinal among the leaves with mass > 0 (leaves only)
+    int32_t count;  // bodies
 };
+
+// Counters of the list passes, zeroed before them.
+struct ListCounters {
+    unsigned long long far, near;              // list entries
+    unsigned long long chunks;                 // far-list chunks (work items) reserved
+    unsigned long long slots;                  // partial sums of leaves with several chunks
+    unsigned long long far_pairs, near_pairs;  // (body, far node) and (body, body) pairs
+    unsigned long long segs;                   // segments of long near lists reserved
+    int ticket, n_long, n_slow, pad;
+};
+constexpr int kNearSeg = 512;  // entries of a segment of a long near list
+constexpr int kWalkStackSlots = 1024;  // entries a walk's stack may hold
 
 // Leaves with mass > 0 (depth-first) and their near / far lists, after the node moments.
 struct TreeListArgs {
@@ -80,6 +91,7 @@ struct TreeListArgs {
     int32_t* mprefix;
     WalkNode* wn;       // n_nodes, filled before the walk
     double theta;
+    int walk_stack;     // at most kWalkStackSlots: where a walk's stack counts as overflowing
     int64_t t_begin, t_end;
     // body-position scratch, n + 1 each
     int32_t* start_flag;
@@ -91,54 +103,60 @@ struct TreeListArgs {
     int32_t* leaf_part;  // n
     int32_t* leaf_node;
     int32_t* node_leaf;  // n_nodes
-    // per-leaf counts and their exclusive sums, n_nodes + 1 each
-    int32_t* far_cnt;
-    int32_t* near_cnt;
-    int32_t* item_cnt;
-    int32_t* slot_cnt;
-    int32_t* far_off;
-    int32_t* near_off;
-    int32_t* item_off;
-    int32_t* slot_off;
-    unsigned long long* totals;  // 6: far, near, items, slots (overflow check), far and near body pairs
-    // fill pass: the near lists unsorted (leaf ordinals), then sorted into near_leaf
-    uint64_t* near_key;
-    int32_t* long_leaf;   // leaves whose near lists are sorted by a separate kernel
-    int32_t* long_count;
+    // Lists of leaf l (n_nodes entries each): near leaves near_leaf[near_beg .. near_end), their
+    // bodies near_src, far chunks far_nch, first partial-sum slot (far_nch > 1) far_slot.
+    int32_t* near_beg;
+    int32_t* near_end;
+    int32_t* near_src;
+    int32_t* far_nch;
+    int64_t* far_slot;
+    ListCounters* counters;
+    // far_cap chunks of kM2PChunk far nodes, each with its work item of the same number
+    // (M2PItem); a leaf's chunks are numbered in walk order but lie anywhere in the pool
     int32_t* far_node;
-    int32_t* near_leaf;
-    void* items;  // M2PItem
+    void* items;
+    int32_t* near_leaf;  // near_cap leaf ordinals
+    // near lists too long for a warp's buffer: linked segments of unsorted ordinals, then the
+    // leaves that have them; and leaves whose walk overflowed its stack
+    int32_t* seg_near;   // seg_cap * kNearSeg
+    int32_t* seg_next;   // seg_cap
+    int32_t* seg_count;  // seg_cap
+    int32_t* long_leaf;  // n_nodes each
+    int32_t* long_head;
+    int32_t* long_near;
+    int32_t* slow_leaf;
     // Capacity mode (nullable cnt_nodes / overflow): n_nodes is the capacity of the node
     // arrays and the count is read on the device (cnt_nodes = the topology build's header
-    // {nodes, levels, flags}; a flag leaves no nodes); far/near/item/slot pools were reserved
-    // by capacity, pool_check marks an overflow when a total exceeds its pool (and records the
-    // largest totals seen in need[5], with a sticky copy of the flag), and the fill pass and
-    // everything after it are skipped.
+    // {nodes, levels, flags}; a flag leaves no nodes); pool_check marks an overflow when a total
+    // exceeds its pool (and records the largest totals seen in need, with a sticky copy of the
+    // flag), and everything after the lists is skipped.
     const int32_t* cnt_nodes;
     int* overflow;
     int* overflow_sticky;
-    unsigned long long* need;  // {nodes, far, near, items, slots}
-    int64_t far_cap, near_cap, item_cap, slot_cap;
+    unsigned long long* need;  // kNeed: {nodes, chunks, near, slots, tree levels, segments}
+    // pools (in both modes; writes past them are left out and the totals tell): chunks,
+    // entries, segments, slots
+    int64_t far_cap, near_cap, seg_cap, slot_cap;
 };
+constexpr int kNeed = 6;
 size_t tree_list_temp_bytes(int32_t n, int32_t n_nodes);
-// Leaf compaction, the count walk and the offsets (sizes become known on the host after it).
-cudaError_t launch_tree_lists_count(const TreeListArgs& a, void* temp, size_t temp_bytes, cudaStream_t st);
-// Capacity mode: after the count pass, the overflow check of the pools (and of the topology
-// build's header tree_hdr).
+// Leaf compaction and the lists with their far-field work items (kernels read the number of leaves
+// on the device; sizes become known on the host, when it wants them, from the counters).
+cudaError_t launch_tree_lists(const TreeListArgs& a, void* temp, size_t temp_bytes, int sms, cudaStream_t st);
 // mprefix from the masses (a.m, a.perm); a mass < 0 or NaN marks an overflow with bit 1 of
 // the sticky word (the caller then evaluates through the host-read path).  temp: scan scratch
 // for n + 1 ints.
 cudaError_t launch_tree_massive(const TreeListArgs& a, void* temp, size_t temp_bytes, cudaStream_t st);
+// Capacity mode: after the lists, the overflow check of the pools (and of the topology build's
+// header tree_hdr).
 cudaError_t launch_pool_check(const TreeListArgs& a, const int32_t* tree_hdr, cudaStream_t st);
-// The fill walk (each leaf's lists sorted into depth-first order) and the far-field work items.
-cudaError_t launch_tree_lists_fill(const TreeListArgs& a, int32_t n_leaves, cudaStream_t st);
-// The far-field items reordered by decreasing cost (targets x nodes) into out.
+// The far-field items reordered by decreasing cost (targets x nodes) into out, completed with
+// their leaves' chunk counts and partial-sum slots.
 struct M2PItem;
 size_t item_order_temp_bytes(int32_t n_items);
 // n_items is the length of the arrays; n_real (nullable: all) the items on the device.
-cudaError_t launch_item_order(const M2PItem* items, const int32_t* leaf_off, int32_t n_items,
-                              const unsigned long long* n_real, const int* overflow, uint32_t* cost,
-                              uint32_t* cost_alt, int32_t* idx, int32_t* idx_alt, void* temp, size_t temp_bytes,
-                              M2PItem* out, cudaStream_t st);
+cudaError_t launch_item_order(const TreeListArgs& a, int32_t n_items, const unsigned long long* n_real,
+                              const int* overflow, uint32_t* cost, uint32_t* cost_alt, int32_t* idx, int32_t* idx_alt,
+                              void* temp, size_t temp_bytes, M2PItem* out, cudaStream_t st);
 
 }  // namespace gx

@@ -13,8 +13,12 @@ struct P2PArgs {
     const double* m;
     const int32_t* leaf_off;   // n_leaves + 1
     const int32_t* leaf_part;  // body indices grouped by leaf
-    const int32_t* near_off;   // n_leaves + 1
-    const int32_t* near_leaf;  // leaf ids
+    // near leaves of leaf l: near_leaf[near_beg[l] .. near_end[l]) (the two halves of CSR offsets,
+    // or places of their own), leaf ids
+    const int32_t* near_beg;
+    const int32_t* near_end;
+    const int32_t* near_leaf;
+    const int32_t* near_src;   // nullable: bodies of leaf l's near leaves
     int32_t n_leaves;
     double* ax;  // accumulated into
     double* ay;
