@@ -274,10 +274,11 @@ void split_layout(int64_t n_src, int jt, int want, int64_t* chunk, int* nsplit) 
     *nsplit = (int)std::max<int64_t>(1, (n_src + c - 1) / c);
 }
 
-// Predicted time of (variant, nsplit) in units of "one SM running one source against one
-// target at full rate".  The CTAs are spread evenly over the SMs (L per SM); an SM runs
-// them in rounds of `occupancy` concurrent CTAs, and a round with fewer CTAs than needed to
-// cover latency (about 12 warps) runs at a proportionally lower rate.
+// Predicted time of (block shape, nsplit) in units of "one SM running one source against one
+// target at full rate".  The CTAs are spread evenly over the SMs (L per SM); an SM runs them in
+// rounds of `occ` concurrent CTAs.  A CTA's fixed work (targets, origin, epilogue) counts as
+// kCtaFixed sources, and w resident warps reach w / (w + 1) of the full rate.
+constexpr int kCtaFixed = 50;
 double rounds_cost(int block, int ipt, int jt, int occ, int64_t n_tgt, int64_t n_src, int ns, int sms) {
     const int64_t tile = (int64_t)block * ipt;
     const int64_t T = (n_tgt + tile - 1) / tile;
@@ -285,37 +286,79 @@ double rounds_cost(int block, int ipt, int jt, int occ, int64_t n_tgt, int64_t n
     int nse;
     split_layout(n_src, jt, ns, &chunk, &nse);
     const int64_t L = (T * nse + sms - 1) / sms;
-    const double W = (double)tile * (double)(chunk + jt);
-    const double warps = block / 32.0;
-    auto eff = [&](int64_t c) { return std::min(1.0, (double)c * warps / 12.0); };
+    const double W = (double)tile * (double)(chunk + kCtaFixed);
+    auto slow = [&](int64_t c) { return 1.0 + 32.0 / ((double)c * block); };
     const int64_t full = L / occ, rem = L % occ;
-    double t = (double)full * (double)occ * W / eff(occ);
-    if (rem) t += (double)rem * W / eff(rem);
-    // the ordered reduction pass reads nse partials per target
+    double t = (double)full * (double)occ * W * slow(occ);
+    if (rem) t += (double)rem * W * slow(rem);
+    // the ordered reduction reads nse partials per target
     if (nse > 1) t += 0.05 * (double)nse * (double)n_tgt * 64.0 / sms;
     return t;
 }
 
-double split_cost(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int ns, int sms) {
-    return rounds_cost(v.block, v.ipt, v.jt, force_occupancy(v), n_tgt, n_src, ns, sms);
-}
-
-int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
-    if (v.precision == kF64Exact) return 1;
+// The split of least cost(ns), a larger one only for more than half a percent.
+template <typename Cost>
+int least_split(int64_t n_src, int jt, Cost cost) {
     int best = 1;
-    double bc = split_cost(v, n_tgt, n_src, 1, sms);
+    double bc = cost(1);
     for (int ns = 2; ns <= 64; ++ns) {
         int64_t chunk;
         int nse;
-        split_layout(n_src, v.jt, ns, &chunk, &nse);
+        split_layout(n_src, jt, ns, &chunk, &nse);
         if (nse != ns) continue;
-        const double c = split_cost(v, n_tgt, n_src, ns, sms);
+        const double c = cost(ns);
         if (c < bc * 0.995) {
             bc = c;
             best = ns;
         }
     }
     return best;
+}
+
+// The j-split of a variant.  FP64, and mixed blocks of two warps: short chunks, so that many small
+// CTAs per SM hide one another's staging and latencies and even out the SMs; smaller still where
+// that leaves the SMs without work, never more than 64 chunks or kMaxPartBytes of partial sums.
+// Measured on B200 (us, sources per chunk): FP64 256 x 2 N = 16,384 512: 285, 1024: 327, one wave of
+// 2 CTAs per SM: 369; N = 49,999 1024: 2478, 2048: 2570, 16,896: 2673; N = 100,000 2048: 9680,
+// 6144: 9888; FP64 256 x 1 N = 8192 256: 84, 512: 94; mixed 64 x 4 N = 5000 256: 31, 512: 33;
+// N = 16,384 256: 145, 512: 135, 1280: 139; N = 23,000 512: 257, 1024: 249, 2560: 264.
+// Mixed blocks of four warps and more follow rounds_cost: whole rounds count most there (256 x 4,
+// N = 65,536: 16 chunks 1720 us, 9 chunks 1840; N = 32,768: 32 chunks 454, 8 chunks 505).
+constexpr int64_t kMaxPartBytes = 256ll << 20;
+int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
+    if (v.precision == kF64Exact) return 1;
+    if (v.precision == kMixed && v.block > 64)
+        return least_split(n_src, v.jt, [&](int ns) {
+            return rounds_cost(v.block, v.ipt, v.jt, force_occupancy(v), n_tgt, n_src, ns, sms);
+        });
+    int64_t chunk = v.precision == kMixed ? (n_src < 7000 ? 256 : n_src < 18000 ? 512 : 1024)
+                                          : (v.block == 64 ? 128 : v.block * v.ipt == 256 ? 256 : 512);
+    const int64_t tiles = (n_tgt + (int64_t)v.block * v.ipt - 1) / ((int64_t)v.block * v.ipt);
+    while (chunk > v.jt && tiles * ((n_src + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
+    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(64, kMaxPartBytes / (24 * n_tgt)));
+    return (int)std::max<int64_t>(1, std::min(most, (n_src + chunk - 1) / chunk));
+}
+
+// What the choice of a mixed variant weighs (heuristic_choice): a whole j tile of fixed work per
+// CTA, and full rate from 12 warps up.
+double mixed_variant_cost(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
+    const int occ = force_occupancy(v);
+    auto cost = [&](int ns) {
+        const int64_t tile = (int64_t)v.block * v.ipt, T = (n_tgt + tile - 1) / tile;
+        int64_t chunk;
+        int nse;
+        split_layout(n_src, v.jt, ns, &chunk, &nse);
+        const int64_t L = (T * nse + sms - 1) / sms;
+        const double W = (double)tile * (double)(chunk + v.jt);
+        const double warps = v.block / 32.0;
+        auto eff = [&](int64_t c) { return std::min(1.0, (double)c * warps / 12.0); };
+        const int64_t full = L / occ, rem = L % occ;
+        double t = (double)full * (double)occ * W / eff(occ);
+        if (rem) t += (double)rem * W / eff(rem);
+        if (nse > 1) t += 0.05 * (double)nse * (double)n_tgt * 64.0 / sms;
+        return t;
+    };
+    return cost(least_split(n_src, v.jt, cost));
 }
 
 std::mutex g_tune_mu;
@@ -329,12 +372,22 @@ double variant_rate_penalty(const ForceVariant& v) {
         if (v.packed == 1) return v.block * v.ipt >= 1024 ? 1.04 : 1.10;  // sources packed
         return 1.25;                                                      // scalar FP32
     }
-    if (v.precision == kF64) return v.block * v.ipt >= 512 ? 1.0 : 1.05;
     return 1.0;
 }
 
-// Untuned choice: the wave model over all variants of the precision, weighted by each
-// variant's measured per-interaction rate.
+// The FP64 variant for n_tgt targets: 256 x 2 from 15,000 up (N = 65,536 4.18 ms; 256 x 1 4.21,
+// 64 x 2 4.26), 256 x 1 below (N = 8192 84 us, 256 x 2 93, 64 x 2 91; N = 3000 25, 36 and 27), 64 x 2
+// for the smallest (N = 500 20 us, 256 x 1 23); softening 0 has 256 x 2 and 64 x 2 only.
+bool f64_shape(const ForceVariant& v, int64_t n_tgt, bool eps0) {
+    const int block = n_tgt >= (eps0 ? 6000 : 1500) ? 256 : 64;
+    const int ipt = block == 64 || eps0 || n_tgt >= 15000 ? 2 : 1;
+    return v.block == block && v.ipt == ipt;
+}
+
+// Untuned choice.  FP64: by n_tgt.  Mixed: the wave model over all variants, weighted by each
+// variant's measured per-interaction rate; a mixed variant also fixes the tiles whose centres are
+// the origins of the FP32 offsets, so its choice keeps to the weights of mixed_variant_cost, while
+// the split of the chosen variant only regroups FP64 sums.
 Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_t n_src) {
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -356,12 +409,12 @@ Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_
     for (int k = 0; k < c; ++k) {
         const ForceVariant& v = all[ids[k]];
         if (precision == kMixed && !v.packed) continue;  // the scalar form is kept for measurement only
-        const int ns = best_split(v, n_tgt, n_src, sms);
-        const double cost = split_cost(v, n_tgt, n_src, ns, sms) * variant_rate_penalty(v);
+        if (precision == kF64 && !f64_shape(v, n_tgt, eps0)) continue;
+        const double cost = precision == kMixed ? mixed_variant_cost(v, n_tgt, n_src, sms) * variant_rate_penalty(v) : 0.0;
         if (cost < bc) {
             bc = cost;
             best.variant = ids[k];
-            best.nsplit = ns;
+            best.nsplit = best_split(v, n_tgt, n_src, sms);
         }
     }
     return best;
@@ -2649,18 +2702,9 @@ extern "C" int gx_direct_vjp(int64_t n, const double* x, const double* y, const 
     int want = 1;
     {
         const VjpShape sh = vjp_shape(precision);
-        double best = rounds_cost(sh.block, sh.ipt, sh.jt, sh.occupancy, n, n, 1, sms);
-        for (int ns = 2; ns <= 64; ++ns) {
-            int64_t chunk;
-            int nse;
-            split_layout(n, sh.jt, ns, &chunk, &nse);
-            if (nse != ns) continue;
-            const double c = rounds_cost(sh.block, sh.ipt, sh.jt, sh.occupancy, n, n, ns, sms);
-            if (c < best * 0.995) {
-                best = c;
-                want = ns;
-            }
-        }
+        want = least_split(n, sh.jt, [&](int ns) {
+            return rounds_cost(sh.block, sh.ipt, sh.jt, sh.occupancy, n, n, ns, sms);
+        });
     }
     split_layout(n, vjp_jt(precision), want, &a.j_chunk, &a.nsplit);
     AsyncBuf part;

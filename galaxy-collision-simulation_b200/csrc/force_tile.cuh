@@ -419,8 +419,8 @@ __device__ __forceinline__ void mixed_tp_tile(const ForceArgs& a, const int64_t 
 // ---------------------------------------------------------------------------------------
 // FP64 with a refined hardware rsqrt: bound by the FP64 pipe, 16 operations per interaction
 // (3 subtractions, 3 FMA, 7 for the weight m s^-3/2 in inv_cube_f64, 3 FMA).  N = 49,999:
-// 2.68 ms = 933 Gint/s, 88% of the measured pipe rate; with the rsqrt refined first and cubed
-// after (17 operations) 2.94 ms.
+// 2.48 ms = 1008 Gint/s, 95% of the measured pipe rate; 2.68 ms with one wave of blocks, 2.94 ms
+// with the rsqrt refined first and cubed after (17 operations) as well.
 // ---------------------------------------------------------------------------------------
 template <int BLOCK, int IPT, int JT, bool EPS0>
 __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, const int chunk) {
