@@ -2697,23 +2697,19 @@ extern "C" int gx_direct_vjp(int64_t n, const double* x, const double* y, const 
     a.G = phys.G;
     a.eps2 = phys.softening * phys.softening;
     a.eps2f = (float)a.eps2;
-    // source split chosen by the same per-SM-rounds model as the forward kernels
-    const int sms = sm_count(dev);
-    int want = 1;
-    {
-        const VjpShape sh = vjp_shape(precision);
-        want = least_split(n, sh.jt, [&](int ns) {
-            return rounds_cost(sh.block, sh.ipt, sh.jt, sh.occupancy, n, n, ns, sms);
-        });
-    }
-    split_layout(n, vjp_jt(precision), want, &a.j_chunk, &a.nsplit);
+    const VjpVariant& v = vjp_variant(n, precision, eps0_of(precision, phys));
+    split_layout(n, v.jt, vjp_split(v, n, sm_count(dev)), &a.j_chunk, &a.nsplit);
     AsyncBuf part;
     a.part = nullptr;
+    a.tile_count = nullptr;
     if (a.nsplit > 1) {
-        GX_TRY(part.alloc((size_t)a.nsplit * 4 * (size_t)n * sizeof(double), st));
-        a.part = part.d();
+        const size_t tb = ((size_t)vjp_tiles(v, n) * sizeof(unsigned) + 255) & ~(size_t)255;
+        GX_TRY(part.alloc(tb + (size_t)a.nsplit * 4 * (size_t)n * sizeof(double), st));
+        a.tile_count = (unsigned*)part.p;
+        a.part = (double*)((char*)part.p + tb);
+        GX_CUDA(cudaMemsetAsync(part.p, 0, tb, st));
     }
-    GX_CUDA(launch_vjp(a, precision, st));
+    GX_CUDA(launch_vjp(v, a, st));
     if (!device) {
         for (int k = 0; k < 4; ++k)
             if (out[k]) GX_TRY(copy_back(k == 0 ? gxo : k == 1 ? gyo : k == 2 ? gzo : gmo, out[k], n, st));
