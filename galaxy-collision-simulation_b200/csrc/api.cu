@@ -327,11 +327,11 @@ int least_split(int64_t n_src, int jt, Cost cost) {
 constexpr int64_t kMaxPartBytes = 256ll << 20;
 int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
     if (v.precision == kF64Exact) return 1;
-    if (v.precision == kMixed && v.block > 64)
+    if (v.precision == kMixed && v.block * v.ipt > 256)
         return least_split(n_src, v.jt, [&](int ns) {
             return rounds_cost(v.block, v.ipt, v.jt, force_occupancy(v), n_tgt, n_src, ns, sms);
         });
-    int64_t chunk = v.precision == kMixed ? (n_src < 7000 ? 256 : n_src < 18000 ? 512 : 1024)
+    int64_t chunk = v.precision == kMixed ? (n_src <= 7000 ? 256 : n_src < 18000 ? 512 : 1024)
                                           : (v.block == 64 ? 128 : v.block * v.ipt == 256 ? 256 : 512);
     const int64_t tiles = (n_tgt + (int64_t)v.block * v.ipt - 1) / ((int64_t)v.block * v.ipt);
     while (chunk > v.jt && tiles * ((n_src + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
@@ -384,6 +384,14 @@ bool f64_shape(const ForceVariant& v, int64_t n_tgt, bool eps0) {
     return v.block == block && v.ipt == ipt;
 }
 
+// Where a mixed twin is the faster one.  256 x 1 for 64 x 4: small systems, whose 64-thread blocks
+// leave each SM a few warps (N = 3000 15.7 against 21.4 us, N = 8192 47.0 / 47.4, N = 16,384 138 /
+// 134).  512 x 2 for 256 x 4: large ones (N = 262,144 26.7 against 27.0 ms, N = 65,536 1.71 / 1.72,
+// N = 32,768 470 / 454 us).
+bool twin_faster(const ForceVariant& v, int64_t n_tgt, int64_t n_src) {
+    return v.block == 256 ? n_src <= 7000 : n_tgt >= 150000;
+}
+
 // Untuned choice.  FP64: by n_tgt.  Mixed: the wave model over all variants, weighted by each
 // variant's measured per-interaction rate; a mixed variant also fixes the tiles whose centres are
 // the origins of the FP32 offsets, so its choice keeps to the weights of mixed_variant_cost, while
@@ -408,7 +416,7 @@ Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_
     double bc = 1e300;
     for (int k = 0; k < c; ++k) {
         const ForceVariant& v = all[ids[k]];
-        if (precision == kMixed && !v.packed) continue;  // the scalar form is kept for measurement only
+        if (precision == kMixed && (!v.packed || v.twin_of >= 0)) continue;  // scalar: for measurement only
         if (precision == kF64 && !f64_shape(v, n_tgt, eps0)) continue;
         const double cost = precision == kMixed ? mixed_variant_cost(v, n_tgt, n_src, sms) * variant_rate_penalty(v) : 0.0;
         if (cost < bc) {
@@ -416,6 +424,13 @@ Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_
             best.variant = ids[k];
             best.nsplit = best_split(v, n_tgt, n_src, sms);
         }
+    }
+    for (int k = 0; k < c && precision == kMixed; ++k) {  // a twin in place of the chosen variant
+        const ForceVariant& v = all[ids[k]];
+        if (v.twin_of < 0 || v.twin_of != best.variant || !twin_faster(v, n_tgt, n_src)) continue;
+        best.variant = ids[k];
+        best.nsplit = best_split(v, n_tgt, n_src, sms);
+        break;
     }
     return best;
 }
@@ -3344,7 +3359,8 @@ extern "C" int gx_direct_accel_noalloc(int64_t n, const double* x, const double*
     int cnt;
     const ForceVariant* all = force_variants(&cnt);
     Choice ch = heuristic_choice(dev, precision, eps0_of(precision, phys), n, n);
-    ch.nsplit = std::min(ch.nsplit, kNoAllocMaxSplit);
+    // as many chunks as the array holds (kNoAllocMaxSplit at the largest n)
+    ch.nsplit = (int)std::min<int64_t>(ch.nsplit, (int64_t)kNoAllocScratchDoubles / (3 * n));
     const ForceVariant& v = all[ch.variant];
     ForceJob j{x, y, z, m, n, nullptr, 0, n, ax, ay, az, nullptr, nullptr, nullptr, 0.0};
     const ForceArgs a = make_args(j, phys, v, ch.nsplit, scratch);

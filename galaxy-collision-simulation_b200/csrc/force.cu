@@ -118,8 +118,11 @@ const ForceVariant kVariants[] = {
     F64(64, 2, 128, true),
     EXACT(16, 8, 2),
     EXSER(64, 128, 8),
+    // twins of the fifth and the eighth mixed variant: the same tiles over other threads
+    {kMixed, 512, 2, 512, 2, 0, (const void*)&force_mixed_tp_kernel<512, 2, 512, false, 1, 8>, 0, 4},
+    {kMixed, 256, 1, 256, 1, 0, (const void*)&force_mixed_kernel<256, 1, 256, true, false>, 0, 7},
 };
-// Which exact variant (the last two above, in that order) for n_tgt targets.  The serial kernel
+// Which exact variant (the two above, in that order) for n_tgt targets.  The serial kernel
 // needs one thread per target and fills the SMs from 592 warps of targets up; below, and until
 // its second round of warps is well filled, the cooperative one is faster in spite of the terms
 // it passes through shared memory.  Measured with n targets and n sources, cooperative /

@@ -52,7 +52,9 @@ struct ForceVariant {
     int packed;  // 0 scalar FP32, 1 two sources per f32x2, 2 two targets per f32x2
     int eps0;  // guards s == 0 pairs (softening 0)
     const void* fn;
-    int targets = 0;  // targets per CTA where that is not block * ipt (the exact form)
+    int targets = 0;   // targets per CTA where that is not block * ipt (the exact form)
+    int twin_of = -1;  // mixed: the variant with the same target tiles, passes and packing, whose
+                       // results it reproduces bit for bit with another number of threads
 };
 
 // All compiled variants; eps0 variants are separate entries.
