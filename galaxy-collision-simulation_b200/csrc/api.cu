@@ -2748,9 +2748,12 @@ struct gx_batch {
     double* buf = nullptr;
     double *x, *y, *z, *vx, *vy, *vz, *ax, *ay, *az, *m;
     int64_t* off_d = nullptr;
-    int2* items_d = nullptr;
+    int4* items_d = nullptr;
     int n_items = 0;
-    int items_tile = 0;
+    int items_variant = -1;       // the variant the items were made for
+    BatchSplit* split_d = nullptr;
+    double* part = nullptr;       // partial sums of split tiles
+    unsigned* tickets = nullptr;  // one per tile
     int* counter = nullptr;
     int cfg[3] = {-1, -1, -1};
     int2* pot_items_d = nullptr;
@@ -2782,35 +2785,97 @@ int batch_default_variant(gx_batch* b, int precision) {
     return ids[0];
 }
 
-// (instance, tile) items for tiles of `tile` targets, largest instances first.
-int batch_build_items(gx_batch* b, int tile) {
-    if (b->items_tile == tile && b->items_d) return GX_OK;
-    std::vector<int> order((size_t)b->ni);
-    for (int i = 0; i < b->ni; ++i) order[(size_t)i] = i;
-    std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
-        return b->off_h[p + 1] - b->off_h[p] > b->off_h[q + 1] - b->off_h[q];
-    });
-    std::vector<int2> items;
-    for (int inst : order) {
-        const int64_t nb = b->off_h[inst + 1] - b->off_h[inst];
-        const int64_t tiles = (nb + tile - 1) / tile;
-        for (int64_t t = 0; t < tiles; ++t) items.push_back(make_int2(inst, (int)t));
+void batch_free_items(gx_batch* b) {
+    for (void* q : {(void*)b->items_d, (void*)b->split_d, (void*)b->part, (void*)b->tickets})
+        if (q && cudaFreeAsync(q, b->stream) != cudaSuccess) cudaGetLastError();
+    b->items_d = nullptr;
+    b->split_d = nullptr;
+    b->part = nullptr;
+    b->tickets = nullptr;
+    b->items_variant = -1;
+}
+
+// (instance, tile, chunk) items of a variant, costliest first.  The sources of an instance are cut
+// into chunks so that an item is at most a 16th of a resident CTA's share of the launch (or one
+// pass of the shared-memory tile), within part_limit of partial sums; without memory for them the
+// tiles stay whole.  At an 8th / 12th / 16th of a share 128 encounters of 1024 to 16,384 bodies
+// take 5.18 / 5.14 / 5.15 ms (mixed) and 12.83 / 12.58 / 12.45 ms (FP64), 8 of them 360 / 361 /
+// 355 us and 810 / 814 / 765 us; whole tiles 5.49 and 14.0 ms, 1.34 and 1.73 ms.
+constexpr double kBatchItemsPerCta = 16.0;
+
+int batch_build_items(gx_batch* b, int vid, int64_t part_limit = kMaxPartBytes) {
+    if (b->items_variant == vid && b->items_d) return GX_OK;
+    int cnt;
+    const BatchVariant& v = batch_variants(&cnt)[vid];
+    const int64_t tile = (int64_t)v.block * v.ipt;
+    auto bodies = [&](int i) { return b->off_h[(size_t)i + 1] - b->off_h[(size_t)i]; };
+    double total = 0.0;
+    for (int i = 0; i < b->ni; ++i) total += (double)bodies(i) * (double)bodies(i);
+    const double share = total / ((double)sm_count(b->device) * batch_occupancy(v));
+    int64_t want = std::max<int64_t>(1, (int64_t)(share / kBatchItemsPerCta / (double)tile));
+    std::vector<BatchSplit> split((size_t)b->ni);
+    int64_t part = 0, tickets = 0;
+    for (;; want *= 2) {
+        part = tickets = 0;
+        for (int i = 0; i < b->ni; ++i) {
+            const int64_t nb = bodies(i);
+            BatchSplit& s = split[(size_t)i];
+            split_layout(std::max<int64_t>(nb, 1), v.jt, (int)std::min<int64_t>(64, (nb + want - 1) / want), &s.j_chunk,
+                         &s.nsplit);
+            s.part_off = part;
+            s.ticket_off = (int)tickets;
+            if (s.nsplit > 1) part += (int64_t)s.nsplit * 3 * nb;
+            tickets += (nb + tile - 1) / tile;
+        }
+        if (part * (int64_t)sizeof(double) <= part_limit || want > b->n) break;
     }
-    if (items.size() > (size_t)INT32_MAX) return fail(GX_ERR_INVALID_ARGUMENT, "batch: too many work items");
-    if (b->items_d) {
-        cudaStreamSynchronize(b->stream);
-        cudaFree(b->items_d);
-        b->items_d = nullptr;
+    struct Item {
+        int4 w;
+        double cost;
+    };
+    std::vector<Item> list;
+    for (int i = 0; i < b->ni; ++i) {
+        const int64_t nb = bodies(i);
+        for (int64_t t = 0; t < (nb + tile - 1) / tile; ++t)
+            for (int c = 0; c < split[(size_t)i].nsplit; ++c) {
+                const int64_t src = std::min(nb - c * split[(size_t)i].j_chunk, split[(size_t)i].j_chunk);
+                list.push_back({make_int4(i, (int)t, c, 0), (double)std::min(tile, nb - t * tile) * (double)src});
+            }
     }
+    if (list.size() > (size_t)INT32_MAX || tickets > INT32_MAX)
+        return fail(GX_ERR_INVALID_ARGUMENT, "batch: too many work items");
+    std::stable_sort(list.begin(), list.end(), [](const Item& p, const Item& q) { return p.cost > q.cost; });
+    std::vector<int4> items;
+    for (const Item& it : list) items.push_back(it.w);
+    GX_CUDA(cudaStreamSynchronize(b->stream));
+    batch_free_items(b);
     void* p;
-    cudaError_t e = dev_alloc(&p, std::max<size_t>(1, items.size()) * sizeof(int2));
-    if (e != cudaSuccess) return fail_cuda(e, "cudaMalloc (batch items)");
-    b->items_d = (int2*)p;
+    cudaError_t e = cudaSuccess;
+    auto grab = [&](size_t bytes) {
+        p = nullptr;
+        if (e == cudaSuccess) e = dev_alloc_async(&p, std::max<size_t>(16, bytes), b->stream);
+        return p;
+    };
+    b->items_d = (int4*)grab(items.size() * sizeof(int4));
+    b->split_d = (BatchSplit*)grab(split.size() * sizeof(BatchSplit));
+    b->tickets = (unsigned*)grab((size_t)tickets * sizeof(unsigned));
+    const bool bookkeeping = e == cudaSuccess;
+    b->part = (double*)grab((size_t)part * sizeof(double));
+    if (e != cudaSuccess) {
+        batch_free_items(b);
+        if (bookkeeping && part > 0) {
+            cudaGetLastError();
+            return batch_build_items(b, vid, 0);
+        }
+        return fail_cuda(e, "cudaMalloc (batch items)");
+    }
     if (!items.empty())
-        GX_CUDA(cudaMemcpyAsync(b->items_d, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, b->stream));
+        GX_CUDA(cudaMemcpyAsync(b->items_d, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream));
+    GX_CUDA(cudaMemcpyAsync(b->split_d, split.data(), split.size() * sizeof(BatchSplit), cudaMemcpyHostToDevice, b->stream));
+    GX_CUDA(cudaMemsetAsync(b->tickets, 0, std::max<size_t>(16, (size_t)tickets * sizeof(unsigned)), b->stream));
     GX_CUDA(cudaStreamSynchronize(b->stream));
     b->n_items = (int)items.size();
-    b->items_tile = tile;
+    b->items_variant = vid;
     b->clear_graphs();
     return GX_OK;
 }
@@ -2821,6 +2886,10 @@ BatchArgs batch_args(gx_batch* b, double kick_dt) {
     a.offsets = b->off_d;
     a.items = b->items_d;
     a.n_items = b->n_items;
+    a.split = b->split_d;
+    a.part = b->part;
+    a.tickets = b->tickets;
+    a.pot_items = b->pot_items_d;
     a.counter = b->counter;
     a.ax = b->ax; a.ay = b->ay; a.az = b->az;
     a.vx = kick_dt != 0.0 ? b->vx : nullptr;
@@ -2838,7 +2907,7 @@ int batch_force(gx_batch* b, int precision, double kick_dt) {
     if (vid < 0) return fail(GX_ERR_UNSUPPORTED, "batch: precision %d has no batched variant", precision);
     int cnt;
     const BatchVariant& v = batch_variants(&cnt)[vid];
-    GX_TRY(batch_build_items(b, v.block * v.ipt));
+    GX_TRY(batch_build_items(b, vid));
     if (b->n_items == 0) return GX_OK;
     const int grid = std::max(1, std::min(b->n_items, sm_count(b->device) * batch_occupancy(v)));
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -2892,7 +2961,8 @@ void batch_release(gx_batch* b) {
         cudaEventDestroy(ev.second);
     }
     b->clear_graphs();
-    void* ptrs[] = {b->buf, b->off_d, b->items_d, b->counter, b->pot_items_d, b->pot_first_d,
+    batch_free_items(b);
+    void* ptrs[] = {b->buf, b->off_d, b->counter, b->pot_items_d, b->pot_first_d,
                     b->pot_count_d, b->pot_part, b->diag_out};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -3090,7 +3160,7 @@ extern "C" int gx_batch_step(gx_batch* b, int64_t n_steps, double dt, int precis
     if (vid < 0) return fail(GX_ERR_UNSUPPORTED, "%s: no batched variant", fn);
     int cnt;
     const BatchVariant& v = batch_variants(&cnt)[vid];
-    GX_TRY(batch_build_items(b, v.block * v.ipt));
+    GX_TRY(batch_build_items(b, vid));
     uint64_t dtb;
     std::memcpy(&dtb, &dt, sizeof(dtb));
     // The whole multi-step run is one graph (capped at 1024 steps per graph).
@@ -3137,7 +3207,6 @@ extern "C" int gx_batch_diagnostics(gx_batch* b, gx_diagnostics* out) {
     if (!out) return fail(GX_ERR_INVALID_ARGUMENT, "gx_batch_diagnostics: null");
     DeviceGuard g(b->device);
     BatchArgs a = batch_args(b, 0.0);
-    a.items = b->pot_items_d;
     a.n_items = b->n_pot_items;
     GX_CUDA(batch_diagnostics_launch(a, b->n_pot_items, b->ni, b->vx, b->vy, b->vz, b->pot_first_d, b->pot_count_d,
                                      b->pot_part, b->diag_out, b->stream));

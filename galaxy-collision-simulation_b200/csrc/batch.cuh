@@ -6,14 +6,27 @@
 
 namespace gx {
 
+// How an instance's tiles are split over its sources: nsplit chunks of j_chunk, their partial sums
+// from part_off on (nsplit * 3 * bodies doubles) and a ticket per tile from ticket_off on.
+struct BatchSplit {
+    int64_t j_chunk;
+    int64_t part_off;
+    int nsplit;
+    int ticket_off;
+};
+
 struct BatchArgs {
     const double* x;
     const double* y;
     const double* z;
     const double* m;
     const int64_t* offsets;  // n_instances + 1 (device)
-    const int2* items;       // (instance, tile) work items, in execution order (device)
+    const int4* items;       // (instance, tile, chunk, -) work items, in execution order (device)
     int n_items;
+    const BatchSplit* split; // per instance (device)
+    double* part;            // partial sums of split tiles
+    unsigned* tickets;       // zero before the first launch, left zero by every launch
+    const int2* pot_items;   // (instance, tile) of the potential (device)
     int* counter;            // ticket counter, zeroed before every launch (device)
     double* ax;
     double* ay;
@@ -43,7 +56,7 @@ int batch_occupancy(const BatchVariant& v);
 cudaError_t batch_force_launch(const BatchVariant& v, const BatchArgs& args, int grid,
                                cudaStream_t st);
 
-// Diagnostics per instance.  pot_args.items lists (instance, tile) items of
+// Diagnostics per instance.  pot_args.pot_items lists (instance, tile) items of
 // batch_potential_tile() targets; item_first/item_count give each instance's items.
 int batch_potential_tile();
 cudaError_t batch_diagnostics_launch(const BatchArgs& pot_args, int n_pot_items,

@@ -23,37 +23,6 @@ __global__ void __launch_bounds__(256) force_reduce_kernel(const ForceArgs a) {
     write_result(a, t, target_body(a, t), a.G * s[0], a.G * s[1], a.G * s[2]);
 }
 
-// Fused reduction, run by every CTA after its tile body has written its partial sums: the
-// CTA that takes the tile's last ticket adds the tile's nsplit partials in chunk order --
-// the sums force_reduce_kernel forms -- and writes the results.  Each thread fences its
-// own partial stores before the ticket is taken; the last CTA reads the partials from L2
-// (ld.global.cg), so no stale L1 line can be seen.  No CTA waits for another.
-template <int BLOCK, int IPT>
-__device__ __forceinline__ void finish_tile(const ForceArgs& a, const int64_t tile, const int64_t t0) {
-    if (a.nsplit <= 1 || !a.tile_count) return;
-    __shared__ unsigned s_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&a.tile_count[tile], 1u) == (unsigned)a.nsplit - 1u;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-#pragma unroll
-    for (int k = 0; k < IPT; ++k) {
-        const int64_t t = t0 + k * BLOCK + threadIdx.x;
-        if (t >= a.n_tgt) continue;
-        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-        for (int c = 0; c < a.nsplit; ++c) {
-            const size_t base = (size_t)c * 3 * (size_t)a.n_tgt + (size_t)t;
-            s0 += __ldcg(a.part + base);
-            s1 += __ldcg(a.part + base + (size_t)a.n_tgt);
-            s2 += __ldcg(a.part + base + 2 * (size_t)a.n_tgt);
-        }
-        write_result(a, t, target_body(a, t), a.G * s0, a.G * s1, a.G * s2);
-    }
-    if (threadIdx.x == 0) a.tile_count[tile] = 0u;
-}
-
 template <int BLOCK, int IPT, int JT, bool PACKED, bool EPS0>
 __global__ void __launch_bounds__(BLOCK) force_mixed_kernel(const ForceArgs a) {
     const int64_t tile = blockIdx.x / a.nsplit;

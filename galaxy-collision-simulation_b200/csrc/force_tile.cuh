@@ -72,6 +72,37 @@ __device__ __forceinline__ void write_partial(const ForceArgs& a, int chunk, int
     a.part[base + 2 * (size_t)a.n_tgt] = sz;
 }
 
+// Fused reduction, run by every CTA after its tile body has written its partial sums: the
+// CTA that takes the tile's last ticket adds the tile's nsplit partials in chunk order --
+// the sums force_reduce_kernel forms -- and writes the results.  Each thread fences its
+// own partial stores before the ticket is taken; the last CTA reads the partials from L2
+// (ld.global.cg), so no stale L1 line can be seen.  No CTA waits for another.
+template <int BLOCK, int IPT>
+__device__ __forceinline__ void finish_tile(const ForceArgs& a, const int64_t tile, const int64_t t0) {
+    if (a.nsplit <= 1 || !a.tile_count) return;
+    __shared__ unsigned s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(&a.tile_count[tile], 1u) == (unsigned)a.nsplit - 1u;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+#pragma unroll
+    for (int k = 0; k < IPT; ++k) {
+        const int64_t t = t0 + k * BLOCK + threadIdx.x;
+        if (t >= a.n_tgt) continue;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+        for (int c = 0; c < a.nsplit; ++c) {
+            const size_t base = (size_t)c * 3 * (size_t)a.n_tgt + (size_t)t;
+            s0 += __ldcg(a.part + base);
+            s1 += __ldcg(a.part + base + (size_t)a.n_tgt);
+            s2 += __ldcg(a.part + base + 2 * (size_t)a.n_tgt);
+        }
+        write_result(a, t, target_body(a, t), a.G * s0, a.G * s1, a.G * s2);
+    }
+    if (threadIdx.x == 0) a.tile_count[tile] = 0u;
+}
+
 
 // ---------------------------------------------------------------------------------------
 // Mixed precision.
@@ -270,8 +301,10 @@ __device__ __forceinline__ void mixed_tile(const ForceArgs& a, const int64_t t0,
 // memory already duplicated ((x, x, y, y), (z, z, m, m): two 16-byte loads per source), so a
 // target pair keeps one 64-bit register per coordinate and per accumulator instead of two:
 // 6 registers fewer per target, which buys occupancy or more targets per thread.
+// ORG: targets per origin when that is a multiple of the CTA's own tile (0: the tile); the origin,
+// and with it every bit of the result, is then that of a CTA with the whole ORG targets.
 // ---------------------------------------------------------------------------------------
-template <int BLOCK, int IPT, int JT, bool EPS0, int UNROLL = 4>
+template <int BLOCK, int IPT, int JT, bool EPS0, int UNROLL = 4, int ORG = 0>
 __device__ __forceinline__ void mixed_tp_tile(const ForceArgs& a, const int64_t t0, const int chunk) {
     static_assert(JT % BLOCK == 0 && BLOCK % 32 == 0 && IPT % 2 == 0, "tile shape");
     constexpr int NW = BLOCK / 32;
@@ -295,6 +328,20 @@ __device__ __forceinline__ void mixed_tp_tile(const ForceArgs& a, const int64_t 
         lo[0] = fmin(lo[0], bx[k]); hi[0] = fmax(hi[0], bx[k]);
         lo[1] = fmin(lo[1], by[k]); hi[1] = fmax(hi[1], by[k]);
         lo[2] = fmin(lo[2], bz[k]); hi[2] = fmax(hi[2], bz[k]);
+    }
+    if constexpr (ORG != 0) {  // the other targets that share the origin
+        static_assert(ORG % (BLOCK * IPT) == 0, "whole tiles share an origin");
+        const int64_t g0 = t0 / ORG * ORG;
+        for (int64_t t = g0 + tid; t < min(g0 + ORG, a.n_tgt); t += BLOCK) {
+            if (t >= t0 && t < t0 + BLOCK * IPT) continue;
+            const int64_t i = target_body(a, t);
+            const double v[3] = {a.x[i], a.y[i], a.z[i]};
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = fmin(lo[c], v[c]);
+                hi[c] = fmax(hi[c], v[c]);
+            }
+        }
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -360,8 +407,7 @@ __device__ __forceinline__ void mixed_tp_tile(const ForceArgs& a, const int64_t 
         f2 PX[NP], PY[NP], PZ[NP];
 #pragma unroll
         for (int q = 0; q < NP; ++q) PX[q] = PY[q] = PZ[q] = Z0;
-#pragma unroll UNROLL
-        for (int jj = 0; jj < JT; ++jj) {
+        const auto source = [&](const int jj) {
             f2 X, Y, Z, M;
             lds_v2b64(reinterpret_cast<const float*>(&sA[jj]), X, Y);
             lds_v2b64(reinterpret_cast<const float*>(&sB[jj]), Z, M);
@@ -388,6 +434,16 @@ __device__ __forceinline__ void mixed_tp_tile(const ForceArgs& a, const int64_t 
                 PY[q] = fma2(dY, W, PY[q]);
                 PZ[q] = fma2(dZ, W, PZ[q]);
             }
+        };
+        if constexpr (ORG != 0) {  // many short chunks: without the massless rest of a last pass
+            static_assert(JT % UNROLL == 0, "whole groups of sources");
+            const int cnt = (int)min((int64_t)JT, je - j0);
+            for (int jg = 0; jg < cnt; jg += UNROLL)
+#pragma unroll
+                for (int u = 0; u < UNROLL; ++u) source(jg + u);
+        } else {
+#pragma unroll UNROLL
+            for (int jj = 0; jj < JT; ++jj) source(jj);
         }
 #pragma unroll
         for (int q = 0; q < NP; ++q) {
@@ -422,7 +478,7 @@ __device__ __forceinline__ void mixed_tp_tile(const ForceArgs& a, const int64_t 
 // 2.48 ms = 1008 Gint/s, 95% of the measured pipe rate; 2.68 ms with one wave of blocks, 2.94 ms
 // with the rsqrt refined first and cubed after (17 operations) as well.
 // ---------------------------------------------------------------------------------------
-template <int BLOCK, int IPT, int JT, bool EPS0>
+template <int BLOCK, int IPT, int JT, bool EPS0, bool SHORT = false>
 __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, const int chunk) {
     static_assert(JT % BLOCK == 0 && JT % 2 == 0, "tile shape");
     __shared__ __align__(16) double sx[JT];
@@ -459,8 +515,7 @@ __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, c
             sm[jj] = in ? a.m[j] : 0.0;
         }
         __syncthreads();
-#pragma unroll 4
-        for (int jj = 0; jj < JT; ++jj) {
+        const auto source = [&](const int jj) {
             const double qx = sx[jj], qy = sy[jj], qz = sz[jj], qm = sm[jj];
 #pragma unroll
             for (int k = 0; k < IPT; ++k) {
@@ -474,6 +529,15 @@ __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, c
                 fy[k] = fma(dy, w, fy[k]);
                 fz[k] = fma(dz, w, fz[k]);
             }
+        };
+        if constexpr (SHORT) {  // many short chunks: without the massless rest of a last pass
+            const int cnt = (int)min((int64_t)JT, je - j0);
+            for (int jg = 0; jg < cnt; jg += 4)
+#pragma unroll
+                for (int u = 0; u < 4; ++u) source(jg + u);
+        } else {
+#pragma unroll 4
+            for (int jj = 0; jj < JT; ++jj) source(jj);
         }
         __syncthreads();
     }
