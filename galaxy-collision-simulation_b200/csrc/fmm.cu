@@ -467,17 +467,26 @@ __global__ void __launch_bounds__(256) fmm_rec32_kernel(const FmmArgs a) {
     reinterpret_cast<float4*>(a.rec32 + (size_t)k * kRec32)[p] = v;
 }
 
-// Shared-memory stride of a staged node record, in elements: slots 0..45 of an FP64 record
-// (16-byte multiple), or a whole mixed record.
-template <typename T>
-__host__ __device__ constexpr int stage_stride() { return sizeof(T) == 8 ? 46 : kRec32; }
 constexpr int kM2PSub = 64;     // node records per shared-memory buffer
 constexpr int kM2PStages = 2;   // buffers in the cp.async ring
-template <typename T>
-constexpr size_t m2p_dyn_smem() { return (size_t)kM2PStages * kM2PSub * stage_stride<T>() * sizeof(T); }
+// Elements of a node record that an order reads, staged in 16-byte pieces one after the other, and
+// the records that a warp stages at once with a lane per piece.
+template <int P, typename T>
+__host__ __device__ constexpr int m2p_pieces() {
+    constexpr int elems = sizeof(T) == 8 ? (P == 0 ? 4 : P == 2 ? kRecTrQ + 1 : 46)
+                                         : (P == 0 ? 7 : P == 2 ? kRecTrQ + 4 : kRecTr2 + 4);
+    return (elems * (int)sizeof(T) + 15) / 16;
+}
+template <int P, typename T>
+__host__ __device__ constexpr int m2p_per_pass() {
+    int n = 1;
+    while (2 * n * m2p_pieces<P, T>() <= 32) n *= 2;
+    return n;
+}
+template <int P, typename T>
+constexpr size_t m2p_dyn_smem() { return (size_t)kM2PStages * kM2PSub * m2p_pieces<P, T>() * 16; }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+__device__ __forceinline__ void cp_async16(const unsigned s, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
@@ -491,22 +500,32 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // most W - 1 threads idle); a buffer is filled with a multiple of S records, so every slot
 // evaluates the same number of nodes between barriers.  The S partial sums of a target are
 // added in slot order, so results do not depend on scheduling.
+// A lane copies one 16-byte piece of a record per pass (two mixed records or one FP64 record per
+// warp), and reads its list entries one buffer ahead.  The mixed form is bound by instruction issue:
+// N = 2^20 leaf 16 (624 M pairs, five targets per leaf: a record is staged for every five pairs)
+// 7.04 ms, against 7.72 with pieces dealt out over the block (15 instructions each, and list
+// reads just before the copies); seven blocks per SM take 0.1 to 0.3 ms less than six or eight.
+// A ring per warp, without block barriers, took 7.9 ms: records shared by two warps are copied
+// twice, and its steps cost more instructions than the barriers.  FP64 is bound by its pipe
+// (66 %): N = 65,536 leaf 64 231 us either way.
 template <int P, typename T>
-__global__ void __launch_bounds__(kM2PBlock) fmm_m2p_kernel(const FmmArgs a) {
-    // record elements the order reads, staged in 16-byte pieces
+__global__ void __launch_bounds__(kM2PBlock, (sizeof(T) == 4 ? 7 : 4)) fmm_m2p_kernel(const FmmArgs a) {
     constexpr bool F64 = sizeof(T) == 8;
-    constexpr int kElems = F64 ? (P == 0 ? 4 : P == 2 ? kRecTrQ + 1 : 46) : (P == 0 ? 7 : P == 2 ? kRecTrQ + 4 : kRecTr2 + 4);
-    constexpr int PIECES = (kElems * (int)sizeof(T) + 15) / 16;
-    constexpr int kPer = 16 / (int)sizeof(T);  // elements per piece
-    constexpr int kStride = stage_stride<T>();
-    constexpr int kGlobal = F64 ? kFmmRec : kRec32;  // record stride in global memory
-    const T* rec = F64 ? reinterpret_cast<const T*>(a.rec) : reinterpret_cast<const T*>(a.rec32);
+    constexpr int PIECES = m2p_pieces<P, T>();
+    constexpr int kStride = PIECES * 16 / (int)sizeof(T);  // elements of a staged record
+    constexpr size_t kGlobal = (size_t)(F64 ? kFmmRec : kRec32) * sizeof(T);  // bytes of a record
+    constexpr int kPerPass = m2p_per_pass<P, T>(), kBlockPass = kM2PBlock / 32 * kPerPass;
+    constexpr int kPasses = (kM2PSub + kBlockPass - 1) / kBlockPass;
+    const char* rec = F64 ? reinterpret_cast<const char*>(a.rec) : reinterpret_cast<const char*>(a.rec32);
     const T eps2 = F64 ? (T)a.eps2 : (T)a.eps2f;
     extern __shared__ __align__(16) unsigned char s_raw[];
-    T* s_dyn = reinterpret_cast<T*>(s_raw);
     __shared__ double s_red[kM2PBlock * 3];
     __shared__ int s_last;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
+    // the record and piece that the lane stages of each pass
+    const int rl = lane < kPerPass * PIECES ? (tid >> 5) * kPerPass + lane / PIECES : kM2PSub;
+    const char* const rec_piece = rec + 16 * (lane % PIECES);
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(s_raw) + rl * (PIECES * 16) + 16 * (lane % PIECES);
     if (a.overflow && *a.overflow) return;
     const int n_items = fmm_items(a);
     for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
@@ -519,19 +538,26 @@ __global__ void __launch_bounds__(kM2PBlock) fmm_m2p_kernel(const FmmArgs a) {
         const int q = tid / W, tl = tid - q * W;
         const int R = S <= kM2PSub ? S * (kM2PSub / S) : kM2PSub;  // records per buffer
         const int nsub = (cnt + R - 1) / R;
+        // the nodes of the lane's records of a buffer, read one buffer ahead of the copies
+        int node[kPasses];
+        auto nodes_of = [&](int sc) {
+            const int m = min(R, cnt - sc * R);
+            const int* const list = a.far_node + w.fb + sc * R + rl;
+#pragma unroll
+            for (int u = 0; u < kPasses; ++u)
+                if (rl + u * kBlockPass < m) node[u] = __ldg(list + u * kBlockPass);
+        };
         // fills buffer sc % kM2PStages with records sc * R ..; one commit group per call, empty
         // past the end, so that the waits below count groups uniformly
         auto stage = [&](int sc) {
-            if (sc < nsub) {
-                T* buf = s_dyn + (sc % kM2PStages) * (kM2PSub * kStride);
-                const int j0 = sc * R, m = min(R, cnt - j0);
-                for (int k = tid; k < m * PIECES; k += kM2PBlock) {
-                    const int j = k / PIECES, pc = k - j * PIECES;
-                    const T* src = rec + (size_t)a.far_node[w.fb + j0 + j] * kGlobal + kPer * pc;
-                    cp_async16(buf + j * kStride + kPer * pc, src);
-                }
-            }
+            const int m = min(R, cnt - sc * R);
+            const unsigned to = dst + (sc % kM2PStages) * (kM2PSub * PIECES * 16);
+#pragma unroll
+            for (int u = 0; u < kPasses; ++u)
+                if (rl + u * kBlockPass < m)
+                    cp_async16(to + u * (kBlockPass * PIECES * 16), rec_piece + (size_t)(unsigned)node[u] * kGlobal);
             cp_async_commit();
+            nodes_of(sc + 1);
         };
         for (int t0 = 0; t0 < nt; t0 += W) {
             const int t = t0 + tl;
@@ -548,12 +574,13 @@ __global__ void __launch_bounds__(kM2PBlock) fmm_m2p_kernel(const FmmArgs a) {
                     i = -1;
                 }
             }
+            nodes_of(0);
             for (int sc = 0; sc < kM2PStages - 1; ++sc) stage(sc);
             for (int sc = 0; sc < nsub; ++sc) {
                 stage(sc + kM2PStages - 1);  // into the buffer released at the end of sc - 1
                 cp_async_wait<kM2PStages - 1>();
                 __syncthreads();
-                const T* buf = s_dyn + (sc % kM2PStages) * (kM2PSub * kStride);
+                const T* buf = reinterpret_cast<const T*>(s_raw) + (sc % kM2PStages) * (kM2PSub * kStride);
                 const int m = min(R, cnt - sc * R);
                 if (i >= 0)
                     for (int j = q; j < m; j += S) m2p_one<P>(buf + j * kStride, tx, ty, tz, eps2, fx, fy, fz);
@@ -617,7 +644,7 @@ template <int P, typename T>
 cudaError_t launch_m2p_order(const FmmArgs& a, cudaStream_t st) {
     // the shared-memory opt-in is a per-device setting of the kernel
     static std::atomic<unsigned long long> set_on{0};
-    constexpr size_t smem = m2p_dyn_smem<T>();
+    constexpr size_t smem = m2p_dyn_smem<P, T>();
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
