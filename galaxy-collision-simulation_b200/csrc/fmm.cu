@@ -547,8 +547,7 @@ __global__ void __launch_bounds__(kM2PBlock, (sizeof(T) == 4 ? 7 : 4)) fmm_m2p_k
             for (int u = 0; u < kPasses; ++u)
                 if (rl + u * kBlockPass < m) node[u] = __ldg(list + u * kBlockPass);
         };
-        // fills buffer sc % kM2PStages with records sc * R ..; one commit group per call, empty
-        // past the end, so that the waits below count groups uniformly
+        // fills buffer sc % kM2PStages with records sc * R ..
         auto stage = [&](int sc) {
             const int m = min(R, cnt - sc * R);
             const unsigned to = dst + (sc % kM2PStages) * (kM2PSub * PIECES * 16);
@@ -575,18 +574,16 @@ __global__ void __launch_bounds__(kM2PBlock, (sizeof(T) == 4 ? 7 : 4)) fmm_m2p_k
                 }
             }
             nodes_of(0);
-            for (int sc = 0; sc < kM2PStages - 1; ++sc) stage(sc);
+            stage(0);
             for (int sc = 0; sc < nsub; ++sc) {
-                stage(sc + kM2PStages - 1);  // into the buffer released at the end of sc - 1
-                cp_async_wait<kM2PStages - 1>();
-                __syncthreads();
+                cp_async_wait<0>();
+                __syncthreads();  // buffer sc is complete, and every thread is done with buffer sc - 1
+                if (sc + 1 < nsub) stage(sc + 1);
                 const T* buf = reinterpret_cast<const T*>(s_raw) + (sc % kM2PStages) * (kM2PSub * kStride);
                 const int m = min(R, cnt - sc * R);
                 if (i >= 0)
                     for (int j = q; j < m; j += S) m2p_one<P>(buf + j * kStride, tx, ty, tz, eps2, fx, fy, fz);
-                __syncthreads();  // a later stage() overwrites this buffer
             }
-            cp_async_wait<0>();  // the empty trailing groups
             s_red[tid * 3 + 0] = (double)fx;
             s_red[tid * 3 + 1] = (double)fy;
             s_red[tid * 3 + 2] = (double)fz;

@@ -138,19 +138,23 @@ __global__ void __launch_bounds__(256) p2p_off_scatter_kernel(const P2PArgs a, c
     if (k < nl) a.plan_item_off[ord[k]] = a.plan_off_sorted[k];
 }
 
-// The whole plan order in one block when the leaf table is small (at most kSmallPlan entries):
-// leaves by decreasing item-cost key (a counting sort on the 7-bit keys; leaves with equal keys
-// land in no fixed order, which changes only the order in which items are handed out, never a
-// sum), the item counts in that order, their exclusive scan (plan_off_sorted and each leaf's
-// first item), and the exclusive scan of the partial-sum needs in leaf order.  It replaces a
-// radix sort, two scans and two scatter kernels -- about nine launches -- with one.
+// The whole plan in one block when the leaf table is small (at most kSmallPlan entries): the leaves'
+// splits (unless p2p_count_kernel has made them), leaves by decreasing item-cost key (a counting
+// sort on the 7-bit keys; leaves with equal keys land in no fixed order, which changes only the
+// order in which items are handed out, never a sum), the exclusive scan of their item counts in
+// that order (plan_off_sorted and each leaf's first item), the item -> leaf table, the exclusive
+// scan of the partial-sum needs in leaf order, and the counters of the leaf kernel.  Only the
+// leaves there are now count, not the capacity of the table; a thread scans a run of them, so each
+// scan takes one round of barriers.  Latency-bound: N = 65,536 leaf 64 TIME_P us (table of 12,700
+// entries, 4,700 leaves) against 52 us in a count kernel, this one over the whole table, an item
+// kernel and two clears; N = 1000 TIME_Q us against 15.
 constexpr int kSmallPlan = 16384;
 constexpr int kSmallPlanThreads = 1024;
 
-// Exclusive scan of v over the block (kSmallPlanThreads threads); *carry holds the running
-// total of the earlier chunks and is advanced.  Ends with a barrier.
+// Exclusive scan of one v per thread over the block (kSmallPlanThreads threads); *total its sum.
+// Ends with a barrier.
 template <typename T>
-__device__ __forceinline__ T block_exclusive_scan(T v, T* s_warp, T* carry) {
+__device__ __forceinline__ T block_exclusive_scan(T v, T* s_warp, T* total) {
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     T x = v;
     for (int o = 1; o < 32; o <<= 1) {
@@ -168,58 +172,71 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* s_warp, T* carry) {
         s_warp[lane] = z;
     }
     __syncthreads();
-    const T incl = x + (w > 0 ? s_warp[w - 1] : T(0)) + *carry;
+    const T ex = x - v + (w > 0 ? s_warp[w - 1] : T(0));
+    *total = s_warp[31];
     __syncthreads();
-    if (t == kSmallPlanThreads - 1) *carry = incl;
-    __syncthreads();
-    return incl - v;
+    return ex;
 }
 
-__global__ void __launch_bounds__(kSmallPlanThreads) p2p_small_plan_kernel(const P2PArgs a, int* ord_sorted, int nl) {
+__global__ void __launch_bounds__(kSmallPlanThreads) p2p_small_plan_kernel(const P2PArgs a, int* ord_sorted, int counted,
+                                                                           int exact, int64_t item_cost) {
     __shared__ int s_bin[128];
     __shared__ int s_wi[32];
     __shared__ long long s_wl[32];
-    __shared__ int s_ci;
-    __shared__ long long s_cl;
     const int t = threadIdx.x;
+    const int nl = p2p_leaves_now(a);
     if (t < 128) s_bin[t] = 0;
-    if (t == 0) {
-        s_ci = 0;
-        s_cl = 0;
+    if (t == 0) *a.ticket = 0;
+    __syncthreads();
+    for (int k = t; k < nl; k += kSmallPlanThreads) {
+        if (!counted) plan_leaf(a, k, nl, a.near_src[k], exact, item_cost);
+        a.plan_done[k] = 0;
+        atomicAdd(&s_bin[a.plan_key[k] & 127], 1);
     }
     __syncthreads();
-    for (int k = t; k < nl; k += kSmallPlanThreads) atomicAdd(&s_bin[a.plan_key[k] & 127], 1);
-    __syncthreads();
-    if (t == 0) {  // bin starts, largest key first
-        int run = 0;
-        for (int b = 127; b >= 0; --b) {
-            const int c = s_bin[b];
-            s_bin[b] = run;
-            run += c;
+    if (t < 32) {  // bin starts, largest key first: lane t holds bins 127 - 4 t .. 124 - 4 t
+        int c[4], sum = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) sum += c[u] = s_bin[127 - 4 * t - u];
+        int run = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, run, o);
+            if (t >= o) run += y;
+        }
+        run -= sum;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            s_bin[127 - 4 * t - u] = run;
+            run += c[u];
         }
     }
     __syncthreads();
-    for (int k = t; k < nl; k += kSmallPlanThreads) {  // plan_ord is the identity here
+    for (int k = t; k < nl; k += kSmallPlanThreads) {
         const int pos = atomicAdd(&s_bin[a.plan_key[k] & 127], 1);
         ord_sorted[pos] = k;
         a.plan_cnt_sorted[pos] = a.plan_cnt[k];
     }
     __syncthreads();
-    for (int c0 = 0; c0 < nl; c0 += kSmallPlanThreads) {
-        const int k = c0 + t;
-        const int v = k < nl ? a.plan_cnt_sorted[k] : 0;
-        const int ex = block_exclusive_scan<int>(v, s_wi, &s_ci);
-        if (k < nl) {
-            a.plan_off_sorted[k] = ex;
-            a.plan_item_off[ord_sorted[k]] = ex;
-        }
+    const int per = (nl + kSmallPlanThreads - 1) / kSmallPlanThreads;
+    const int k0 = min(t * per, nl), k1 = min(k0 + per, nl);
+    int items = 0, n_items;
+    long long need = 0, n_need;
+    for (int k = k0; k < k1; ++k) {
+        items += a.plan_cnt_sorted[k];
+        need += a.plan_need[k];
     }
-    for (int c0 = 0; c0 < nl; c0 += kSmallPlanThreads) {
-        const int k = c0 + t;
-        const long long v = k < nl ? (long long)a.plan_need[k] : 0;
-        const long long ex = block_exclusive_scan<long long>(v, s_wl, &s_cl);
-        if (k < nl) a.plan_scratch[k] = (int64_t)ex;
+    items = block_exclusive_scan<int>(items, s_wi, &n_items);
+    need = block_exclusive_scan<long long>(need, s_wl, &n_need);
+    for (int k = k0; k < k1; ++k) {
+        const int l = ord_sorted[k], c = a.plan_cnt_sorted[k];
+        a.plan_off_sorted[k] = items;
+        a.plan_item_off[l] = items;
+        for (int q = 0; q < c && items + q < a.plan_item_cap; ++q) a.plan_item_leaf[items + q] = l;
+        items += c;
+        a.plan_scratch[k] = (int64_t)need;
+        need += a.plan_need[k];
     }
+    if (t == 0) *a.plan_n_items = n_items;
 }
 
 // The leaf of every item: item plan_item_off[l] + k belongs to leaf l (k < plan_cnt[l]).  One
@@ -322,7 +339,7 @@ __global__ void __launch_bounds__(BS, p2p_threads_per_sm(MODE, TPT) / BS) p2p_ke
         if (item < a.plan_item_cap) {
             leaf = a.plan_item_leaf[item];
         } else {
-            int lo = 0, hi = a.n_leaves;  // largest k with plan_off_sorted[k] <= item
+            int lo = 0, hi = p2p_leaves_now(a);  // largest k with plan_off_sorted[k] <= item
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
                 if (a.plan_off_sorted[mid] <= item) lo = mid;
@@ -799,24 +816,28 @@ cudaError_t launch_p2p(P2PArgs a, int64_t n_bodies, int precision, void* scratch
     const int forced = g_p2p_tpt.load();
     const int tpt = forced ? forced : 2;
     const int64_t item_cost = (int64_t)1024 * bs;
-    cudaError_t e = cudaMemsetAsync(a.plan_done, 0, nl * 4, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a.ticket, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-    p2p_gather_kernel<<<sms * 8, 256, 0, st>>>(a, n_bodies);
-    const int exact = precision == kF64Exact ? 1 : 0;
-    if (a.near_src) p2p_count_src_kernel<<<(a.n_leaves + 256) / 256, 256, 0, st>>>(a, exact, item_cost);
-    else p2p_count_kernel<<<(a.n_leaves + 8) / 8, 256, 0, st>>>(a, exact, item_cost);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     // With few items per block, the leaves by decreasing item cost and the items numbered in
     // that order: without it the last items handed out can be the largest, and at
     // N = 65,536 leaf 64 (3011 leaves, 740 blocks) the SMs sat idle for 18% of the P2P kernel.
     // With many items per block the tail is small and the sort (four launches) is skipped,
     // except in the exact form, whose leaves are never split (N = 2^20 leaf 16: 17 ms sorted,
     // 28 ms in leaf order).
-    size_t tb = temp_bytes;
     const bool sorted = precision == kF64Exact || leaves_est <= 16 * 4 * sms;
-    if (sorted && nl <= (size_t)kSmallPlan) {
-        p2p_small_plan_kernel<<<1, kSmallPlanThreads, 0, st>>>(a, ord_sorted, (int)nl);
+    const bool small = sorted && nl <= (size_t)kSmallPlan;
+    const int exact = precision == kF64Exact ? 1 : 0;
+    cudaError_t e = cudaSuccess;
+    if (!small) {
+        e = cudaMemsetAsync(a.plan_done, 0, nl * 4, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(a.ticket, 0, sizeof(int), st);
+        if (e != cudaSuccess) return e;
+    }
+    p2p_gather_kernel<<<sms * 8, 256, 0, st>>>(a, n_bodies);
+    if (!a.near_src) p2p_count_kernel<<<(a.n_leaves + 8) / 8, 256, 0, st>>>(a, exact, item_cost);
+    else if (!small) p2p_count_src_kernel<<<(a.n_leaves + 256) / 256, 256, 0, st>>>(a, exact, item_cost);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    size_t tb = temp_bytes;
+    if (small) {
+        p2p_small_plan_kernel<<<1, kSmallPlanThreads, 0, st>>>(a, ord_sorted, a.near_src ? 0 : 1, exact, item_cost);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         a.plan_ord = ord_sorted;
     } else if (sorted) {
@@ -839,13 +860,13 @@ cudaError_t launch_p2p(P2PArgs a, int64_t n_bodies, int precision, void* scratch
             return e;
         a.plan_off_sorted = a.plan_item_off;
     }
-    if (!(sorted && nl <= (size_t)kSmallPlan)) {  // the small plan kernel scanned the needs already
+    if (!small) {
         tb = temp_bytes;
         if ((e = cub::DeviceScan::ExclusiveSum(temp, tb, a.plan_need, a.plan_scratch, (int)nl, st)) != cudaSuccess)
             return e;
+        p2p_item_leaf_kernel<<<(a.n_leaves + 255) / 256, 256, 0, st>>>(a);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    p2p_item_leaf_kernel<<<(a.n_leaves + 255) / 256, 256, 0, st>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (precision == kF64Exact) return launch_bs<kF64Exact, false>(a, bs, 2, sms, st);
     if (precision == kF64)
         return eps0 ? launch_bs<kF64, true>(a, bs, tpt, sms, st) : launch_bs<kF64, false>(a, bs, tpt, sms, st);
