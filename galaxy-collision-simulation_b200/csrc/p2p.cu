@@ -65,7 +65,8 @@ __device__ __forceinline__ void plan_none(const P2PArgs& a, int l) {
     a.plan_ord[l] = l;
 }
 
-__device__ __forceinline__ void plan_leaf(const P2PArgs& a, int l, int nl, int64_t src, int exact, int64_t item_cost) {
+__device__ __forceinline__ void plan_leaf(const P2PArgs& a, int l, int nl, int64_t src, int exact, int64_t item_cost,
+                                          int min_chunk = kMinChunk) {
     const int nt = a.leaf_off[l + 1] - a.leaf_off[l];
     int chunks = 0, groups = 1;
     if (nt > 0 && src > 0) {
@@ -78,7 +79,7 @@ __device__ __forceinline__ void plan_leaf(const P2PArgs& a, int l, int nl, int64
             groups = (int)((nt + g - 1) / g);
             g = (nt + groups - 1) / groups;  // equal groups
             const int64_t c_cost = (src * (g + kStageCost) + item_cost - 1) / item_cost;
-            const int64_t c_src = (src + kMinChunk - 1) / kMinChunk;
+            const int64_t c_src = (src + min_chunk - 1) / min_chunk;
             chunks = (int)max((int64_t)1, min((int64_t)kMaxChunks, min(c_cost, c_src)));
             if (a.leaf_off[nl] > a.split_max_slots) chunks = 1;
         }
@@ -145,11 +146,18 @@ __global__ void __launch_bounds__(256) p2p_off_scatter_kernel(const P2PArgs a, c
 // that order (plan_off_sorted and each leaf's first item), the item -> leaf table, the exclusive
 // scan of the partial-sum needs in leaf order, and the counters of the leaf kernel.  Only the
 // leaves there are now count, not the capacity of the table; a thread scans a run of them, so each
-// scan takes one round of barriers.  Latency-bound: N = 65,536 leaf 64 TIME_P us (table of 12,700
-// entries, 4,700 leaves) against 52 us in a count kernel, this one over the whole table, an item
-// kernel and two clears; N = 1000 TIME_Q us against 15.
+// scan takes one round of barriers.  Latency-bound: N = 65,536 leaf 64 17 us (table of 12,700
+// entries) against 52 us in a count kernel, this one over the whole table, an item
+// kernel and two clears; N = 1000 6 us against 15.
 constexpr int kSmallPlan = 16384;
 constexpr int kSmallPlanThreads = 1024;
+// FP64 items of few bodies: the cost of an item falls to the total / resident blocks, so that a small
+// system's leaves still occupy the chip (the mixed form keeps its chunks, which group FP32 sums).
+// Whole evaluation, N = 1000 leaf 16: 335 -> 311 us, N = 4000 leaf 64: 488 -> 426, N = 16,000 leaf
+// 64: 590 -> 547, N = 65,536 unchanged; two and four items per block take 437 and 460 us at
+// N = 4000 leaf 64.
+constexpr int kFillMinCost = 1024;
+constexpr int kFillMinChunk = 64;
 
 // Exclusive scan of one v per thread over the block (kSmallPlanThreads threads); *total its sum.
 // Ends with a barrier.
@@ -179,7 +187,7 @@ __device__ __forceinline__ T block_exclusive_scan(T v, T* s_warp, T* total) {
 }
 
 __global__ void __launch_bounds__(kSmallPlanThreads) p2p_small_plan_kernel(const P2PArgs a, int* ord_sorted, int counted,
-                                                                           int exact, int64_t item_cost) {
+                                                                           int exact, int64_t item_cost, int fill) {
     __shared__ int s_bin[128];
     __shared__ int s_wi[32];
     __shared__ long long s_wl[32];
@@ -188,8 +196,17 @@ __global__ void __launch_bounds__(kSmallPlanThreads) p2p_small_plan_kernel(const
     if (t < 128) s_bin[t] = 0;
     if (t == 0) *a.ticket = 0;
     __syncthreads();
+    int min_chunk = kMinChunk;
+    if (fill > 0) {  // smaller items when there is less than one of the usual cost per resident block
+        long long cost = 0, total;
+        for (int k = t; k < nl; k += kSmallPlanThreads)
+            cost += (long long)a.near_src[k] * (a.leaf_off[k + 1] - a.leaf_off[k] + kStageCost);
+        block_exclusive_scan<long long>(cost, s_wl, &total);
+        item_cost = min((long long)item_cost, max((long long)kFillMinCost, total / fill));
+        min_chunk = kFillMinChunk;
+    }
     for (int k = t; k < nl; k += kSmallPlanThreads) {
-        if (!counted) plan_leaf(a, k, nl, a.near_src[k], exact, item_cost);
+        if (!counted) plan_leaf(a, k, nl, a.near_src[k], exact, item_cost, min_chunk);
         a.plan_done[k] = 0;
         atomicAdd(&s_bin[a.plan_key[k] & 127], 1);
     }
@@ -837,7 +854,8 @@ cudaError_t launch_p2p(P2PArgs a, int64_t n_bodies, int precision, void* scratch
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     size_t tb = temp_bytes;
     if (small) {
-        p2p_small_plan_kernel<<<1, kSmallPlanThreads, 0, st>>>(a, ord_sorted, a.near_src ? 0 : 1, exact, item_cost);
+        p2p_small_plan_kernel<<<1, kSmallPlanThreads, 0, st>>>(a, ord_sorted, a.near_src ? 0 : 1, exact, item_cost,
+                                                               a.near_src && precision == kF64 ? sms * (640 / bs) : 0);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         a.plan_ord = ord_sorted;
     } else if (sorted) {
