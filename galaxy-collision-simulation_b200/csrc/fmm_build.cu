@@ -78,15 +78,25 @@ __global__ void __launch_bounds__(kBboxThreads) bbox_partial_kernel(const TreeBu
     }
 }
 
-// Root cell (fmm_solver.cpp:62-85): one block reduces the partial extrema.
-__global__ void __launch_bounds__(kBboxThreads) bbox_final_kernel(const TreeBuildArgs t, int blocks) {
+__device__ __forceinline__ int octant_of(double x, double y, double z, double cx, double cy, double cz) {
+    return (x >= cx ? 1 : 0) + (y >= cy ? 2 : 0) + (z >= cz ? 4 : 0);
+}
+
+// Child centre (subdivide, fmm_solver.cpp:111-131): centre + sign * (half_width * 0.5).
+__device__ __forceinline__ double child_centre(double c, double chw, bool up) { return dadd(c, up ? chw : -chw); }
+
+// Root cell (fmm_solver.cpp:62-85) from the partial extrema -- every block reduces them for itself
+// (minima and maxima do not depend on the order), block 0 stores it -- and the path keys.  Block 0
+// also clears the build's flags and the ticket of split_count_kernel.
+__global__ void __launch_bounds__(kBboxThreads) keys_kernel(const TreeBuildArgs t, int blocks, int* ticket) {
+    __shared__ double s[6][kBboxThreads / 32];
+    __shared__ double s_root[4];
     double lo[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, hi[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
     for (int b = threadIdx.x; b < blocks; b += kBboxThreads)
         for (int c = 0; c < 3; ++c) {
             lo[c] = fmin(lo[c], t.part[b * 6 + c]);
             hi[c] = fmax(hi[c], t.part[b * 6 + 3 + c]);
         }
-    __shared__ double s[6][kBboxThreads / 32];
     for (int c = 0; c < 3; ++c) {
         lo[c] = warp_min(lo[c]);
         hi[c] = warp_max(hi[c]);
@@ -98,42 +108,39 @@ __global__ void __launch_bounds__(kBboxThreads) bbox_final_kernel(const TreeBuil
             s[3 + c][w] = hi[c];
         }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int c = 0; c < 3; ++c)
-        for (int k = 1; k < kBboxThreads / 32; ++k) {
-            s[c][0] = fmin(s[c][0], s[c][k]);
-            s[3 + c][0] = fmax(s[3 + c][0], s[3 + c][k]);
+    if (threadIdx.x == 0) {
+        for (int c = 0; c < 3; ++c)
+            for (int k = 1; k < kBboxThreads / 32; ++k) {
+                s[c][0] = fmin(s[c][0], s[c][k]);
+                s[3 + c][0] = fmax(s[3 + c][0], s[3 + c][k]);
+            }
+        for (int c = 0; c < 3; ++c) s_root[c] = dmul(dadd(s[c][0], s[3 + c][0]), 0.5);
+        double hw = dmul(0.5, fmax(fmax(dsub(s[3][0], s[0][0]), dsub(s[4][0], s[1][0])), dsub(s[5][0], s[2][0])));
+        hw = fmax(hw, dadd(t.softening, 1.0e-6));
+        s_root[3] = dmul(hw, 1.0001);
+        if (blockIdx.x == 0) {
+            for (int c = 0; c < 4; ++c) t.root[c] = s_root[c];
+            for (int c = 0; c < 3; ++c) t.hdr[c] = 0;
+            *ticket = 0;
         }
-    for (int c = 0; c < 3; ++c) t.root[c] = dmul(dadd(s[c][0], s[3 + c][0]), 0.5);
-    double hw = dmul(0.5, fmax(fmax(dsub(s[3][0], s[0][0]), dsub(s[4][0], s[1][0])), dsub(s[5][0], s[2][0])));
-    hw = fmax(hw, dadd(t.softening, 1.0e-6));
-    t.root[3] = dmul(hw, 1.0001);
-}
-
-__device__ __forceinline__ int octant_of(double x, double y, double z, double cx, double cy, double cz) {
-    return (x >= cx ? 1 : 0) + (y >= cy ? 2 : 0) + (z >= cz ? 4 : 0);
-}
-
-// Child centre (subdivide, fmm_solver.cpp:111-131): centre + sign * (half_width * 0.5).
-__device__ __forceinline__ double child_centre(double c, double chw, bool up) { return dadd(c, up ? chw : -chw); }
-
-__global__ void __launch_bounds__(256) keys_kernel(const TreeBuildArgs t) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= t.n) return;
-    const double x = t.x[i], y = t.y[i], z = t.z[i];
-    double cx = t.root[0], cy = t.root[1], cz = t.root[2], hw = t.root[3];
-    uint64_t key = 0;
-    for (int l = 0; l < kKeyLevels; ++l) {
-        const int o = octant_of(x, y, z, cx, cy, cz);
-        key |= (uint64_t)o << (3 * (kKeyLevels - 1 - l));
-        const double chw = dmul(hw, 0.5);
-        cx = child_centre(cx, chw, o & 1);
-        cy = child_centre(cy, chw, o & 2);
-        cz = child_centre(cz, chw, o & 4);
-        hw = chw;
     }
-    t.keys[i] = key;
-    t.idx[i] = i;
+    __syncthreads();
+    for (int i = blockIdx.x * kBboxThreads + threadIdx.x; i < t.n; i += gridDim.x * kBboxThreads) {
+        const double x = t.x[i], y = t.y[i], z = t.z[i];
+        double cx = s_root[0], cy = s_root[1], cz = s_root[2], hw = s_root[3];
+        uint64_t key = 0;
+        for (int l = 0; l < kKeyLevels; ++l) {
+            const int o = octant_of(x, y, z, cx, cy, cz);
+            key |= (uint64_t)o << (3 * (kKeyLevels - 1 - l));
+            const double chw = dmul(hw, 0.5);
+            cx = child_centre(cx, chw, o & 1);
+            cy = child_centre(cy, chw, o & 2);
+            cz = child_centre(cz, chw, o & 4);
+            hw = chw;
+        }
+        t.keys[i] = key;
+        t.idx[i] = i;
+    }
 }
 
 // First position p in [b, e) whose octant at shift sh is >= o (octants are non-decreasing
@@ -151,13 +158,18 @@ __device__ __forceinline__ int lower_octant(const uint64_t* keys, int b, int e, 
 // L octants (key >> 3 (kKeyLevels - L)); it splits when it holds more than cap bodies and
 // L < max_depth, and a splitting node's 8 children (all of them, empty ones included) are
 // the nodes of depth L + 1.  Nodes are numbered breadth-first with children in octant order,
-// i.e. level by level in key-prefix order, so a node's number follows from counts alone:
-//   flags[L n + i] = 1 when sorted body i is the first body of a splitting depth-L prefix,
-//   E = exclusive scan of flags over all levels (kKeyLevels n + 1 entries, in place),
-//   S_L = splitting nodes of depth L = E[(L + 1) n] - E[L n],
-//   level_off[L + 1] = level_off[L] + 8 S_(L-1)  (level_off[0] = 0, level_off[1] = 1),
-//   the rank of body i's depth-L prefix among the splitting ones = E[L n + i] - E[L n],
-//   and its children start at level_off[L + 1] + 8 rank.
+// i.e. level by level in key-prefix order, so a node's number follows from counts alone.  Sorted
+// body i is the first of a splitting prefix for the depths [lo, hi] where lo - 1 octants are common
+// to it and body i - 1, and hi octants to it and body i + cap (SplitRange), so
+//   split_count_kernel counts the splitting prefixes per depth and block of bodies, and its last
+//   block scans the counts: S_L, level_off[L + 1] = level_off[L] + 8 S_(L-1) (level_off[0] = 0,
+//   level_off[1] = 1), and each block's first rank of every depth;
+//   split_emit_kernel ranks them by ballots and lists them in (depth, key) order with their own
+//   node's number, which the rank of their parent's prefix gives;
+//   tree_children_kernel writes the children's records, from level_off[L + 1] + 8 rank on.
+// Latency-bound, so what counts is launches and dependent loads: N = 65,536 leaf 64 30 us for the
+// three, N = 1000 26 and N = 2^20 leaf 16 52, against 62, 45 and 130 us with a flag per body
+// and depth, a scan of all of them (22 M at N = 2^20) and binary searches over whole prefixes.
 // A node's centre is the reference's recurrence (subdivide, fmm_solver.cpp:111-131) walked
 // from the root along its prefix -- the same operations in the same order as building level
 // by level, so the same bits.  A prefix of depth kKeyLevels that would still split needs a
@@ -170,92 +182,178 @@ __device__ __forceinline__ uint64_t key_prefix(uint64_t key, int L) {
     return sh >= 64 ? 0 : key >> sh;
 }
 
-// Position one past the last body of the depth-L prefix that starts at sorted body i:
-// galloping from i, then a binary search in the last gap (log of the prefix's size).
-__device__ __forceinline__ int prefix_end(const uint64_t* keys, int n, int i, int L) {
-    const uint64_t p = key_prefix(keys[i], L);
-    int lo = i + 1, step = 1;  // keys[lo - 1] has prefix p
-    while (lo < n && key_prefix(keys[lo], L) == p) {
-        const int nxt = lo + step;
-        if (nxt >= n || key_prefix(keys[nxt], L) != p) {
-            int b = lo + 1, e = min(nxt, n);  // first mismatch in (lo, nxt]
-            while (b < e) {
-                const int mid = (b + e) >> 1;
-                if (key_prefix(keys[mid], L) == p) b = mid + 1;
-                else e = mid;
+// Leading octants that two keys have in common.
+__device__ __forceinline__ int common_levels(uint64_t p, uint64_t q) {
+    return p == q ? kKeyLevels : (__clzll((long long)(p ^ q)) - 1) / 3;
+}
+
+// Depths at which sorted body i starts a splitting prefix (hi < lo: none).  flags: what the build
+// cannot do, as hdr[2] bits -- a prefix of all kKeyLevels that would split (1), or one at a depth
+// whose children the sort has not ordered (4).
+struct SplitRange {
+    int lo, hi, flags;
+    __device__ __forceinline__ SplitRange(const TreeBuildArgs& t, const uint64_t* keys, int i) : lo(0), hi(-1), flags(0) {
+        if (i >= t.n || (int64_t)i + t.cap >= (int64_t)t.n) return;
+        const int sorted = t.key_levels > 0 ? t.key_levels : kKeyLevels;  // levels the sort ordered
+        const int lmax = min(t.max_depth, kKeyLevels + 1);
+        const uint64_t key = keys[i];
+        if (i > 0) lo = common_levels(key, keys[i - 1]) + 1;
+        hi = min(common_levels(key, keys[i + t.cap]), lmax - 1);
+        if (lo <= kKeyLevels && hi >= kKeyLevels) flags |= 1;
+        hi = min(hi, kKeyLevels - 1);
+        if (lo <= hi && hi >= sorted) flags |= 4;
+        hi = min(hi, sorted - 1);
+    }
+};
+
+// Depths in which any body of a warp starts a splitting prefix (hi < lo: none).
+__device__ __forceinline__ int2 warp_depths(const SplitRange& r) {
+    const bool any = r.lo <= r.hi;
+    return make_int2(__reduce_min_sync(0xffffffffu, any ? r.lo : kKeyLevels),
+                     __reduce_max_sync(0xffffffffu, any ? r.hi : -1));
+}
+
+constexpr int kTopoThreads = 256;
+constexpr int kTopoPer = 4;                                   // bodies per thread
+constexpr int kTopoBodies = kTopoThreads * kTopoPer;          // ... and per block
+constexpr int kTopoGroups = kTopoBodies / 32;                 // groups of 32 bodies (one ballot each)
+static_assert(kTopoGroups == 32, "a warp scans the groups of a block");
+
+// What split_count_kernel leaves for the other two: start[L] = splitting prefixes above depth L
+// (start[kKeyLevels]: all), first[L * blocks + b] = rank at depth L of block b's first.
+struct Topology {
+    int* ticket;
+    int* start;  // kKeyLevels + 1
+    int* first;  // kKeyLevels * blocks
+    int2* split; // (first body, node) in (depth, key) order
+    int blocks;
+    int split_cap;
+};
+
+__global__ void __launch_bounds__(kTopoThreads) split_count_kernel(const TreeBuildArgs t, const uint64_t* keys,
+                                                                   const Topology p) {
+    __shared__ int s_cnt[kKeyLevels][kTopoGroups];
+    __shared__ int s_total[kKeyLevels];
+    __shared__ int s_last;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    for (int k = tid; k < kKeyLevels * kTopoGroups; k += kTopoThreads) (&s_cnt[0][0])[k] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kTopoPer; ++u) {
+        const SplitRange r(t, keys, blockIdx.x * kTopoBodies + u * kTopoThreads + tid);
+        if (r.flags) atomicOr(&t.hdr[2], r.flags);
+        const int2 d = warp_depths(r);
+        for (int L = d.x; L <= d.y; ++L) {
+            const unsigned m = __ballot_sync(0xffffffffu, r.lo <= L && L <= r.hi);
+            if (lane == 0) s_cnt[L][u * (kTopoThreads / 32) + w] = __popc(m);
+        }
+    }
+    __syncthreads();
+    for (int L = w; L < kKeyLevels; L += kTopoThreads / 32) {
+        const int c = __reduce_add_sync(0xffffffffu, s_cnt[L][lane]);
+        if (lane == 0) p.first[(size_t)L * p.blocks + blockIdx.x] = c;
+    }
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) s_last = atomicAdd(p.ticket, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    // the last block: exclusive scans over the blocks, a warp per depth
+    for (int L = w; L < kKeyLevels; L += kTopoThreads / 32) {
+        int* const f = p.first + (size_t)L * p.blocks;
+        int carry = 0;
+#pragma unroll 4
+        for (int b = lane; b - lane < p.blocks; b += 32) {
+            const int c = b < p.blocks ? __ldcg(f + b) : 0;
+            int run = c;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, run, o);
+                if (lane >= o) run += y;
             }
-            return b;
+            if (b < p.blocks) f[b] = carry + run - c;
+            carry += __shfl_sync(0xffffffffu, run, 31);
         }
-        lo = nxt + 1;
-        step <<= 1;
+        if (lane == 0) s_total[L] = carry;
     }
-    return lo;
+    __syncthreads();
+    if (w != 0) return;
+    // lane L: depth L; S_L = 0 ends the tree
+    const int c = lane < kKeyLevels ? s_total[lane] : 0;
+    int64_t run = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += y;
+    }
+    if (lane <= kKeyLevels) p.start[lane] = (int)(run - c);
+    const int deep = __ffs(__ballot_sync(0xffffffffu, c == 0)) - 1;  // depths with splitting nodes
+    const int64_t off = 1 + 8 * run;
+    const int32_t off32 = off <= 0x7fffffffLL ? (int32_t)off : 0x7fffffff;
+    if (lane < deep) t.level_off[lane + 2] = off32;
+    if (lane == deep) {  // run: all of them
+        t.level_off[0] = 0;
+        t.level_off[1] = 1;
+        t.level_off[deep + 2] = off32;
+        t.hdr[0] = off32;
+        t.hdr[1] = deep + 1;
+        if (off > t.capacity) atomicOr(&t.hdr[2], 2);
+    }
 }
 
-__device__ __forceinline__ bool prefix_first(const uint64_t* keys, int i, int L) {
-    return i == 0 || key_prefix(keys[i], L) != key_prefix(keys[i - 1], L);
-}
-
-// flags[L n + i] = 1 when sorted body i starts a depth-L prefix holding more than cap bodies
-// (it does exactly when body i + cap shares the prefix: the keys are sorted) and L < max_depth.
-__global__ void __launch_bounds__(256) split_flags_kernel(const TreeBuildArgs t, const uint64_t* keys, int32_t* flags) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i == 0) flags[(size_t)kKeyLevels * t.n] = 0;
-    if (i >= t.n) return;
-    const int lmax = min(t.max_depth, kKeyLevels + 1);
-    const int sorted = t.key_levels > 0 ? t.key_levels : kKeyLevels;  // levels the sort ordered
-    const uint64_t key = keys[i];
-    const bool big = (int64_t)i + t.cap < (int64_t)t.n;
-    const uint64_t far = big ? keys[i + t.cap] : 0;
-    for (int L = 0; L <= kKeyLevels; ++L) {
-        bool split = false;
-        if (L < lmax && big && prefix_first(keys, i, L) && key_prefix(far, L) == key_prefix(key, L)) {
-            if (L == kKeyLevels) atomicOr(&t.hdr[2], 1);
-            else if (L >= sorted) atomicOr(&t.hdr[2], 4);  // the children need deeper sorted keys
-            else split = true;
+// The splitting nodes in (depth, key) order; every node starts as a leaf (child -1); the root's record.
+__global__ void __launch_bounds__(kTopoThreads) split_emit_kernel(const TreeBuildArgs t, const uint64_t* keys,
+                                                                  const Topology p) {
+    __shared__ int s_cnt[kKeyLevels][kTopoGroups];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    SplitRange r[kTopoPer] = {{t, keys, (int)blockIdx.x * kTopoBodies + tid},
+                              {t, keys, (int)blockIdx.x * kTopoBodies + kTopoThreads + tid},
+                              {t, keys, (int)blockIdx.x * kTopoBodies + 2 * kTopoThreads + tid},
+                              {t, keys, (int)blockIdx.x * kTopoBodies + 3 * kTopoThreads + tid}};
+    for (int k = tid; k < kKeyLevels * kTopoGroups; k += kTopoThreads) (&s_cnt[0][0])[k] = 0;
+    __syncthreads();
+    int2 d[kTopoPer];
+#pragma unroll
+    for (int u = 0; u < kTopoPer; ++u) {
+        d[u] = warp_depths(r[u]);
+        for (int L = d[u].x; L <= d[u].y; ++L) {
+            const unsigned m = __ballot_sync(0xffffffffu, r[u].lo <= L && L <= r[u].hi);
+            if (lane == 0) s_cnt[L][u * (kTopoThreads / 32) + w] = __popc(m);
         }
-        if (L < kKeyLevels) flags[(size_t)L * t.n + i] = split ? 1 : 0;
     }
-}
-
-// One thread: level offsets, node and level counts from the scanned flags.
-__global__ void tree_levels_kernel(const TreeBuildArgs t, const int32_t* E) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const size_t n = (size_t)t.n;
-    int64_t off = 1;
-    int levels = 1;
-    t.level_off[0] = 0;
-    t.level_off[1] = 1;
-    for (int L = 0; L < kKeyLevels; ++L) {
-        const int64_t s = (int64_t)E[(L + 1) * n] - (int64_t)E[L * n];
-        if (s == 0) break;
-        off += 8 * s;
-        t.level_off[L + 2] = off <= 0x7fffffffLL ? (int32_t)off : 0x7fffffff;
-        ++levels;
+    __syncthreads();
+    for (int L = w; L < kKeyLevels; L += kTopoThreads / 32) {  // rank of each group's first
+        const int c = s_cnt[L][lane];
+        int run = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += y;
+        }
+        s_cnt[L][lane] = p.first[(size_t)L * p.blocks + blockIdx.x] + run - c;
     }
-    t.level_off[levels + 1] = t.level_off[levels];
-    t.hdr[0] = t.level_off[levels];
-    t.hdr[1] = levels;
-    if (off > t.capacity) atomicOr(&t.hdr[2], 2);
-}
-
-// The splitting nodes in global (level, key) order: split_pos[E[L n + i]] = L n + i.
-__global__ void __launch_bounds__(256) split_list_kernel(const TreeBuildArgs t, const int32_t* E, int32_t* split_pos,
-                                                         int split_cap) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i >= t.n) return;
-    const size_t n = (size_t)t.n;
-    for (int L = 0; L < kKeyLevels; ++L) {
-        const int32_t e0 = E[L * n + i];
-        if (E[L * n + i + 1] != e0 && e0 < split_cap) split_pos[e0] = L * t.n + i;
+    __syncthreads();
+    const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+    for (int u = 0; u < kTopoPer; ++u) {
+        const int i = blockIdx.x * kTopoBodies + u * kTopoThreads + tid;
+        const int g = u * (kTopoThreads / 32) + w;
+        // splitting prefixes one depth up that start at or before body i
+        int parents = d[u].x > 0 && d[u].x < kKeyLevels ? s_cnt[d[u].x - 1][g] : 0;
+        for (int L = d[u].x; L <= d[u].y; ++L) {
+            const bool mine = r[u].lo <= L && L <= r[u].hi;
+            const unsigned m = __ballot_sync(0xffffffffu, mine);
+            const int rank = s_cnt[L][g] + __popc(m & below);
+            if (mine) {
+                const int e = p.start[L] + rank;
+                int self = 0;
+                if (L > 0) self = t.level_off[L] + 8 * (parents - 1) + (int)((keys[i] >> (3 * (kKeyLevels - L))) & 7);
+                if (e < p.split_cap) p.split[e] = make_int2(i, self);
+            }
+            parents = rank + (mine ? 1 : 0);
+        }
     }
-}
-
-// Every node starts as a leaf (child -1); the root's record.
-__global__ void __launch_bounds__(256) tree_init_kernel(const TreeBuildArgs t) {
     const int nodes = min(t.hdr[0], t.capacity);
-    for (int k = blockIdx.x * 256 + threadIdx.x; k < nodes; k += gridDim.x * 256) t.child[k] = -1;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    for (int k = blockIdx.x * kTopoThreads + tid; k < nodes; k += gridDim.x * kTopoThreads) t.child[k] = -1;
+    if (blockIdx.x == 0 && tid == 0) {
         t.beg[0] = 0;
         t.end[0] = t.n;
         t.cx[0] = t.root[0];
@@ -265,30 +363,41 @@ __global__ void __launch_bounds__(256) tree_init_kernel(const TreeBuildArgs t) {
     }
 }
 
-// One thread per (splitting node, child octant c): the node's child index (c == 0) and child
-// c's record -- its body range by binary search on the octant at depth L inside the node's
-// range, its centre by the reference's recurrence walked from the root along the path.
-__global__ void __launch_bounds__(256) tree_children_kernel(const TreeBuildArgs t, const uint64_t* keys,
-                                                            const int32_t* E, const int32_t* split_pos, int split_cap) {
+// Eight lanes per splitting node: its end by a search with eight probes a round, each child's first
+// body by binary search on the octant inside the node's range, and the children's records, their
+// centres by the reference's recurrence walked from the root along the path.
+__global__ void __launch_bounds__(256) tree_children_kernel(const TreeBuildArgs t, const uint64_t* keys, const Topology p) {
     if (t.hdr[2] & 2) return;
-    const size_t n = (size_t)t.n;
-    const int total = min(E[kKeyLevels * n], split_cap);
-    for (int q = blockIdx.x * 256 + threadIdx.x; q < 8 * total; q += gridDim.x * 256) {
-        const int sidx = q >> 3, c = q & 7;
-        const int pos = split_pos[sidx];
-        const int L = pos / t.n, i = pos - L * t.n;
-        const uint64_t key = keys[i];
-        int self = 0;
-        if (L > 0) {
-            const int parent_rank = E[(L - 1) * n + i + 1] - E[(L - 1) * n] - 1;
-            self = t.level_off[L] + 8 * parent_rank + (int)((key >> (3 * (kKeyLevels - L))) & 7);
+    __shared__ int s_start[kKeyLevels + 1];
+    if (threadIdx.x <= kKeyLevels) s_start[threadIdx.x] = p.start[threadIdx.x];
+    __syncthreads();
+    const int total = min(s_start[kKeyLevels], p.split_cap);
+    const int lane = threadIdx.x & 31, c = lane & 7;
+    const unsigned group = 0xffu << (lane & 24);
+    for (int64_t q = (int64_t)blockIdx.x * 256 + threadIdx.x; q < 8 * (int64_t)total; q += (int64_t)gridDim.x * 256) {
+        const int k = (int)(q >> 3);
+        int L = 0;
+        while (L < kKeyLevels - 1 && s_start[L + 1] <= k) ++L;
+        const int2 sp = p.split[k];
+        const int i = sp.x;
+        const uint64_t key = keys[i], prefix = key_prefix(key, L);
+        // bodies i .. i + cap share the prefix; keys[lo - 1] has it, keys[hi] (if any) has not
+        int lo = i + (int)t.cap + 1, hi = t.n;
+        while (lo < hi) {
+            const int step = (hi - lo + 7) >> 3;
+            const int64_t at = lo + (int64_t)c * step;
+            const bool same = at < hi && key_prefix(keys[at], L) == prefix;
+            const int m = __popc(__ballot_sync(group, same) & group);
+            if (m == 0) break;
+            hi = (int)min((int64_t)hi, lo + (int64_t)m * step);
+            lo += (m - 1) * step + 1;
         }
-        const int c0 = t.level_off[L + 1] + 8 * (sidx - E[L * n]);
-        if (c == 0) t.child[self] = c0;
-        const int e = prefix_end(keys, t.n, i, L);
+        const int e = lo;
         const int sh = 3 * (kKeyLevels - 1 - L);
         const int cb = c == 0 ? i : lower_octant(keys, i, e, sh, c);
-        const int ce = c == 7 ? e : lower_octant(keys, cb, e, sh, c + 1);
+        __syncwarp(group);
+        const int next = __shfl_sync(group, cb, (lane & 24) | ((c + 1) & 7));
+        const int ce = c == 7 ? e : next;
         double cx = t.root[0], cy = t.root[1], cz = t.root[2], hw = t.root[3];
         for (int d = 0; d < L; ++d) {
             const int o = (int)((key >> (3 * (kKeyLevels - 1 - d))) & 7);
@@ -298,6 +407,8 @@ __global__ void __launch_bounds__(256) tree_children_kernel(const TreeBuildArgs 
             cz = child_centre(cz, hw, o & 4);
         }
         const double chw = dmul(hw, 0.5);
+        const int c0 = t.level_off[L + 1] + 8 * (k - s_start[L]);
+        if (c == 0) t.child[sp.y] = c0;
         t.beg[c0 + c] = cb;
         t.end[c0 + c] = ce;
         t.cx[c0 + c] = child_centre(cx, chw, c & 1);
@@ -992,10 +1103,9 @@ size_t scan_bytes(int count) {
 
 }  // namespace
 
-// Temporary storage of launch_tree_build: the split flags / their scan (kKeyLevels n + 1 ints),
-// the list of splitting nodes (at most kKeyLevels (n / (cap + 1) + 1): the depth-L prefixes that
-// split hold more than cap bodies each and are disjoint), then the radix sort's or the scan's
-// own storage (one after the other, sharing the space).
+// Temporary storage of launch_tree_build: ticket and depth starts, each block's first ranks, the
+// list of splitting nodes (at most kKeyLevels (n / (cap + 1) + 1): the depth-L prefixes that
+// split hold more than cap bodies each and are disjoint), then the radix sort's own storage.
 namespace {
 int split_capacity(int32_t n, int64_t cap) {
     const int64_t c = (int64_t)kKeyLevels * ((int64_t)n / (std::max<int64_t>(cap, 0) + 1) + 1);
@@ -1003,34 +1113,40 @@ int split_capacity(int32_t n, int64_t cap) {
 }
 }  // namespace
 
+namespace {
+size_t aligned(size_t b) { return (b + 255) & ~(size_t)255; }
+int topo_blocks(int32_t n) { return (n + kTopoBodies - 1) / kTopoBodies; }
+constexpr size_t kTopoHead = 256;  // ticket and kKeyLevels + 1 starts
+static_assert((kKeyLevels + 2) * sizeof(int) <= kTopoHead, "head of the build's scratch");
+}  // namespace
+
 size_t tree_build_temp_bytes(int32_t n, int64_t cap) {
     size_t b = 0;
     cub::DoubleBuffer<uint64_t> k(nullptr, nullptr);
     cub::DoubleBuffer<int32_t> v(nullptr, nullptr);
     cub::DeviceRadixSort::SortPairs(nullptr, b, k, v, n, 0, 3 * kKeyLevels);
-    size_t sb = 0;
-    const int items = kKeyLevels * n + 1;
-    cub::DeviceScan::ExclusiveSum(nullptr, sb, (int32_t*)nullptr, (int32_t*)nullptr, items);
-    const size_t flags = ((size_t)items * sizeof(int32_t) + 255) & ~(size_t)255;
-    const size_t splits = ((size_t)split_capacity(n, cap) * sizeof(int32_t) + 255) & ~(size_t)255;
-    return flags + splits + std::max((b + 255) & ~(size_t)255, sb);
+    return kTopoHead + aligned((size_t)kKeyLevels * topo_blocks(n) * sizeof(int)) +
+           aligned((size_t)split_capacity(n, cap) * sizeof(int2)) + aligned(b);
 }
 
 cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_bytes, cudaStream_t st) {
-    const int items = kKeyLevels * t.n + 1;
-    const size_t flag_bytes = ((size_t)items * sizeof(int32_t) + 255) & ~(size_t)255;
-    const int split_cap = split_capacity(t.n, t.cap);
-    const size_t split_bytes = ((size_t)split_cap * sizeof(int32_t) + 255) & ~(size_t)255;
-    int32_t* flags = (int32_t*)temp;
-    int32_t* split_pos = (int32_t*)((char*)temp + flag_bytes);
-    void* work = (char*)temp + flag_bytes + split_bytes;
-    size_t work_bytes = temp_bytes - flag_bytes - split_bytes;
-    cudaError_t e = cudaMemsetAsync(t.hdr, 0, 3 * sizeof(int32_t), st);
+    Topology p;
+    p.blocks = topo_blocks(t.n);
+    p.split_cap = split_capacity(t.n, t.cap);
+    p.ticket = (int*)temp;
+    p.start = p.ticket + 1;
+    const size_t firsts = aligned((size_t)kKeyLevels * p.blocks * sizeof(int));
+    p.first = (int*)((char*)temp + kTopoHead);
+    p.split = (int2*)((char*)temp + kTopoHead + firsts);
+    const size_t used = kTopoHead + firsts + aligned((size_t)p.split_cap * sizeof(int2));
+    void* work = (char*)temp + used;
+    size_t work_bytes = temp_bytes - used;
+    const int gn = (t.n + kBboxThreads - 1) / kBboxThreads;
+    const int bbox_blocks = std::min(gn, kBboxBlocks);
+    bbox_partial_kernel<<<bbox_blocks, kBboxThreads, 0, st>>>(t);
+    keys_kernel<<<std::min(gn, 148 * 8), kBboxThreads, 0, st>>>(t, bbox_blocks, p.ticket);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    bbox_partial_kernel<<<kBboxBlocks, kBboxThreads, 0, st>>>(t);
-    bbox_final_kernel<<<1, kBboxThreads, 0, st>>>(t, kBboxBlocks);
-    keys_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(t);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     cub::DoubleBuffer<uint64_t> k(t.keys, t.keys_alt);
     cub::DoubleBuffer<int32_t> v(t.idx, t.perm);
     const int sorted = t.key_levels > 0 ? std::min(t.key_levels, kKeyLevels) : kKeyLevels;
@@ -1038,14 +1154,9 @@ cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_by
                                              st)) != cudaSuccess)
         return e;
     if (v.Current() != t.perm) gather_perm_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(v.Current(), t.perm, t.n);
-    split_flags_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(t, k.Current(), flags);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    work_bytes = temp_bytes - flag_bytes - split_bytes;
-    if ((e = cub::DeviceScan::ExclusiveSum(work, work_bytes, flags, flags, items, st)) != cudaSuccess) return e;
-    tree_levels_kernel<<<1, 32, 0, st>>>(t, flags);
-    split_list_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(t, flags, split_pos, split_cap);
-    tree_init_kernel<<<148 * 4, 256, 0, st>>>(t);
-    tree_children_kernel<<<148 * 8, 256, 0, st>>>(t, k.Current(), flags, split_pos, split_cap);
+    split_count_kernel<<<p.blocks, kTopoThreads, 0, st>>>(t, k.Current(), p);
+    split_emit_kernel<<<p.blocks, kTopoThreads, 0, st>>>(t, k.Current(), p);
+    tree_children_kernel<<<148 * 8, 256, 0, st>>>(t, k.Current(), p);
     return cudaGetLastError();
 }
 
