@@ -1874,10 +1874,8 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     la.t_begin = begin;
     la.t_end = end;
     const int64_t nb = n + 1, lb = (int64_t)P.n_nodes + 1;
-    GX_TRY(dev_array(hs, nb, &la.start_flag));
-    GX_TRY(dev_array(hs, nb, &la.start_ord));
-    GX_TRY(dev_array(hs, nb, &la.keep));
-    GX_TRY(dev_array(hs, nb, &la.newpos));
+    GX_TRY(dev_array(hs, nb, &la.mark));
+    GX_TRY(dev_array(hs, nb, &la.place));
     GX_TRY(dev_array(hs, lb, &la.leaf_off));
     GX_TRY(dev_array(hs, n, &la.leaf_part));
     GX_TRY(dev_array(hs, lb, &la.leaf_node));
@@ -1916,7 +1914,7 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
         GX_TRY(dev_array(hs, la.seg_cap, &la.seg_count));
         GX_CUDA(launch_tree_lists(la, list_temp, list_bytes, sm_count(dev), st));
         int m2m_err = 0;
-        GX_CUDA(cudaMemcpyAsync(&nl, la.start_ord + n, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GX_CUDA(cudaMemcpyAsync(&nl, leaf_count_of(la), sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaMemcpyAsync(&tot, la.counters, sizeof(tot), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaMemcpyAsync(&m2m_err, m2m, sizeof(int), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaStreamSynchronize(st));
@@ -2282,7 +2280,7 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     la.seg_cap = w.seg_cap;
     la.walk_stack = fmm_walk_stack();
     la.slot_cap = w.slot_cap;
-    for (int32_t** q : {&la.start_flag, &la.start_ord, &la.keep, &la.newpos}) GX_TRY(w.grab(n + 1, q));
+    for (int64_t** q : {&la.mark, &la.place}) GX_TRY(w.grab(n + 1, q));
     GX_TRY(w.grab((int64_t)NC + 1, &la.leaf_off));
     GX_TRY(w.grab(n, &la.leaf_part));
     GX_TRY(w.grab((int64_t)NC + 1, &la.leaf_node));
@@ -2311,7 +2309,7 @@ int fmm_work_create(std::unique_ptr<FmmWork>& W, int64_t n, gx_physics phys, gx_
     GX_TRY(w.grab((int64_t)w.order_bytes, (char**)&w.order_temp));
 
     fa.n_leaves = NC;
-    fa.cnt_leaves = la.start_ord + n;
+    fa.cnt_leaves = leaf_count_of(la);
     fa.leaf_off = la.leaf_off;
     fa.leaf_part = la.leaf_part;
     fa.far_node = la.far_node;
@@ -2380,7 +2378,7 @@ int fmm_work_enqueue(FmmWork& w, const double* x, const double* y, const double*
     pa.leaf_off = la.leaf_off; pa.leaf_part = la.leaf_part; pa.near_beg = la.near_beg; pa.near_end = la.near_end; pa.near_leaf = la.near_leaf;
     pa.near_src = la.near_src;
     pa.n_leaves = w.node_cap;
-    pa.cnt_leaves = la.start_ord + n;
+    pa.cnt_leaves = leaf_count_of(la);
     pa.overflow = w.flags;
     pa.leaves_hint = w.leaves_hint;
     pa.ax = nx; pa.ay = ny; pa.az = nz;

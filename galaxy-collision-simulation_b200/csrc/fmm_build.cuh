@@ -94,10 +94,8 @@ struct TreeListArgs {
     int walk_stack;     // at most kWalkStackSlots: where a walk's stack counts as overflowing
     int64_t t_begin, t_end;
     // body-position scratch, n + 1 each
-    int32_t* start_flag;
-    int32_t* start_ord;
-    int32_t* keep;
-    int32_t* newpos;
+    int64_t* mark;   // bodies of leaves with mass > 0: 1 in the high word, the leaf's first also in the low
+    int64_t* place;  // its exclusive scan: place among those bodies, leaves before
     // leaves, n_nodes + 1 each
     int32_t* leaf_off;
     int32_t* leaf_part;  // n
@@ -139,6 +137,10 @@ struct TreeListArgs {
     int64_t far_cap, near_cap, seg_cap, slot_cap;
 };
 constexpr int kNeed = 6;
+// Where the scan leaves the number of leaves (device memory).
+__host__ __device__ inline const int32_t* leaf_count_of(const TreeListArgs& a) {
+    return reinterpret_cast<const int32_t*>(a.place + a.n);
+}
 size_t tree_list_temp_bytes(int32_t n, int32_t n_nodes);
 // Leaf compaction and the lists with their far-field work items (kernels read the number of leaves
 // on the device; sizes become known on the host, when it wants them, from the counters).
