@@ -1092,8 +1092,8 @@ __global__ void __launch_bounds__(256) item_gather_kernel(const TreeListArgs a, 
     if (k >= n) return;
     M2PItem it;
     it.leaf = -1;
-    if (cost[k] > 0) {  // real and valid
-        it = ((const M2PItem*)a.items)[idx[k]];
+    if (cost ? cost[k] > 0 : item_valid(a, ((const M2PItem*)a.items)[k])) {  // real and valid
+        it = ((const M2PItem*)a.items)[cost ? idx[k] : k];
         it.nchunks = abs(a.far_nch[it.leaf]);
         it.scratch = a.far_slot[it.leaf];
     }
@@ -1231,6 +1231,12 @@ cudaError_t launch_item_order(const TreeListArgs& a, int32_t n_items, const unsi
                               void* temp, size_t temp_bytes, M2PItem* out, cudaStream_t st) {
     if (n_items == 0) return cudaSuccess;
     const int g = (n_items + 255) / 256;
+    // Items that are all resident at once (M2P runs at least four blocks per SM) need no order: at
+    // N = 1000 the costs and the sort take two launches, 10 of 176 us of device time.
+    if (!n_real && n_items <= 148 * 4) {
+        item_gather_kernel<<<g, 256, 0, st>>>(a, nullptr, n_items, nullptr, out);
+        return cudaGetLastError();
+    }
     item_cost_kernel<<<g, 256, 0, st>>>(a, n_items, n_real, overflow, cost, idx);
     cub::DoubleBuffer<uint32_t> k(cost, cost_alt);
     cub::DoubleBuffer<int32_t> v(idx, idx_alt);
