@@ -529,6 +529,8 @@ int run_force(const ForceJob& j, const gx_physics& ph, int precision, Choice ch,
 struct HostStage {
     cudaStream_t st;
     std::deque<AsyncBuf> bufs;  // stable addresses; released in reverse order at scope exit
+    char* shared = nullptr;     // the rest of the last allocation that small arrays share (dev_array)
+    size_t shared_left = 0;
     explicit HostStage(cudaStream_t s) : st(s) {}
     // Device copy of a host array (nullptr stays nullptr).
     int in(const double* h, int64_t n, double** d) {
@@ -1669,9 +1671,24 @@ struct FmmPlan {
 
 template <typename T>
 int dev_array(HostStage& hs, int64_t count, T** p) {
-    hs.bufs.emplace_back();
-    GX_TRY(hs.bufs.back().alloc((size_t)std::max<int64_t>(count, 1) * sizeof(T), hs.st));
-    *p = (T*)hs.bufs.back().p;
+    // Small arrays share allocations (an evaluation has about fifty; N = 1000: 271 us per call
+    // against 290 with one allocation each).
+    constexpr size_t kShared = 2u << 20, kSmall = kShared / 4;
+    const size_t bytes = ((size_t)std::max<int64_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255;
+    const bool small = bytes <= kSmall;
+    if (!small || hs.shared_left < bytes) {
+        hs.bufs.emplace_back();
+        GX_TRY(hs.bufs.back().alloc(small ? kShared : bytes, hs.st));
+        if (!small) {
+            *p = (T*)hs.bufs.back().p;
+            return GX_OK;
+        }
+        hs.shared = (char*)hs.bufs.back().p;
+        hs.shared_left = kShared;
+    }
+    *p = (T*)hs.shared;
+    hs.shared += bytes;
+    hs.shared_left -= bytes;
     return GX_OK;
 }
 
