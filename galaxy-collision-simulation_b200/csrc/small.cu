@@ -23,8 +23,11 @@
 //     so each target is summed exactly as compute_direct_accelerations_for_targets sums it.  The skipped self pair
 //     and the s2 == 0 pair add +0.0, which leaves the running sum unchanged: it starts at
 //     +0.0 and, in round-to-nearest, a sum is -0.0 only when both addends are -0.0.
-// The grid barrier is an arrival counter and a generation word in global memory; a CTA
-// waits on the generation with ld.acquire for at most a.timeout_ns (and 2^30 polls), after
+// The step is a chain of latencies: barrier, sources from L2, pair terms, shuffles.  FP64, N = 1000:
+// 4.3 us per step (N = 250: 2.9, N = 4096: 32.8) against 6.0 (3.9, 34.6) with 512 sources per pass
+// fetched when needed and a barrier whose last arrival releases the others.
+// The grid barrier is an arrival counter in global memory; a CTA
+// waits on it with ld.acquire for at most a.timeout_ns (and 2^30 polls), after
 // which it sets the status word and the whole launch stops early: the state arrays are then
 // left as they were before the launch and the host reports GX_ERR_TIMEOUT.  The test hook
 // a.stall_step makes CTA 0 leave without arriving, so that the others' waits run out.
@@ -39,7 +42,8 @@ namespace {
 
 constexpr int kSmallThreads = 256;
 constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr int kSmallJT = 512;  // sources staged per shared-memory pass
+// Sources staged per shared-memory pass (the exact form also holds its contributions there).
+__host__ __device__ constexpr int small_pass(int prec) { return prec == kF64 ? 1024 : 512; }
 constexpr size_t kSmallHeader = 256;  // barrier words + status, then the position buffers
 std::atomic<int> g_small_tpw{0};      // 0: chosen from n; 1, 2 or 4: forced (measurement)
 std::atomic<int> g_small_wpt{0};      // 0: chosen; 1 or 2 warps per target: forced (measurement)
@@ -61,37 +65,30 @@ __device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
 }
 
 // Grid-wide barrier; false on every thread of the CTA when the launch has to stop.
-// `gen` (thread 0 only) is the generation this CTA waits to see pass.  One returning atomic
-// per CTA (the arrival); the last arrival resets the counter with a plain store and, after a
-// fence, releases the others with a non-returning release add on the generation word, so no
-// second returning round trip to L2 sits on the path.  A status set by a CTA that gave up is seen by the others at their
-// next wait (polled every 256 loads); the launch then ends within one barrier.
-__device__ bool grid_barrier(const SmallArgs& a, unsigned& gen) {
+// `goal` (thread 0 only) is the arrival count that ends this barrier: the counter only grows (the
+// host clears it before every launch), so a CTA arrives with one non-returning release add and
+// polls the counter itself -- no last arrival has to reset it and release the others, which
+// put a returning atomic and a second trip through L2 on the path.  A status set by a CTA that gave
+// up is seen by the others at their next wait (polled every 256 loads); the launch then ends
+// within one barrier.
+__device__ bool grid_barrier(const SmallArgs& a, unsigned& goal) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        __threadfence();  // after the CTA barrier: the CTA's position stores before its arrival
-        const unsigned arrived = atomicAdd(&a.bar[0], 1u);
-        if (arrived == gridDim.x - 1) {
-            *(volatile unsigned*)&a.bar[0] = 0u;  // nobody arrives again before the release below
-            __threadfence();  // every arrival seen through the counter, before the release
-            red_release_add_u32(&a.bar[1], 1u);
-        } else {
-            const unsigned long long t0 = global_ns();
-            unsigned polls = 0;
-            while (ld_acquire_u32(&a.bar[1]) == gen) {
-                if ((++polls & 255u) == 0) {
-                    if (polls >= (1u << 30) || global_ns() - t0 > a.timeout_ns ||
-                        *(volatile int*)a.status) {
-                        ok = 0;
-                        break;
-                    }
+        goal += gridDim.x;
+        red_release_add_u32(&a.bar[0], 1u);  // after the CTA barrier: the CTA's position stores before it
+        const unsigned long long t0 = global_ns();
+        unsigned polls = 0;
+        while ((int)(ld_acquire_u32(&a.bar[0]) - goal) < 0) {
+            if ((++polls & 255u) == 0) {
+                if (polls >= (1u << 30) || global_ns() - t0 > a.timeout_ns || *(volatile int*)a.status) {
+                    ok = 0;
+                    break;
                 }
             }
         }
         if (!ok) atomicExch(a.status, 1);
-        gen += 1;
         s_ok = ok;
     }
     __syncthreads();
@@ -104,6 +101,8 @@ __device__ bool grid_barrier(const SmallArgs& a, unsigned& gen) {
 template <int PREC, int TPW, bool EPS0, int WPT>
 __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(const SmallArgs a) {
     constexpr int kBlock = kSmallThreads * WPT;
+    constexpr int kSmallJT = small_pass(PREC);
+    constexpr int kPer = (kSmallJT + kBlock - 1) / kBlock;  // sources a thread stages per pass
     static_assert(PREC == kF64 || WPT == 1, "the exact form sums each target in one warp");
     __shared__ double s_part[WPT > 1 ? kSmallWarps * WPT * TPW * 3 : 1];
     __shared__ __align__(16) double sx[kSmallJT];
@@ -130,8 +129,7 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
         U[k] = a.vx[t]; V[k] = a.vy[t]; W[k] = a.vz[t];
         AX[k] = a.ax[t]; AY[k] = a.ay[t]; AZ[k] = a.az[t];
     }
-    unsigned gen = 0;
-    if (threadIdx.x == 0) gen = ld_acquire_u32(&a.bar[1]);
+    unsigned goal = 0;
 
     for (int64_t s = 0; s < a.steps; ++s) {
         double* px = a.buf + (size_t)((s & 1) * 3) * n;
@@ -154,20 +152,37 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
             }
         }
         if (s == a.stall_step && blockIdx.x == 0) return;
-        if (!grid_barrier(a, gen)) return;
+        if (!grid_barrier(a, goal)) return;
 
         double fx[TPW], fy[TPW], fz[TPW];
 #pragma unroll
         for (int k = 0; k < TPW; ++k) fx[k] = fy[k] = fz[k] = 0.0;
+        // a pass's sources are in flight while the pass before is computed
+        double4 src[kPer];
+        auto fetch = [&](int j0) {
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) {
+                const int j = j0 + threadIdx.x + u * kBlock;
+                if (j < min(n, j0 + kSmallJT))
+                    src[u] = make_double4(__ldcg(px + j), __ldcg(py + j), __ldcg(pz + j), __ldg(a.m + j));
+            }
+        };
+        fetch(0);
         for (int j0 = 0; j0 < n; j0 += kSmallJT) {
             const int cnt = min(kSmallJT, n - j0);
-            for (int jj = threadIdx.x; jj < cnt; jj += kBlock) {
-                sx[jj] = __ldcg(px + j0 + jj);
-                sy[jj] = __ldcg(py + j0 + jj);
-                sz[jj] = __ldcg(pz + j0 + jj);
-                sm[jj] = __ldg(a.m + j0 + jj);
+            if (j0 > 0) __syncthreads();
+#pragma unroll
+            for (int u = 0; u < kPer; ++u) {
+                const int jj = threadIdx.x + u * kBlock;
+                if (jj < cnt) {
+                    sx[jj] = src[u].x;
+                    sy[jj] = src[u].y;
+                    sz[jj] = src[u].z;
+                    sm[jj] = src[u].w;
+                }
             }
             __syncthreads();
+            if (j0 + kSmallJT < n) fetch(j0 + kSmallJT);
             if constexpr (PREC == kF64) {
 #pragma unroll 4
                 for (int jj = part * 32 + lane; jj < cnt; jj += 32 * WPT) {
@@ -223,7 +238,6 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
                     __syncwarp();
                 }
             }
-            __syncthreads();
         }
         // results and the closing kick (dt/2)
         if constexpr (PREC == kF64) {
@@ -328,8 +342,9 @@ cudaError_t small_steps_launch(const SmallArgs& a, int precision, bool eps0, int
     if (!coop) return cudaErrorNotSupported;
     // Shape: targets per warp (tpw) and, in the FP64 form, warps per target (wpt), the first
     // of (1, 2), (1, 1), (2, 2), (2, 1), (4, 2), (4, 1) whose grid is co-resident.  Measured on
-    // B200 (steps/s of the FP64 form): n = 1000: 155k at (1, 2), 128k at (1, 1), 111k at
-    // (2, 2), 90k at (2, 1); n = 4096: 26.4k at (2, 1) and (2, 2), 18.8k at (4, 1).  Forced
+    // B200 (steps/s of the FP64 form, before the sources were prefetched): n = 1000: 155k at (1, 2),
+    // 128k at (1, 1), 111k at (2, 2), 90k at (2, 1); n = 4096: 26.4k at (2, 1) and (2, 2), 18.8k at
+    // (4, 1).  Forced
     // shapes (measurement knobs) skip the others.
     const int f_tpw = g_small_tpw.load(), f_wpt = g_small_wpt.load();
     const void* fn = nullptr;

@@ -14,7 +14,7 @@ struct SmallArgs {
     double *x, *y, *z, *vx, *vy, *vz, *ax, *ay, *az;  // state: read at the start, written at the end
     const double* m;
     double* buf;       // two position buffers, buf[(p * 3 + c) * n + i]
-    unsigned* bar;     // grid barrier: [0] arrivals, [1] generation
+    unsigned* bar;     // grid barrier: arrivals since the launch began
     int* status;       // 0, or 1 when a barrier wait gave up (the launch then stops early)
     double G, eps2, dt;
     int64_t steps;
