@@ -18,9 +18,11 @@
 //     lanes of a warp split the sources (lane l takes j = l mod 32) and a butterfly of
 //     shuffles adds the 32 partial sums (every lane ends with the same bits);
 //   * kF64Exact -- the reference's operation order (direct_solver.cpp:8-23, 59-83): lane l
-//     computes the contribution of source j0 + l into shared memory, and lane c (c < 3)
-//     adds component c of the 32 contributions in ascending j order into one running sum,
-//     so each target is summed exactly as compute_direct_accelerations_for_targets sums it.  The skipped self pair
+//     computes the contribution of source j0 + l into shared memory (with exact_inv), and a lane
+//     per owned target and component adds the 32 contributions in ascending j order into one
+//     running sum while the next 32 are computed (N = 1000: 15.8 us per step, N = 4096: 85,
+//     against 18.7 and 171 with IEEE root and division and the sums one target after the
+//     other), so each target is summed exactly as compute_direct_accelerations_for_targets sums it.  The skipped self pair
 //     and the s2 == 0 pair add +0.0, which leaves the running sum unchanged: it starts at
 //     +0.0 and, in round-to-nearest, a sum is -0.0 only when both addends are -0.0.
 // The step is a chain of latencies: barrier, sources from L2, pair terms, shuffles.  FP64, N = 1000:
@@ -110,8 +112,10 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
     __shared__ __align__(16) double sz[kSmallJT];
     __shared__ __align__(16) double sm[kSmallJT];
     // exact form: each warp's 32 contributions (3 doubles each) per owned target
-    __shared__ double s_con_all[PREC == kF64Exact ? kSmallWarps * TPW * 96 : 1];
-    double* const s_con = s_con_all + (PREC == kF64Exact ? (threadIdx.x >> 5) * TPW * 96 : 0);
+    // (targets 100 doubles apart: their components lie in other banks)
+    constexpr int kConStride = 100;
+    __shared__ double s_con_all[PREC == kF64Exact ? kSmallWarps * TPW * kConStride : 1];
+    double* const s_con = s_con_all + (PREC == kF64Exact ? (threadIdx.x >> 5) * TPW * kConStride : 0);
     const int lane = threadIdx.x & 31;
     const int n = a.n;
     const int total_warps = gridDim.x * kSmallWarps;  // target slots of the grid
@@ -178,7 +182,7 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
                     sx[jj] = src[u].x;
                     sy[jj] = src[u].y;
                     sz[jj] = src[u].z;
-                    sm[jj] = src[u].w;
+                    sm[jj] = PREC == kF64Exact ? dmul(G, src[u].w) : src[u].w;
                 }
             }
             __syncthreads();
@@ -202,41 +206,63 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
                     }
                 }
             } else {
-                // lane l computes the contribution of source jb + l for each owned target into
-                // the warp's shared slots; then lane c (c < 3) adds component c of the 32
-                // contributions in ascending j, one running sum per target (fx holds it)
-                for (int jb = 0; jb < cnt; jb += 32) {
-                    const int jj = jb + lane;
-                    const int lim = min(32, cnt - jb);
+                // lane l computes the contribution of source jb + 32 + l to each owned target while
+                // lane 3 k + c adds component c of target k's contributions from sources jb ..
+                // jb + 31 in ascending order (the other lanes add along); then the new contributions
+                // take the old ones' place.  Past the last source they are +0.0.
+                double cx[TPW], cy[TPW], cz[TPW];
+                auto terms = [&](int jb) {
+                    const int jj = min(jb + lane, kSmallJT - 1);
+                    const double qx = sx[jj], qy = sy[jj], qz = sz[jj], qg = sm[jj];
+                    bool on[TPW];
+                    double s2[TPW], inv[TPW];
+                    ExactGuard guard;
 #pragma unroll
                     for (int k = 0; k < TPW; ++k) {
-                        double cx = 0.0, cy = 0.0, cz = 0.0;
-                        if (T[k] < n && jj < cnt && j0 + jj != T[k]) {
-                            const double rx = dsub(sx[jj], X[k]), ry = dsub(sy[jj], Y[k]), rz = dsub(sz[jj], Z[k]);
-                            const double s2 = dadd(dadd(dadd(dmul(rx, rx), dmul(ry, ry)), dmul(rz, rz)), e2);
-                            if (s2 != 0.0) {
-                                const double inv = __ddiv_rn(1.0, __dsqrt_rn(s2));
-                                const double inv3 = dmul(dmul(inv, inv), inv);
-                                const double scale = dmul(dmul(G, sm[jj]), inv3);
-                                cx = dmul(rx, scale);
-                                cy = dmul(ry, scale);
-                                cz = dmul(rz, scale);
-                            }
-                        }
-                        double* slot = s_con + (k * 32 + lane) * 3;
-                        slot[0] = cx;
-                        slot[1] = cy;
-                        slot[2] = cz;
+                        on[k] = jb + lane < cnt && j0 + jj != T[k];
+                        cx[k] = dsub(qx, X[k]);
+                        cy[k] = dsub(qy, Y[k]);
+                        cz[k] = dsub(qz, Z[k]);
+                        s2[k] = dadd(dadd(dadd(dmul(cx[k], cx[k]), dmul(cy[k], cy[k])), dmul(cz[k], cz[k])), e2);
+                        if (!on[k]) s2[k] = 1.0;
+                        inv[k] = exact_inv(s2[k], guard);
                     }
-                    __syncwarp();
-                    if (lane < 3) {
-                        for (int q = 0; q < lim; ++q) {
+                    if (!guard.clean()) {
 #pragma unroll
-                            for (int k = 0; k < TPW; ++k) fx[k] = dadd(fx[k], s_con[(k * 32 + q) * 3 + lane]);
+                        for (int k = 0; k < TPW; ++k) {
+                            inv[k] = ieee_inv(s2[k]);
+                            if (s2[k] == 0.0) on[k] = false;
                         }
                     }
+#pragma unroll
+                    for (int k = 0; k < TPW; ++k) {
+                        const double scale = dmul(qg, dmul(dmul(inv[k], inv[k]), inv[k]));
+                        cx[k] = on[k] ? dmul(cx[k], scale) : 0.0;
+                        cy[k] = on[k] ? dmul(cy[k], scale) : 0.0;
+                        cz[k] = on[k] ? dmul(cz[k], scale) : 0.0;
+                    }
+                };
+                auto store = [&] {
+#pragma unroll
+                    for (int k = 0; k < TPW; ++k) {
+                        double* const slot = s_con + k * kConStride + lane * 3;
+                        slot[0] = cx[k];
+                        slot[1] = cy[k];
+                        slot[2] = cz[k];
+                    }
                     __syncwarp();
+                };
+                const double* const mine = s_con + (lane / 3) % TPW * kConStride + lane % 3;
+                terms(0);
+                store();
+                for (int jb = 0; jb < cnt; jb += 32) {
+                    if (jb + 32 < cnt) terms(jb + 32);
+#pragma unroll
+                    for (int q = 0; q < 32; ++q) fx[0] = dadd(fx[0], mine[q * 3]);
+                    __syncwarp();
+                    if (jb + 32 < cnt) store();
                 }
+                __syncwarp();
             }
         }
         // results and the closing kick (dt/2)
@@ -284,10 +310,10 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
             }
         } else {
 #pragma unroll
-            for (int k = 0; k < TPW; ++k) {  // lane c holds component c
-                AX[k] = __shfl_sync(0xffffffffu, fx[k], 0);
-                AY[k] = __shfl_sync(0xffffffffu, fx[k], 1);
-                AZ[k] = __shfl_sync(0xffffffffu, fx[k], 2);
+            for (int k = 0; k < TPW; ++k) {  // lane 3 k + c holds component c of target k
+                AX[k] = __shfl_sync(0xffffffffu, fx[0], 3 * k);
+                AY[k] = __shfl_sync(0xffffffffu, fx[0], 3 * k + 1);
+                AZ[k] = __shfl_sync(0xffffffffu, fx[0], 3 * k + 2);
             }
         }
 #pragma unroll
@@ -361,6 +387,10 @@ cudaError_t small_steps_launch(const SmallArgs& a, int precision, bool eps0, int
             int occ = 0;
             if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, g, kSmallThreads * wpt, 0)) != cudaSuccess)
                 return e;
+            // The exact form first looks for a shape with one CTA per SM: its warps' chains of additions
+            // slow down by half when two share an SM (us per step, one / two targets per warp: N = 1400
+            // 31.5 / 23.0, N = 2368 51.6 / 36.8; two / four: N = 3000 73.0 / 64.0).
+            if (precision == kF64Exact && !f_tpw && tpw < 4 && b > sms) continue;
             if ((int64_t)occ * sms < b) continue;
             fn = g;
             blocks = b;
