@@ -10,8 +10,9 @@
 //   1. root cell from the bounding box (:62-85);
 //   2. every body's path as a 63-bit key, 3 bits per level, level 0 in the top bits;
 //   3. a stable radix sort of (key, body): depth-first tree order;
-//   4. one CTA walks the levels: a node with more than leaf_capacity bodies splits into 8
-//      children whose body ranges are found by binary search on the sorted keys;
+//   4. the octants that a sorted body has in common with its neighbour and with the body
+//      leaf_capacity places on tell at which levels it starts a node that splits; counts per
+//      level and block of bodies number the nodes, and eight lanes per node find its children;
 //   5. one warp per leaf sorts the leaf's bodies into ascending index order, the order
 //      the reference's sums run in.
 // Nodes are numbered breadth-first.  Trees that need a split below level 21 (more than

@@ -8,9 +8,9 @@
 // (near-list order, then leaf order).  Leaf costs are very uneven (in the N = 65,536
 // two-disk tree the heaviest leaf has 13x the mean number of sources), so a leaf is cut into
 // target groups x source chunks (at most kMaxChunks chunks of at least kMinChunk sources),
-// items of bounded cost.  A plan computed on the device (p2p_count_kernel, then one block's
-// counting sort of the leaves by item cost and its scans, or a CUB sort and scans for large
-// leaf tables) numbers the items, the leaves with the costliest items first;
+// items of bounded cost.  A plan computed on the device (one block that splits the leaves, sorts them
+// by item cost and scans, or a count kernel with a CUB sort and scans for large leaf tables)
+// numbers the items, the leaves with the costliest items first;
 // a persistent grid takes them from a ticket counter, so that the last items handed out are
 // the cheapest and the blocks finish together.  Items of an
 // unsplit leaf add their sums to the accelerations directly (target groups are disjoint).
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(BS, p2p_threads_per_sm(MODE, TPT) / BS) p2p_ke
         const int item = s_item;
         __syncthreads();
         if (item >= n_items) return;
-        // leaf owning the item: one load from the table p2p_item_leaf_kernel filled; items past
+        // leaf owning the item: one load from the plan's table; items past
         // the table (possible only with device CSR arrays that repeat bodies) search the offsets
         int leaf;
         if (item < a.plan_item_cap) {
