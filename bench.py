@@ -363,7 +363,7 @@ def run_single(gx, torch, p, args, eps, dt, prec) -> dict:
     if clk.get("sm_mhz"):
         roof["frac_at_observed_clock"] = achieved / (sms * FP32_LANES_PER_SM * clk["sm_mhz"] * 1e6 / 1e12)
     if prec == gx.PRECISION_F64:
-        roof["note"] = "FP64 form: 17 FP64 pipe ops per interaction; frac is against the FP32 pipe"
+        roof["note"] = "FP64 form: 16 FP64 pipe ops per interaction; frac is against the FP32 pipe"
     out["roofline"] = roof
     out["clocks"] = clk
     out["config"] = {"workload": f"direct-mixed-n{n}" if prec == gx.PRECISION_MIXED else f"direct-f64-n{n}",
@@ -885,10 +885,10 @@ FP64_LANES_PER_SM = 64
 # (m2p_one<4> in csrc/fmm.cu: offsets, softened r^-1 with one refinement step, g1..g5,
 # the quadrupole, octupole and hexadecapole contractions and the accumulation; 171.3
 # measured as DADD + DMUL + DFMA thread instructions per pair), and of one FP64 near-field
-# interaction (offsets, r^2 + eps^2, r^-3 with one refinement step, m r^-3, three
+# interaction (offsets, r^2 + eps^2, m r^-3 from the rsqrt seed with one correction, three
 # accumulations), the count of the direct FP64 kernel.
 FP64_OPS_PER_M2P_PAIR = 171
-FP64_OPS_PER_P2P_PAIR = 17
+FP64_OPS_PER_P2P_PAIR = 16
 
 
 def wl_fmm_session(gx, torch, args) -> dict:
