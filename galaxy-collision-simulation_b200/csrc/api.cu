@@ -2373,10 +2373,12 @@ int fmm_work_enqueue(FmmWork& w, const double* x, const double* y, const double*
     GX_CUDA(launch_tree_massive(la, w.list_temp, w.list_bytes, st));
     GX_CUDA(launch_tree_lists(la, w.list_temp, w.list_bytes, sm_count(dev), st));
     GX_CUDA(launch_pool_check(la, t.hdr, st));
-    GX_CUDA(launch_item_order(la, (int32_t)w.far_cap, &la.counters->chunks, w.flags, w.cost, w.cost_alt, w.idx, w.idx_alt,
-                              w.order_temp, w.order_bytes, w.sorted, st));
     GX_CUDA(cudaEventRecord(w.fork, st));
     GX_CUDA(cudaStreamWaitEvent(w.aux, w.fork, 0));
+    // only the far field needs its items in order (N = 65,536 leaf 64: the near field starts 20 us
+    // earlier, a step takes 662 us against 698)
+    GX_CUDA(launch_item_order(la, (int32_t)w.far_cap, &la.counters->chunks, w.flags, w.cost, w.cost_alt, w.idx, w.idx_alt,
+                              w.order_temp, w.order_bytes, w.sorted, w.aux));
     for (double* p : {ax, ay, az}) GX_CUDA(cudaMemsetAsync(p, 0, (size_t)n * sizeof(double), w.aux));
     fa.ax = ax;
     fa.ay = ay;
