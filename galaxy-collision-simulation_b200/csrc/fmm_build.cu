@@ -491,6 +491,7 @@ __global__ void __launch_bounds__(256) leaf_mark_kernel(const TreeListArgs a) {
 // copying its bodies, two scans and a pass of its own for the records.
 __global__ void __launch_bounds__(256) leaf_emit_kernel(const TreeListArgs a) {
     const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k == 0) a.counters->leaves = leaf_count(a);
     if (k < a.n && a.mark[k] != 0) a.leaf_part[(int)(a.place[k] >> 32)] = a.perm[k];
     if (k >= list_nodes(a)) return;
     const int b = a.beg[k], e = a.end[k];

@@ -65,7 +65,8 @@ struct ListCounters {
     unsigned long long slots;                  // partial sums of leaves with several chunks
     unsigned long long far_pairs, near_pairs;  // (body, far node) and (body, body) pairs
     unsigned long long segs;                   // segments of long near lists reserved
-    int ticket, n_long, n_slow, pad;
+    int ticket, n_long, n_slow;
+    int leaves;                                // leaves with mass > 0
 };
 constexpr int kNearSeg = 512;  // entries of a segment of a long near list
 constexpr int kWalkStackSlots = 1024;  // entries a walk's stack may hold
