@@ -326,7 +326,7 @@ int least_split(int64_t n_src, int jt, Cost cost) {
 // N = 65,536: 16 chunks 1720 us, 9 chunks 1840; N = 32,768: 32 chunks 454, 8 chunks 505).
 constexpr int64_t kMaxPartBytes = 256ll << 20;
 int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
-    if (v.precision == kF64Exact) return 1;
+    if (v.precision == kF64Exact || n_tgt <= 0) return 1;  // a range without targets is legal
     if (v.precision == kMixed && v.block * v.ipt > 256)
         return least_split(n_src, v.jt, [&](int ns) {
             return rounds_cost(v.block, v.ipt, v.jt, force_occupancy(v), n_tgt, n_src, ns, sms);
