@@ -922,7 +922,8 @@ int session_choice(gx_session* s, int precision, Choice* out) {
 int session_ensure_part(gx_session* s, const Choice& ch) {
     int cnt;
     const ForceVariant* all = force_variants(&cnt);
-    const size_t need = part_bytes(all[ch.variant], s->n, s->n, ch.nsplit);
+    // by the session's own targets: a rank's chunks are many, its partial sums few
+    const size_t need = part_bytes(all[ch.variant], s->n, s->t_count, ch.nsplit);
     if (need <= s->part_cap) return GX_OK;
     if (s->part) {
         cudaStreamSynchronize(s->stream);
