@@ -927,6 +927,7 @@ int session_ensure_part(gx_session* s, const Choice& ch) {
     if (need <= s->part_cap) return GX_OK;
     if (s->part) {
         cudaStreamSynchronize(s->stream);
+        s->clear_graphs();  // recorded steps (of another precision or split) write to the old scratch
         cudaFree(s->part);
         s->part = nullptr;
         s->part_cap = 0;

@@ -40,3 +40,30 @@ def test_scratch_follows_the_targets(prec):
         assert e.max() <= 1e-11
     else:
         assert np.median(e) <= 1e-6 and e.max() <= 1e-4
+
+
+@pytest.mark.parametrize("n", [20000, 40001])
+def test_recorded_steps_follow_the_scratch(n):
+    """Steps recorded before the scratch grew (FP64 takes more chunks than mixed) run with the new one:
+    the same bits as in a session whose scratch was large from the start, and nothing is written to
+    memory that somebody else holds by then."""
+    p = gx.ics.two_disk_encounter(n - n // 2, n // 2, 29, 0.05)
+    out = []
+    for large_first in (True, False):
+        with gx.Session(n, gx.PhysicsParams(1.0, 0.05)) as s:
+            if large_first:
+                s.set_particles(p)
+                s.compute_accelerations(F64)
+            s.set_particles(p)
+            s.compute_accelerations(MIX)
+            s.step(2, 0.002, MIX)
+            s.compute_accelerations(F64)
+            s.synchronize()
+            torch.cuda.empty_cache()
+            held = [torch.full((k << 18,), 7.0, dtype=torch.float64, device="cuda") for k in (1, 2, 4, 8)]
+            torch.cuda.synchronize()
+            s.step(2, 0.002, MIX)
+            out.append(s.get_state())
+            assert all(bool((t == 7.0).all()) for t in held)
+    for f in out[0]:
+        assert np.array_equal(out[0][f], out[1][f]), f
