@@ -180,6 +180,7 @@ _SIGNATURES = {
     "gx_variant_count": [c_int, POINTER(c_int)],
     "gx_variant_describe": [c_int, c_int, c_char_p, c_int],
     "gx_debug_fail_allocations": [c_int],
+    "gx_debug_alloc_limit": [I64],
     "gx_debug_stall_barrier": [I64],
     "gx_debug_p2p_targets_per_thread": [c_int],
     "gx_debug_small_targets_per_warp": [c_int],

@@ -42,6 +42,7 @@ using namespace gx;
 namespace {
 thread_local std::string g_err;
 std::atomic<int> g_fail_allocs{0};
+std::atomic<int64_t> g_alloc_limit{0};  // test hook: larger allocations fail (0: none)
 std::atomic<int64_t> g_stall_step{-1};  // gx_debug_stall_barrier
 std::atomic<int> g_fmm_tight_pools{0};  // gx_debug_fmm_tight_pools: no headroom (tests of the regrowth)
 
@@ -83,11 +84,18 @@ int fail_cuda(cudaError_t e, const char* what) {
         return fail(GX_ERR_CUDA, "unexpected C++ exception inside the gx library");  \
     }
 
-cudaError_t dev_alloc(void** p, size_t bytes) {
+// An allocation that a test wants to fail.
+bool alloc_refused(size_t bytes) {
     int left = g_fail_allocs.load();
     while (left > 0) {
-        if (g_fail_allocs.compare_exchange_weak(left, left - 1)) return cudaErrorMemoryAllocation;
+        if (g_fail_allocs.compare_exchange_weak(left, left - 1)) return true;
     }
+    const int64_t limit = g_alloc_limit.load();
+    return limit > 0 && bytes > (size_t)limit;
+}
+
+cudaError_t dev_alloc(void** p, size_t bytes) {
+    if (alloc_refused(bytes)) return cudaErrorMemoryAllocation;
     return cudaMalloc(p, bytes ? bytes : 16);
 }
 
@@ -96,10 +104,7 @@ cudaMemPool_t library_pool(int dev);
 // Stream-ordered scratch from the library's own memory pool (library_pool), never from the
 // device's default pool that the host application may be using.
 cudaError_t dev_alloc_async(void** p, size_t bytes, cudaStream_t st) {
-    int left = g_fail_allocs.load();
-    while (left > 0) {
-        if (g_fail_allocs.compare_exchange_weak(left, left - 1)) return cudaErrorMemoryAllocation;
-    }
+    if (alloc_refused(bytes)) return cudaErrorMemoryAllocation;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -532,6 +537,18 @@ struct HostStage {
     char* shared = nullptr;     // the rest of the last allocation that small arrays share (dev_array)
     size_t shared_left = 0;
     explicit HostStage(cudaStream_t s) : st(s) {}
+    // What has been allocated so far, and the release (stream-ordered) of all that came after.
+    struct Mark {
+        size_t bufs;
+        char* shared;
+        size_t left;
+    };
+    Mark mark() const { return {bufs.size(), shared, shared_left}; }
+    void release_to(const Mark& m) {
+        while (bufs.size() > m.bufs) bufs.pop_back();
+        shared = m.shared;
+        shared_left = m.left;
+    }
     // Device copy of a host array (nullptr stays nullptr).
     int in(const double* h, int64_t n, double** d) {
         if (!h) {
@@ -588,6 +605,11 @@ extern "C" int gx_device_available(int* available) {
 
 extern "C" int gx_debug_fail_allocations(int count) {
     g_fail_allocs.store(count < 0 ? 0 : count);
+    return GX_OK;
+}
+
+extern "C" int gx_debug_alloc_limit(int64_t bytes) {
+    g_alloc_limit.store(bytes < 0 ? 0 : bytes);
     return GX_OK;
 }
 
@@ -1916,28 +1938,43 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     void* list_temp;
     GX_TRY(dev_array(hs, (int64_t)list_bytes, (char**)&list_temp));
     // Pools for the lists: a guess from the number of leaves and theta (a leaf of a two-disk system
-    // has 300 to 600 far nodes and 80 to 150 near leaves at theta 0.6, growing as theta falls); when
-    // it is too small, the totals tell what is needed and the lists are made again.
+    // has 300 to 600 far nodes and 80 to 150 near leaves at theta 0.6, growing as theta falls), at
+    // most kListPoolBytes each; when it is too small, the totals tell what is needed and the lists
+    // are made again.  So are they when the guess does not fit in memory: pools of one entry then
+    // count what the lists really need.
+    constexpr int64_t kListPoolBytes = 2ll << 30;
     const double wide = std::min(8.0, std::max(1.0, 0.36 / (la.theta * la.theta)));
-    const int64_t leaf_bound = P.n_nodes - P.n_nodes / 8 + 1;
-    la.far_cap = (int64_t)(2.0 * wide * (double)leaf_bound) + 64;
+    const int64_t leaf_bound = std::min<int64_t>(P.n_nodes - P.n_nodes / 8 + 1, n);  // leaves with bodies
+    la.far_cap = std::min<int64_t>((int64_t)(2.0 * wide * (double)leaf_bound) + 64,
+                                   kListPoolBytes / (int64_t)(kM2PChunk * sizeof(int32_t)));
     la.near_cap = std::min<int64_t>((int64_t)(256.0 * wide * (double)leaf_bound) + 4096,
-                                    std::numeric_limits<int32_t>::max());
-    la.seg_cap = (int64_t)(wide * (double)leaf_bound / 16.0) + 256;
+                                    kListPoolBytes / (int64_t)sizeof(int32_t));
+    la.seg_cap = std::min<int64_t>((int64_t)(wide * (double)leaf_bound / 16.0) + 256,
+                                   kListPoolBytes / (int64_t)(kNearSeg * sizeof(int32_t)));
     la.slot_cap = std::numeric_limits<int64_t>::max();
     if (g_fmm_tight_pools.load()) la.far_cap = la.near_cap = la.seg_cap = 1;
     la.walk_stack = fmm_walk_stack();
     M2PItem* items;
     int32_t nl = 0;
     ListCounters tot;
-    for (int attempt = 0;; ++attempt) {
+    const HostStage::Mark before = hs.mark();
+    auto pools = [&]() -> int {
+        hs.release_to(before);
         GX_TRY(dev_array(hs, la.far_cap * kM2PChunk, &la.far_node));
         GX_TRY(dev_array(hs, la.far_cap, &items));
         la.items = items;
         GX_TRY(dev_array(hs, la.near_cap, &la.near_leaf));
         GX_TRY(dev_array(hs, la.seg_cap * kNearSeg, &la.seg_near));
         GX_TRY(dev_array(hs, la.seg_cap, &la.seg_next));
-        GX_TRY(dev_array(hs, la.seg_cap, &la.seg_count));
+        return dev_array(hs, la.seg_cap, &la.seg_count);
+    };
+    for (int attempt = 0;; ++attempt) {
+        int made = pools();
+        if (made == GX_ERR_OUT_OF_MEMORY && attempt == 0) {
+            la.far_cap = la.near_cap = la.seg_cap = 1;
+            made = pools();
+        }
+        GX_TRY(made);
         GX_CUDA(launch_tree_lists(la, list_temp, list_bytes, sm_count(dev), st));
         Totals all;
         GX_CUDA(cudaMemcpyAsync(&all, counters, offsetof(Totals, m2m_err) + sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -434,6 +434,9 @@ int gx_variant_describe(int precision, int variant, char* buf, int buflen);
  * participant that leaves a bounded wait) ----------------------------------------------- */
 /* The next `count` device allocations made by the library fail with GX_ERR_OUT_OF_MEMORY. */
 int gx_debug_fail_allocations(int count);
+/* Device allocations of more than `bytes` bytes made by the library fail with
+ * GX_ERR_OUT_OF_MEMORY until the limit is lifted with 0. */
+int gx_debug_alloc_limit(int64_t bytes);
 /* The next single-launch session step loop (gx_session_step on a small system) loses one
  * participant: its first CTA leaves before the barrier of step `step` instead of arriving,
  * and the barrier waits are cut to 0.2 s, so the other CTAs give up, the launch ends early
