@@ -1690,7 +1690,6 @@ struct FmmPlan {
     const int32_t* near_end = nullptr;
     const int32_t* near_leaf = nullptr;
     const int32_t* near_src = nullptr;
-    int64_t near_len = 0;  // length of near_leaf
 };
 
 template <typename T>
@@ -1769,7 +1768,6 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
     GX_TRY(dev_copy(hs, T.far_node, &fa.far_node));
     GX_TRY(dev_copy(hs, T.near_off, &P.near_beg));
     P.near_end = P.near_beg + 1;
-    P.near_len = P.n_near;
     GX_TRY(dev_copy(hs, T.near_leaf, &P.near_leaf));
     GX_TRY(mark(tm, 1, hs.st));
     GX_TRY(dev_array(hs, (int64_t)P.n_nodes * kFmmRec, &fa.rec));
@@ -2032,7 +2030,6 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     P.near_end = la.near_end;
     P.near_leaf = la.near_leaf;
     P.near_src = la.near_src;
-    P.near_len = la.near_cap;
     return GX_OK;
 }
 
@@ -2702,7 +2699,7 @@ extern "C" int gxi_leaf_lists_from_device(int64_t n, const double* x, const doub
     const int32_t nl = P->n_leaves;
     T->leaf_off.resize((size_t)nl + 1);
     T->near_off.assign((size_t)nl + 1, 0);
-    std::vector<int32_t> beg((size_t)nl), end((size_t)nl), near((size_t)P->near_len);
+    std::vector<int32_t> beg((size_t)nl), end((size_t)nl);
     auto fetch = [&](std::vector<int32_t>& v, const int32_t* d) -> int {
         if (!v.empty()) GX_CUDA(cudaMemcpyAsync(v.data(), d, v.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         return GX_OK;
@@ -2710,18 +2707,23 @@ extern "C" int gxi_leaf_lists_from_device(int64_t n, const double* x, const doub
     GX_TRY(fetch(T->leaf_off, P->fa.leaf_off));
     GX_TRY(fetch(beg, P->near_beg));
     GX_TRY(fetch(end, P->near_end));
-    GX_TRY(fetch(near, P->near_leaf));
     GX_CUDA(cudaStreamSynchronize(st));
     T->leaf_part.resize((size_t)T->leaf_off[nl]);
     GX_TRY(fetch(T->leaf_part, P->fa.leaf_part));
-    T->near_leaf.clear();
-    T->near_leaf.reserve((size_t)P->n_near);
-    for (int32_t l = 0; l < nl; ++l) {  // the device's lists lie in any order
-        T->near_leaf.insert(T->near_leaf.end(), near.begin() + beg[(size_t)l], near.begin() + end[(size_t)l]);
-        T->near_off[(size_t)l + 1] = (int32_t)T->near_leaf.size();
-    }
+    // the device's lists lie in any order: gathered leaf by leaf there, and only they are copied
+    for (size_t l = 0; l < (size_t)nl; ++l) T->near_off[l + 1] = T->near_off[l] + (end[l] - beg[l]);
+    T->near_leaf.resize((size_t)T->near_off[nl]);
+    int32_t *off, *near;
+    GX_TRY(hs.in_any(T->near_off.data(), (int64_t)nl + 1, &off));
+    GX_TRY(dev_array(hs, (int64_t)T->near_leaf.size(), &near));
+    GX_CUDA(launch_near_gather(nl, P->near_beg, P->near_leaf, off, near, st));
+    GX_TRY(fetch(T->near_leaf, near));
     GX_CUDA(cudaStreamSynchronize(st));
     T->n_far = P->n_far;
+    if (P->on_device) {
+        T->n_pairs = P->near_pairs;
+        return GX_OK;
+    }
     T->n_pairs = 0;
     for (int32_t l = 0; l < nl; ++l)
         for (int32_t k = T->near_off[l]; k < T->near_off[l + 1]; ++k)

@@ -146,6 +146,10 @@ size_t tree_list_temp_bytes(int32_t n, int32_t n_nodes);
 // Leaf compaction and the lists with their far-field work items (kernels read the number of leaves
 // on the device; sizes become known on the host, when it wants them, from the counters).
 cudaError_t launch_tree_lists(const TreeListArgs& a, void* temp, size_t temp_bytes, int sms, cudaStream_t st);
+// The near lists one after the other in leaf order: leaf l's, from near_beg[l] of near_leaf on, to
+// out[off[l] .. off[l + 1]).
+cudaError_t launch_near_gather(int32_t n_leaves, const int32_t* near_beg, const int32_t* near_leaf, const int32_t* off,
+                               int32_t* out, cudaStream_t st);
 // mprefix from the masses (a.m, a.perm); a mass < 0 or NaN marks an overflow with bit 1 of
 // the sticky word (the caller then evaluates through the host-read path).  temp: scan scratch
 // for n + 1 ints.
