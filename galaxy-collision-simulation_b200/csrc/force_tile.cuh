@@ -523,8 +523,7 @@ __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, c
                 double r = fma(dx, dx, e2);
                 r = fma(dy, dy, r);
                 r = fma(dz, dz, r);
-                double w = inv_cube_f64(r, qm);
-                if (EPS0) w = (r == 0.0) ? 0.0 : w;
+                const double w = EPS0 ? inv_cube_unsoftened(r, qm) : inv_cube_f64(r, qm);
                 fx[k] = fma(dx, w, fx[k]);
                 fy[k] = fma(dy, w, fy[k]);
                 fz[k] = fma(dz, w, fz[k]);

@@ -28,7 +28,7 @@ __device__ __forceinline__ double rsqrt_f64(double s) {
 // s^(-3/2) = y t (1 - e)^(-3/2) = y t (1 + 3e/2 + 15e^2/8 + O(e^3)), so the correction is
 // applied to the product m y t itself: 7 FP64 pipe operations after the seed, where refining
 // y first (5) and cubing it (3) took 8, and three roundings of the result instead of six.
-// The truncated term is about (35/16) e^3 < 2^-55.  s == 0 as in rsqrt_f64.
+// The truncated term is about (35/16) e^3 < 2^-55.  s > 0.
 __device__ __forceinline__ double inv_cube_f64(double s, double m) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
@@ -37,6 +37,18 @@ __device__ __forceinline__ double inv_cube_f64(double s, double m) {
     const double p = fma(1.875, e, 1.5);
     const double w = (m * y) * t;
     return fma(w * e, p, w);
+}
+
+// The same without softening.  Coincident bodies and massless ones weigh nothing; below s = 1e-200
+// (softened sums are always above), where the cube of 1 / sqrt(s) may overflow and the correction
+// would turn an infinite weight into NaN, the cube is taken first, as the reference takes it.
+__device__ __forceinline__ double inv_cube_unsoftened(double s, double m) {
+    if (s < 1e-200) {
+        if (s == 0.0 || m == 0.0) return 0.0;
+        const double y = rsqrt_f64(s);
+        return m * (y * y * y);
+    }
+    return inv_cube_f64(s, m);
 }
 
 // RN(1 / RN(sqrt(s))), the value IEEE square root and division give, without their branches.

@@ -583,8 +583,8 @@ __global__ void __launch_bounds__(BS, p2p_threads_per_sm(MODE, TPT) / BS) p2p_ke
                             for (int h = 0; h < TPT; ++h) {
                                 const double dx = xy.x - xt[h], dy = xy.y - yt[h], dz = zm.x - zt[h];
                                 const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, a.eps2)));
-                                double w = inv_cube_f64(r2, zm.y);
-                                if (EPS0) w = (r2 == 0.0 || I[r] == ti[h]) ? 0.0 : w;
+                                double w = EPS0 ? inv_cube_unsoftened(r2, zm.y) : inv_cube_f64(r2, zm.y);
+                                if (EPS0) w = I[r] == ti[h] ? 0.0 : w;
                                 f[3 * h] = fma(dx, w, f[3 * h]);
                                 f[3 * h + 1] = fma(dy, w, f[3 * h + 1]);
                                 f[3 * h + 2] = fma(dz, w, f[3 * h + 2]);

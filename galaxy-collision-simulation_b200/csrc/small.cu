@@ -198,8 +198,7 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
                         double r = fma(dx, dx, e2);
                         r = fma(dy, dy, r);
                         r = fma(dz, dz, r);
-                        double wgt = inv_cube_f64(r, qm);
-                        if (EPS0) wgt = (r == 0.0) ? 0.0 : wgt;
+                        const double wgt = EPS0 ? inv_cube_unsoftened(r, qm) : inv_cube_f64(r, qm);
                         fx[k] = fma(dx, wgt, fx[k]);
                         fy[k] = fma(dy, wgt, fy[k]);
                         fz[k] = fma(dz, wgt, fz[k]);
