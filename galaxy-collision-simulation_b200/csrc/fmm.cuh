@@ -34,6 +34,12 @@ struct M2PItem {
     int64_t scratch;  // first partial-sum slot of the leaf (targets), when nchunks > 1
 };
 
+// Pairs of an item, from 1 (an item of cost 0 counts as none) to what 31 bits hold.
+__host__ __device__ inline uint32_t far_item_cost(int32_t targets, int32_t nodes) {
+    const int64_t c = (int64_t)targets * nodes + 1;
+    return c < 0x7fffffff ? (uint32_t)c : 0x7fffffffu;
+}
+
 struct FmmArgs {
     const double* x;
     const double* y;

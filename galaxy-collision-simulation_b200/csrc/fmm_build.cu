@@ -1057,8 +1057,7 @@ __global__ void __launch_bounds__(256) item_cost_kernel(const TreeListArgs a, in
     if (k < real) {
         const M2PItem it = ((const M2PItem*)a.items)[k];
         if (item_valid(a, it)) {
-            const uint32_t v = min((uint32_t)(a.leaf_off[it.leaf + 1] - a.leaf_off[it.leaf]) * (uint32_t)it.count + 1u,
-                                   0x7fffffffu);
+            const uint32_t v = far_item_cost(a.leaf_off[it.leaf + 1] - a.leaf_off[it.leaf], it.count);
             const int msb = 31 - __clz(v);
             c = v < 4u ? v : (uint32_t)(msb * 4 + ((v >> (msb - 2)) & 3));
         }
