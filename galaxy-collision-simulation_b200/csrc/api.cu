@@ -1772,7 +1772,9 @@ int fmm_plan_host(FmmPlan& P, int64_t n, const double* hx, const double* hy, con
     GX_TRY(mark(tm, 1, hs.st));
     GX_TRY(dev_array(hs, (int64_t)P.n_nodes * kFmmRec, &fa.rec));
     GX_TRY(dev_array(hs, (int64_t)fmm_octets(P.n_nodes), &fa.octet_parent));
-    GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), T.n_levels(), hs.st));
+    int dev = 0;
+    GX_CUDA(cudaGetDevice(&dev));
+    GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), T.n_levels(), sm_count(dev), hs.st));
     GX_TRY(mark(tm, 2, hs.st));
     // far-field work items for the leaves that hold a target in [begin, end)
     std::vector<M2PItem> items;
@@ -1825,6 +1827,8 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     GX_TRY(mark(tm, 0, st));
     *deep = false;
     P.on_device = true;
+    int dev = 0;
+    GX_CUDA(cudaGetDevice(&dev));
     const int64_t cap = std::max<int64_t>(1, opt.leaf_capacity);
     TreeBuildArgs t{};
     t.n = (int32_t)n;
@@ -1862,7 +1866,7 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
         GX_TRY(dev_array(hs, capacity, &t.cy));
         GX_TRY(dev_array(hs, capacity, &t.cz));
         GX_TRY(dev_array(hs, capacity, &t.hw));
-        GX_CUDA(launch_tree_build(t, sort_temp, sort_bytes, st));
+        GX_CUDA(launch_tree_build(t, sort_temp, sort_bytes, sm_count(dev), st));
         GX_CUDA(cudaMemcpyAsync(hdr, t.hdr, sizeof(hdr), cudaMemcpyDeviceToHost, st));
         GX_CUDA(cudaStreamSynchronize(st));
         if (hdr[2] & 1) {
@@ -1899,8 +1903,6 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
                      (char**)&counters));
     int* const m2m = (int*)(counters + 1);
     GX_CUDA(cudaMemsetAsync(m2m, 0, 2 * sizeof(int), st));
-    int dev = 0;
-    GX_CUDA(cudaGetDevice(&dev));
     GX_CUDA(launch_fmm_moments_tree(fa, m2m + 2, m2m + 3, m2m, sm_count(dev), st));
     GX_TRY(mark(tm, 2, st));
 
@@ -1982,7 +1984,7 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
         if (all.m2m_err != 0 && attempt < 3) {
             // a bounded wait of the one-launch upward pass gave up: the passes again, level by level
             GX_CUDA(cudaMemsetAsync(m2m, 0, sizeof(int), st));
-            GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), hdr[1], st));
+            GX_CUDA(launch_fmm_moments(fa, P.level_off.data(), hdr[1], sm_count(dev), st));
             continue;
         }
         if (tot.far > (unsigned long long)std::numeric_limits<int32_t>::max() ||
@@ -2019,7 +2021,7 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     void* order_temp;
     GX_TRY(dev_array(hs, (int64_t)order_bytes, (char**)&order_temp));
     GX_CUDA(launch_item_order(la, fa.n_items, nullptr, nullptr, cost, cost_alt, idx, idx_alt, order_temp, order_bytes,
-                              sorted_items, st));
+                              sorted_items, sm_count(dev), st));
     items = sorted_items;
     GX_TRY(mark(tm, 3, st));
     fa.leaf_off = la.leaf_off;
@@ -2395,7 +2397,7 @@ int fmm_work_enqueue(FmmWork& w, const double* x, const double* y, const double*
     t.y = y;
     t.z = z;
     GX_CUDA(cudaMemsetAsync(w.flags, 0, sizeof(int), st));
-    GX_CUDA(launch_tree_build(t, w.tree_temp, w.tree_bytes, st));
+    GX_CUDA(launch_tree_build(t, w.tree_temp, w.tree_bytes, sm_count(dev), st));
     GX_CUDA(launch_tree_leaf_order(t, w.node_cap, w.tree_temp, w.tree_bytes, st));
     FmmArgs& fa = w.fa;
     fa.x = x;
@@ -2421,7 +2423,7 @@ int fmm_work_enqueue(FmmWork& w, const double* x, const double* y, const double*
     // only the far field needs its items in order (N = 65,536 leaf 64: the near field starts 20 us
     // earlier, a step takes 662 us against 698)
     GX_CUDA(launch_item_order(la, (int32_t)w.far_cap, &la.counters->chunks, w.flags, w.cost, w.cost_alt, w.idx, w.idx_alt,
-                              w.order_temp, w.order_bytes, w.sorted, w.aux));
+                              w.order_temp, w.order_bytes, w.sorted, sm_count(dev), w.aux));
     for (double* p : {ax, ay, az}) GX_CUDA(cudaMemsetAsync(p, 0, (size_t)n * sizeof(double), w.aux));
     fa.ax = ax;
     fa.ay = ay;

@@ -704,7 +704,8 @@ cudaError_t launch_fmm_add_near(int64_t n, double* ax, double* ay, double* az, c
     return cudaGetLastError();
 }
 
-cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, int n_levels, cudaStream_t st) {
+cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, int n_levels, int sms,
+                               cudaStream_t st) {
     constexpr int wpb = kMomBlock / 32;
     if (a.n_nodes == 0) return cudaSuccess;
     fmm_leaf_kernel<<<(a.n_nodes + wpb - 1) / wpb, kMomBlock, 0, st>>>(a);
@@ -713,7 +714,7 @@ cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, 
     for (int d = n_levels - 2; d >= 0; --d) {  // octets whose children are level d + 1
         const int ob = (level_off_host[d + 1] - 1) >> 3, oe = (level_off_host[d + 2] - 1) >> 3;
         if (oe <= ob) continue;
-        fmm_m2m_kernel<<<std::min(oe - ob, 148 * 8), kM2MBlock, 0, st>>>(a, ob, oe);
+        fmm_m2m_kernel<<<std::min(oe - ob, sms * 8), kM2MBlock, 0, st>>>(a, ob, oe);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

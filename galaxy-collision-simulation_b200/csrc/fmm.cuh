@@ -103,7 +103,8 @@ int fmm_effective_order(int expansion_order);
 constexpr int kM2PChunk = 512;  // far nodes per work item
 
 // Stream-ordered: leaf moments, then one launch per level (deepest first).
-cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, int n_levels, cudaStream_t st);
+cudaError_t launch_fmm_moments(const FmmArgs& a, const int32_t* level_off_host, int n_levels, int sms,
+                               cudaStream_t st);
 // The same with every internal node in one launch (blocks wait on their children's flags):
 // ticket (1 int) and ready (fmm_octets(n_nodes) ints) are scratch; a wait that times out sets
 // bit 0 of err[0] and err[1].

@@ -30,6 +30,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <atomic>
 #include <cfloat>
 
 namespace gx {
@@ -1147,7 +1148,7 @@ size_t tree_build_temp_bytes(int32_t n, int64_t cap) {
            aligned((size_t)split_capacity(n, cap) * sizeof(int2)) + aligned(b);
 }
 
-cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_bytes, cudaStream_t st) {
+cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_bytes, int sms, cudaStream_t st) {
     Topology p;
     p.blocks = topo_blocks(t.n);
     p.split_cap = split_capacity(t.n, t.cap);
@@ -1162,7 +1163,7 @@ cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_by
     const int gn = (t.n + kBboxThreads - 1) / kBboxThreads;
     const int bbox_blocks = std::min(gn, kBboxBlocks);
     bbox_partial_kernel<<<bbox_blocks, kBboxThreads, 0, st>>>(t);
-    keys_kernel<<<std::min(gn, 148 * 8), kBboxThreads, 0, st>>>(t, bbox_blocks, p.ticket);
+    keys_kernel<<<std::min(gn, sms * 8), kBboxThreads, 0, st>>>(t, bbox_blocks, p.ticket);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     cub::DoubleBuffer<uint64_t> k(t.keys, t.keys_alt);
@@ -1174,7 +1175,7 @@ cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_by
     if (v.Current() != t.perm) gather_perm_kernel<<<(t.n + 255) / 256, 256, 0, st>>>(v.Current(), t.perm, t.n);
     split_count_kernel<<<p.blocks, kTopoThreads, 0, st>>>(t, k.Current(), p);
     split_emit_kernel<<<p.blocks, kTopoThreads, 0, st>>>(t, k.Current(), p);
-    tree_children_kernel<<<148 * 8, 256, 0, st>>>(t, k.Current(), p);
+    tree_children_kernel<<<sms * 8, 256, 0, st>>>(t, k.Current(), p);
     return cudaGetLastError();
 }
 
@@ -1193,11 +1194,18 @@ size_t tree_list_temp_bytes(int32_t n, int32_t n_nodes) {
     return std::max(b, scan_bytes(n + 1));
 }
 
-// The walk prefers a 70% shared-memory carveout (8 blocks of 19 KiB; the rest is L1).
+// The walk prefers a 70% shared-memory carveout (8 blocks of 19 KiB; the rest is L1): a setting of
+// the current device's copy of the kernel.
 static cudaError_t walk_carveout() {
-    static cudaError_t once =
-        cudaFuncSetAttribute(walk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 70);
-    return once;
+    static std::atomic<unsigned long long> set_on{0};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (set_on.load() & bit) return cudaSuccess;
+    e = cudaFuncSetAttribute(walk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 70);
+    if (e == cudaSuccess) set_on.fetch_or(bit);
+    return e;
 }
 
 cudaError_t launch_tree_lists(const TreeListArgs& a, void* temp, size_t temp_bytes, int sms, cudaStream_t st) {
@@ -1248,12 +1256,12 @@ size_t item_order_temp_bytes(int32_t n_items) {
 
 cudaError_t launch_item_order(const TreeListArgs& a, int32_t n_items, const unsigned long long* n_real,
                               const int* overflow, uint32_t* cost, uint32_t* cost_alt, int32_t* idx, int32_t* idx_alt,
-                              void* temp, size_t temp_bytes, M2PItem* out, cudaStream_t st) {
+                              void* temp, size_t temp_bytes, M2PItem* out, int sms, cudaStream_t st) {
     if (n_items == 0) return cudaSuccess;
     const int g = (n_items + 255) / 256;
     // Items that are all resident at once (M2P runs at least four blocks per SM) need no order: at
     // N = 1000 the costs and the sort take two launches, 10 of 176 us of device time.
-    if (!n_real && n_items <= 148 * 4) {
+    if (!n_real && n_items <= sms * 4) {
         item_gather_kernel<<<g, 256, 0, st>>>(a, nullptr, n_items, nullptr, out);
         return cudaGetLastError();
     }

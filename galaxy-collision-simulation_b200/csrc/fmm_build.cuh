@@ -43,7 +43,7 @@ struct TreeBuildArgs {
     int key_levels;
 };
 size_t tree_build_temp_bytes(int32_t n, int64_t cap);
-cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_bytes, cudaStream_t st);
+cudaError_t launch_tree_build(const TreeBuildArgs& t, void* temp, size_t temp_bytes, int sms, cudaStream_t st);
 // After a successful build: bodies of every leaf in ascending index order in t.perm
 // (uses t.idx as scratch).
 cudaError_t launch_tree_leaf_order(const TreeBuildArgs& t, int32_t n_nodes, void* temp, size_t temp_bytes,
@@ -164,6 +164,6 @@ size_t item_order_temp_bytes(int32_t n_items);
 // n_items is the length of the arrays; n_real (nullable: all) the items on the device.
 cudaError_t launch_item_order(const TreeListArgs& a, int32_t n_items, const unsigned long long* n_real,
                               const int* overflow, uint32_t* cost, uint32_t* cost_alt, int32_t* idx, int32_t* idx_alt,
-                              void* temp, size_t temp_bytes, M2PItem* out, cudaStream_t st);
+                              void* temp, size_t temp_bytes, M2PItem* out, int sms, cudaStream_t st);
 
 }  // namespace gx
