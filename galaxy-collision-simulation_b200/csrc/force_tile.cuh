@@ -523,7 +523,8 @@ __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, c
                 double r = fma(dx, dx, e2);
                 r = fma(dy, dy, r);
                 r = fma(dz, dz, r);
-                const double w = EPS0 ? inv_cube_unsoftened(r, qm) : inv_cube_f64(r, qm);
+                double w = inv_cube_f64(r, qm);
+                if (EPS0) w = (r == 0.0) ? 0.0 : w;
                 fx[k] = fma(dx, w, fx[k]);
                 fy[k] = fma(dy, w, fy[k]);
                 fz[k] = fma(dz, w, fz[k]);
@@ -544,6 +545,16 @@ __device__ __forceinline__ void f64_tile(const ForceArgs& a, const int64_t t0, c
     for (int k = 0; k < IPT; ++k) {
         const int64_t t = t0 + k * BLOCK + tid;
         if (t >= a.n_tgt) continue;
+        if (EPS0 && sum_overflowed(fx[k], fy[k], fz[k])) {
+            fx[k] = fy[k] = fz[k] = 0.0;
+            for (int64_t j = jb; j < je; ++j) {
+                const double dx = a.x[j] - xi[k], dy = a.y[j] - yi[k], dz = a.z[j] - zi[k];
+                const double w = inv_cube_first(fma(dz, dz, fma(dy, dy, fma(dx, dx, e2))), a.m[j]);
+                fx[k] = fma(dx, w, fx[k]);
+                fy[k] = fma(dy, w, fy[k]);
+                fz[k] = fma(dz, w, fz[k]);
+            }
+        }
         if (a.nsplit == 1)
             write_result(a, t, body[k], a.G * fx[k], a.G * fy[k], a.G * fz[k]);
         else

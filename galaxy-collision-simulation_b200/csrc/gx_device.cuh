@@ -39,16 +39,19 @@ __device__ __forceinline__ double inv_cube_f64(double s, double m) {
     return fma(w * e, p, w);
 }
 
-// The same without softening.  Coincident bodies and massless ones weigh nothing; below s = 1e-200
-// (softened sums are always above), where the cube of 1 / sqrt(s) may overflow and the correction
-// would turn an infinite weight into NaN, the cube is taken first, as the reference takes it.
-__device__ __forceinline__ double inv_cube_unsoftened(double s, double m) {
-    if (s < 1e-200) {
-        if (s == 0.0 || m == 0.0) return 0.0;
-        const double y = rsqrt_f64(s);
-        return m * (y * y * y);
-    }
-    return inv_cube_f64(s, m);
+// Sums without softening.  Where s^(-3/2) overflows (s below 3.1e-206; softened sums are always
+// above) the reference's weight is infinite, but inv_cube_f64's correction can turn it into NaN.
+// Testing every pair costs a fifth of the sum (N = 131,072: 21.7 ms with integer tests, 19.8 with a
+// branch, against 18.2), so a target's share of the sum is looked at when it is complete: a term of
+// such a pair is some 1e205 times the mass, beyond any sum of ordinary ones, and the share is then
+// added up once more with the cube taken first, as the reference takes it.
+__device__ __forceinline__ bool sum_overflowed(double fx, double fy, double fz) {
+    return !(fabs(fx) < 1e180 && fabs(fy) < 1e180 && fabs(fz) < 1e180);  // NaN included
+}
+__device__ __forceinline__ double inv_cube_first(double s, double m) {
+    if (s == 0.0 || m == 0.0) return 0.0;
+    const double y = rsqrt_f64(s);
+    return m * (y * y * y);
 }
 
 // RN(1 / RN(sqrt(s))), the value IEEE square root and division give, without their branches.

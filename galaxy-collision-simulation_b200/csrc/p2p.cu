@@ -306,6 +306,32 @@ constexpr int p2p_threads_per_sm(int mode, int tpt) { return tpt == 2 ? 640 : mo
 
 // BS threads per block (a multiple of 32), 4 x BS sources staged per pass, TPT targets per
 // thread in the fast forms (2 or 4).
+// The sum of body i over the source slots [c_lo, c_hi) of n_near near leaves with the cube taken first
+// (see sum_overflowed); a call of its own, since code inside the kernel costs its registers (13 % of
+// the near field).
+__device__ __noinline__ double3 sum_again(const int32_t* near, int n_near, const int32_t* leaf_off,
+                                          const int32_t* leaf_part, const double* x, const double* y, const double* z,
+                                          const double* m, double eps2, int64_t c_lo, int64_t c_hi, int i) {
+    double3 f = make_double3(0.0, 0.0, 0.0);
+    const double xi = x[i], yi = y[i], zi = z[i];
+    int64_t base = 0;
+    for (int q = 0; q < n_near && base < c_hi; ++q) {
+        const int b = leaf_off[near[q]], len = leaf_off[near[q] + 1] - b;
+        const int lo = (int)max((int64_t)0, c_lo - base), hi = (int)min((int64_t)len, c_hi - base);
+        for (int k = lo; k < hi; ++k) {
+            const int j = leaf_part[b + k];
+            if (j == i) continue;
+            const double dx = x[j] - xi, dy = y[j] - yi, dz = z[j] - zi;
+            const double w = inv_cube_first(fma(dz, dz, fma(dy, dy, fma(dx, dx, eps2))), m[j]);
+            f.x = fma(dx, w, f.x);
+            f.y = fma(dy, w, f.y);
+            f.z = fma(dz, w, f.z);
+        }
+        base += len;
+    }
+    return f;
+}
+
 template <int MODE, bool EPS0, int BS, int TPT>
 __global__ void __launch_bounds__(BS, p2p_threads_per_sm(MODE, TPT) / BS) p2p_kernel(const P2PArgs a) {
     constexpr int kP2PBlock = BS;
@@ -583,8 +609,8 @@ __global__ void __launch_bounds__(BS, p2p_threads_per_sm(MODE, TPT) / BS) p2p_ke
                             for (int h = 0; h < TPT; ++h) {
                                 const double dx = xy.x - xt[h], dy = xy.y - yt[h], dz = zm.x - zt[h];
                                 const double r2 = fma(dz, dz, fma(dy, dy, fma(dx, dx, a.eps2)));
-                                double w = EPS0 ? inv_cube_unsoftened(r2, zm.y) : inv_cube_f64(r2, zm.y);
-                                if (EPS0) w = I[r] == ti[h] ? 0.0 : w;
+                                double w = inv_cube_f64(r2, zm.y);
+                                if (EPS0) w = (r2 == 0.0 || I[r] == ti[h]) ? 0.0 : w;
                                 f[3 * h] = fma(dx, w, f[3 * h]);
                                 f[3 * h + 1] = fma(dy, w, f[3 * h + 1]);
                                 f[3 * h + 2] = fma(dz, w, f[3 * h + 2]);
@@ -681,6 +707,13 @@ __global__ void __launch_bounds__(BS, p2p_threads_per_sm(MODE, TPT) / BS) p2p_ke
                         const int t = t0 + row + h * H;
                         const int i = ti[h];
                         if (i < a.t_begin || i >= a.t_end) continue;
+                        if (MODE == kF64 && EPS0 && sum_overflowed(S[3 * h], S[3 * h + 1], S[3 * h + 2])) {
+                            const double3 F = sum_again(a.near_leaf + nb, ne - nb, a.leaf_off, a.leaf_part, a.x, a.y, a.z,
+                                                        a.m, a.eps2, c_lo, c_hi, i);
+                            S[3 * h] = F.x;
+                            S[3 * h + 1] = F.y;
+                            S[3 * h + 2] = F.z;
+                        }
                         if (chunks == 1) {
                             a.ax[i] = a.ax[i] + a.G * S[3 * h];
                             a.ay[i] = a.ay[i] + a.G * S[3 * h + 1];

@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
                         double r = fma(dx, dx, e2);
                         r = fma(dy, dy, r);
                         r = fma(dz, dz, r);
-                        const double wgt = EPS0 ? inv_cube_unsoftened(r, qm) : inv_cube_f64(r, qm);
+                        double wgt = inv_cube_f64(r, qm);
+                        if (EPS0) wgt = (r == 0.0) ? 0.0 : wgt;
                         fx[k] = fma(dx, wgt, fx[k]);
                         fy[k] = fma(dy, wgt, fy[k]);
                         fz[k] = fma(dz, wgt, fz[k]);
@@ -268,6 +269,16 @@ __global__ void __launch_bounds__(kSmallThreads * WPT, 1) small_steps_kernel(con
         if constexpr (PREC == kF64) {
 #pragma unroll
             for (int k = 0; k < TPW; ++k) {
+                if (EPS0 && T[k] < n && sum_overflowed(fx[k], fy[k], fz[k])) {  // this lane's sources again
+                    fx[k] = fy[k] = fz[k] = 0.0;
+                    for (int j = part * 32 + lane; j < n; j += 32 * WPT) {
+                        const double dx = __ldcg(px + j) - X[k], dy = __ldcg(py + j) - Y[k], dz = __ldcg(pz + j) - Z[k];
+                        const double wgt = inv_cube_first(fma(dz, dz, fma(dy, dy, fma(dx, dx, e2))), a.m[j]);
+                        fx[k] = fma(dx, wgt, fx[k]);
+                        fy[k] = fma(dy, wgt, fy[k]);
+                        fz[k] = fma(dz, wgt, fz[k]);
+                    }
+                }
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) {
                     fx[k] += __shfl_xor_sync(0xffffffffu, fx[k], o);
