@@ -322,11 +322,16 @@ int least_split(int64_t n_src, int jt, Cost cost) {
 
 // The j-split of a variant.  FP64, and mixed blocks of two warps: short chunks, so that many small
 // CTAs per SM hide one another's staging and latencies and even out the SMs; smaller still where
-// that leaves the SMs without work, never more than 64 chunks or kMaxPartBytes of partial sums.
+// that leaves the SMs without work, at most kMaxPartBytes of partial sums and 64 chunks -- in FP64
+// sqrt(n_src) / 2 chunks when the tiles are so few that 64 leave SMs empty (a rank's or a list's targets
+// against many sources: the last block adds the chunks one after the other, so their number and
+// their length balance at the square root).
 // Measured on B200 (us, sources per chunk): FP64 256 x 2 N = 16,384 512: 285, 1024: 327, one wave of
 // 2 CTAs per SM: 369; N = 49,999 1024: 2478, 2048: 2570, 16,896: 2673; N = 100,000 2048: 9680,
 // 6144: 9888; FP64 256 x 1 N = 8192 256: 84, 512: 94; mixed 64 x 4 N = 5000 256: 31, 512: 33;
-// N = 16,384 256: 145, 512: 135, 1280: 139; N = 23,000 512: 257, 1024: 249, 2560: 264.
+// N = 16,384 256: 145, 512: 135, 1280: 139; N = 23,000 512: 257, 1024: 249, 2560: 264.  FP64, 100 targets
+// against 65,536 sources, 256 x 1: 128 chunks 48 us, 64 72 (64 x 2, 64 chunks: 107); 1400 against 2^20: 512
+// chunks 1665 us, 128 1938, 49 1953; 3000 against 2^20: 256 3248, 128 3443, 64 3843.
 // Mixed blocks of four warps and more follow rounds_cost: whole rounds count most there (256 x 4,
 // N = 65,536: 16 chunks 1720 us, 9 chunks 1840; N = 32,768: 32 chunks 454, 8 chunks 505).
 constexpr int64_t kMaxPartBytes = 256ll << 20;
@@ -340,7 +345,14 @@ int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
                                           : (v.block == 64 ? 128 : v.block * v.ipt == 256 ? 256 : 512);
     const int64_t tiles = (n_tgt + (int64_t)v.block * v.ipt - 1) / ((int64_t)v.block * v.ipt);
     while (chunk > v.jt && tiles * ((n_src + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
-    const int64_t most = std::max<int64_t>(1, std::min<int64_t>(64, kMaxPartBytes / (24 * n_tgt)));
+    int64_t most = 64;
+    // 2048 blocks of 256 threads fill the SMs several times over
+    const int64_t wide = std::min<int64_t>((int64_t)(0.5 * std::sqrt((double)n_src)), 2048 * 256 / (tiles * v.block));
+    if (v.precision == kF64 && wide > most) {
+        chunk = std::max<int64_t>(chunk, (n_src / wide + v.jt / 2) / v.jt * v.jt);  // in whole passes
+        most = (n_src + chunk - 1) / chunk;
+    }
+    most = std::max<int64_t>(1, std::min(most, kMaxPartBytes / (24 * n_tgt)));
     return (int)std::max<int64_t>(1, std::min(most, (n_src + chunk - 1) / chunk));
 }
 
@@ -382,9 +394,11 @@ double variant_rate_penalty(const ForceVariant& v) {
 
 // The FP64 variant for n_tgt targets: 256 x 2 from 15,000 up (N = 65,536 4.18 ms; 256 x 1 4.21,
 // 64 x 2 4.26), 256 x 1 below (N = 8192 84 us, 256 x 2 93, 64 x 2 91; N = 3000 25, 36 and 27), 64 x 2
-// for the smallest (N = 500 20 us, 256 x 1 23); softening 0 has 256 x 2 and 64 x 2 only.
-bool f64_shape(const ForceVariant& v, int64_t n_tgt, bool eps0) {
-    const int block = n_tgt >= (eps0 ? 6000 : 1500) ? 256 : 64;
+// for the smallest systems (N = 500 20 us, 256 x 1 23) -- not for few targets of large ones, whose
+// blocks are too few to hide its short passes (100 of 16,384: 40 us, 256 x 1 27); softening 0 has 256 x 2
+// and 64 x 2 only.
+bool f64_shape(const ForceVariant& v, int64_t n_tgt, int64_t n_src, bool eps0) {
+    const int block = n_tgt >= (eps0 ? 6000 : 1500) || (!eps0 && n_src > 8192) ? 256 : 64;
     const int ipt = block == 64 || eps0 || n_tgt >= 15000 ? 2 : 1;
     return v.block == block && v.ipt == ipt;
 }
@@ -422,7 +436,7 @@ Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_
     for (int k = 0; k < c; ++k) {
         const ForceVariant& v = all[ids[k]];
         if (precision == kMixed && (!v.packed || v.twin_of >= 0)) continue;  // scalar: for measurement only
-        if (precision == kF64 && !f64_shape(v, n_tgt, eps0)) continue;
+        if (precision == kF64 && !f64_shape(v, n_tgt, n_src, eps0)) continue;
         const double cost = precision == kMixed ? mixed_variant_cost(v, n_tgt, n_src, sms) * variant_rate_penalty(v) : 0.0;
         if (cost < bc) {
             bc = cost;

@@ -1,0 +1,55 @@
+"""Default shapes and source splits where one rule of n alone chose badly (B200).
+
+The chosen configuration is read back (threads at work, block shape) and the sums are checked against
+the oracle: FP64 1e-11 relative, mixed median 1e-6 and 1e-4 at most.
+"""
+import re
+
+import numpy as np
+import pytest
+
+import gx
+import oracle
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+F64, MIX = gx.PRECISION_F64, gx.PRECISION_MIXED
+
+
+def chosen(s, prec):
+    """(block, targets per thread, chunks) of the session's configuration."""
+    v, js = s.get_config(prec)
+    block, ipt = re.search(r"block=(\d+) ipt=(\d+)", gx.describe_variant(prec, v)).groups()
+    return int(block), int(ipt), js
+
+
+def check(p, s, prec, eps, begin, count):
+    s.set_targets(begin, count)
+    s.compute_accelerations(prec)
+    st = s.get_state()
+    idx = np.unique(np.linspace(begin, begin + count - 1, 41).astype(np.int64))
+    e = rel_err(np.stack([st[f][idx] for f in ("ax", "ay", "az")], 1),
+                oracle.direct_indexed(p.x, p.y, p.z, p.m, 1.0, eps, idx))
+    if prec == F64:
+        assert e.max() <= 1e-11
+    elif eps > 0.0:
+        assert np.median(e) <= 1e-6 and e.max() <= 1e-4
+    else:  # close pairs amplify FP32 offset rounding without softening: the bulk only
+        assert np.median(e) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [8192, 8193, 16384, 70001, 262144])
+@pytest.mark.parametrize("eps", [0.02, 0.0])
+def test_few_targets_of_a_large_system_occupy_the_chip(n, eps):
+    """At least half as many threads as sources, or one block of 256 on each of 128 SMs."""
+    p = gx.ics.two_disk_encounter(n - n // 2, n // 2, n, 0.02)
+    with gx.Session(n, gx.PhysicsParams(1.0, eps)) as s:
+        s.set_particles(p)
+        for count in (1, 100, 1499, 3000):
+            check(p, s, F64, eps, n // 3, count)
+            block, ipt, js = chosen(s, F64)
+            tiles = -(-count // (block * ipt))
+            assert tiles * js * block >= min(n // 2, 128 * 256) or eps == 0.0
+            if n > 65536:
+                assert js > 64
