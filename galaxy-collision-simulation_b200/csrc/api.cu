@@ -329,9 +329,11 @@ int least_split(int64_t n_src, int jt, Cost cost) {
 // Measured on B200 (us, sources per chunk): FP64 256 x 2 N = 16,384 512: 285, 1024: 327, one wave of
 // 2 CTAs per SM: 369; N = 49,999 1024: 2478, 2048: 2570, 16,896: 2673; N = 100,000 2048: 9680,
 // 6144: 9888; FP64 256 x 1 N = 8192 256: 84, 512: 94; mixed 64 x 4 N = 5000 256: 31, 512: 33;
-// N = 16,384 256: 145, 512: 135, 1280: 139; N = 23,000 512: 257, 1024: 249, 2560: 264.  FP64, 100 targets
-// against 65,536 sources, 256 x 1: 128 chunks 48 us, 64 72 (64 x 2, 64 chunks: 107); 1400 against 2^20: 512
-// chunks 1665 us, 128 1938, 49 1953; 3000 against 2^20: 256 3248, 128 3443, 64 3843.
+// N = 16,384 256: 145, 512: 135, 1280: 139; N = 23,000 512: 257, 1024: 249, 2560: 264.  FP64 64 x 2
+// without softening N = 3000 128: 27, 256: 33; N = 5000 128: 52, 256: 48; N = 11,000 256: 162, 512: 171;
+// N = 18,000 256: 384, 512: 384.  FP64 256 x 1, 100 targets against 65,536 sources: 128 chunks 48, 64
+// chunks 72 (64 x 2, 64 chunks 107); 1400 against 2^20: 512 chunks 1665, 128 1938, 49 1953; 3000
+// against 2^20: 256 chunks 3248, 128 3443, 64 3843.
 // Mixed blocks of four warps and more follow rounds_cost: whole rounds count most there (256 x 4,
 // N = 65,536: 16 chunks 1720 us, 9 chunks 1840; N = 32,768: 32 chunks 454, 8 chunks 505).
 constexpr int64_t kMaxPartBytes = 256ll << 20;
@@ -342,7 +344,8 @@ int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
             return rounds_cost(v.block, v.ipt, v.jt, force_occupancy(v), n_tgt, n_src, ns, sms);
         });
     int64_t chunk = v.precision == kMixed ? (n_src <= 7000 ? 256 : n_src < 18000 ? 512 : 1024)
-                                          : (v.block == 64 ? 128 : v.block * v.ipt == 256 ? 256 : 512);
+                                          : v.block == 64 ? (n_src <= 4500 ? 128 : n_src <= 16384 ? 256 : 512)
+                                                          : (v.block * v.ipt == 256 ? 256 : 512);
     const int64_t tiles = (n_tgt + (int64_t)v.block * v.ipt - 1) / ((int64_t)v.block * v.ipt);
     while (chunk > v.jt && tiles * ((n_src + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
     int64_t most = 64;
@@ -395,10 +398,11 @@ double variant_rate_penalty(const ForceVariant& v) {
 // The FP64 variant for n_tgt targets: 256 x 2 from 15,000 up (N = 65,536 4.18 ms; 256 x 1 4.21,
 // 64 x 2 4.26), 256 x 1 below (N = 8192 84 us, 256 x 2 93, 64 x 2 91; N = 3000 25, 36 and 27), 64 x 2
 // for the smallest systems (N = 500 20 us, 256 x 1 23) -- not for few targets of large ones, whose
-// blocks are too few to hide its short passes (100 of 16,384: 40 us, 256 x 1 27); softening 0 has 256 x 2
-// and 64 x 2 only.
+// blocks are too few to hide its short passes (100 of 16,384: 40 us, 256 x 1 27).  Softening 0 has 256 x 2
+// and 64 x 2 only: the latter up to 20,000 targets (N = 9000 118 against 148 us, 11,000 162 / 197, 20,000
+// 466 / 476; 25,000 708 / 705).
 bool f64_shape(const ForceVariant& v, int64_t n_tgt, int64_t n_src, bool eps0) {
-    const int block = n_tgt >= (eps0 ? 6000 : 1500) || (!eps0 && n_src > 8192) ? 256 : 64;
+    const int block = n_tgt >= (eps0 ? 20000 : 1500) || (!eps0 && n_src > 8192) ? 256 : 64;
     const int ipt = block == 64 || eps0 || n_tgt >= 15000 ? 2 : 1;
     return v.block == block && v.ipt == ipt;
 }

@@ -53,3 +53,15 @@ def test_few_targets_of_a_large_system_occupy_the_chip(n, eps):
             assert tiles * js * block >= min(n // 2, 128 * 256) or eps == 0.0
             if n > 65536:
                 assert js > 64
+
+
+@pytest.mark.parametrize("n", [4500, 4501, 6000, 9000, 14000, 16384, 16385, 19999, 20000])
+def test_fp64_without_softening(n):
+    """64-thread blocks below 20,000 bodies, in chunks that leave each SM two blocks at least."""
+    p = gx.ics.two_disk_encounter(n - n // 2, n // 2, n, 0.02)
+    with gx.Session(n, gx.PhysicsParams(1.0, 0.0)) as s:
+        s.set_particles(p)
+        check(p, s, F64, 0.0, 0, n)
+        block, ipt, js = chosen(s, F64)
+        assert block == (64 if n < 20000 else 256)
+        assert -(-n // (block * ipt)) * js >= 2 * 148
