@@ -320,22 +320,24 @@ int least_split(int64_t n_src, int jt, Cost cost) {
     return best;
 }
 
-// The j-split of a variant.  FP64, and mixed blocks of two warps: short chunks, so that many small
-// CTAs per SM hide one another's staging and latencies and even out the SMs; smaller still where
-// that leaves the SMs without work, at most kMaxPartBytes of partial sums and 64 chunks -- in FP64
-// sqrt(n_src) / 2 chunks when the tiles are so few that 64 leave SMs empty (a rank's or a list's targets
-// against many sources: the last block adds the chunks one after the other, so their number and
-// their length balance at the square root).
-// Measured on B200 (us, sources per chunk): FP64 256 x 2 N = 16,384 512: 285, 1024: 327, one wave of
-// 2 CTAs per SM: 369; N = 49,999 1024: 2478, 2048: 2570, 16,896: 2673; N = 100,000 2048: 9680,
-// 6144: 9888; FP64 256 x 1 N = 8192 256: 84, 512: 94; mixed 64 x 4 N = 5000 256: 31, 512: 33;
-// N = 16,384 256: 145, 512: 135, 1280: 139; N = 23,000 512: 257, 1024: 249, 2560: 264.  FP64 64 x 2
-// without softening N = 3000 128: 27, 256: 33; N = 5000 128: 52, 256: 48; N = 11,000 256: 162, 512: 171;
-// N = 18,000 256: 384, 512: 384.  FP64 256 x 1, 100 targets against 65,536 sources: 128 chunks 48, 64
-// chunks 72 (64 x 2, 64 chunks 107); 1400 against 2^20: 512 chunks 1665, 128 1938, 49 1953; 3000
-// against 2^20: 256 chunks 3248, 128 3443, 64 3843.
-// Mixed blocks of four warps and more follow rounds_cost: whole rounds count most there (256 x 4,
-// N = 65,536: 16 chunks 1720 us, 9 chunks 1840; N = 32,768: 32 chunks 454, 8 chunks 505).
+// The j-split of a variant; at most kMaxPartBytes of partial sums where the rule is a chunk length.
+// Measured on B200 (us, sources per chunk):
+// FP64: short chunks, so that many CTAs per SM hide one another's staging and latencies and even out the
+// SMs; smaller still where that leaves the SMs without work.  256 x 2 N = 16,384 512: 285, 1024: 327, one
+// wave of 2 CTAs per SM: 369; N = 49,999 1024: 2478, 2048: 2570, 16,896: 2673; N = 100,000 2048:
+// 9680, 6144: 9888; 256 x 1 N = 8192 256: 84, 512: 94; 64 x 2 without softening N = 3000 128: 27, 256:
+// 33; N = 5000 128: 52, 256: 48; N = 11,000 256: 162, 512: 171; N = 18,000 256: 384, 512: 384.  At most 64
+// chunks, or sqrt(n_src) / 2 when the tiles are so few that 64 leave SMs empty (a rank's or a list's
+// targets against many sources: the last block adds the chunks one after the other, so their
+// number and their length balance at the square root).  256 x 1, 100 targets against 65,536 sources: 128
+// chunks 48, 64 chunks 72 (64 x 2, 64 chunks 107); 1400 against 2^20: 512 chunks 1665, 128 1938, 49
+// 1953; 3000 against 2^20: 256 chunks 3248, 128 3443, 64 3843.
+// Mixed: whole rounds count most.  Blocks of 256 threads and more by their cost: 256 x 4 and larger by
+// rounds_cost (N = 65,536: 16 chunks 1720 us, 9 chunks 1840; N = 32,768: 32 chunks 454, 8 chunks 505), 256
+// x 1 by rounds of four blocks (N = 9000 12 chunks 52, 18 58; N = 7001 10 chunks 39, 28 44; over 46 sizes
+// up to 12,000 0.2 % from the best split, 2.6 % at most).  64 x 4, whose few warps also want short
+// chunks, takes them of 512 sources (256 below 7200) unless rounds of six blocks find another 6 %
+// better (softening 0: N = 12,800 107 against 117, N = 7411 52 / 62; 1.2 % from the best split, 10 % at most).
 constexpr int64_t kMaxPartBytes = 256ll << 20;
 int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
     if (v.precision == kF64Exact || n_tgt <= 0) return 1;  // a range without targets is legal
@@ -343,10 +345,22 @@ int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
         return least_split(n_src, v.jt, [&](int ns) {
             return rounds_cost(v.block, v.ipt, v.jt, force_occupancy(v), n_tgt, n_src, ns, sms);
         });
-    int64_t chunk = v.precision == kMixed ? (n_src <= 7000 ? 256 : n_src < 18000 ? 512 : 1024)
-                                          : v.block == 64 ? (n_src <= 4500 ? 128 : n_src <= 16384 ? 256 : 512)
-                                                          : (v.block * v.ipt == 256 ? 256 : 512);
     const int64_t tiles = (n_tgt + (int64_t)v.block * v.ipt - 1) / ((int64_t)v.block * v.ipt);
+    const int64_t limit = std::max<int64_t>(1, kMaxPartBytes / (24 * n_tgt));
+    // an SM's blocks in rounds of occ; fixed work of `fixed` sources, and a rate by the threads at work
+    auto rounds = [&](int ns, double fixed, double idle, int64_t occ) {
+        int64_t c;
+        int nse;
+        split_layout(n_src, v.jt, ns, &c, &nse);
+        const int64_t L = (tiles * nse + sms - 1) / sms, rem = L % occ;
+        auto slow = [&](int64_t k) { return 1.0 + idle / (double)(k * v.block); };
+        return ((double)c + fixed) * ((double)(L - rem) * slow(occ) + (rem ? (double)rem * slow(rem) : 0.0));
+    };
+    if (v.precision == kMixed && v.block >= 256)
+        return (int)std::min<int64_t>(limit, least_split(n_src, v.jt, [&](int ns) { return rounds(ns, 120.0, 64.0, 4); }));
+    int64_t chunk = v.precision == kMixed ? (n_src < 7200 ? 256 : 512)
+                    : v.block == 64       ? (n_src <= 4500 ? 128 : n_src <= 16384 ? 256 : 512)
+                                          : (v.block * v.ipt == 256 ? 256 : 512);
     while (chunk > v.jt && tiles * ((n_src + chunk - 1) / chunk) < 2 * sms) chunk /= 2;
     int64_t most = 64;
     // 2048 blocks of 256 threads fill the SMs several times over
@@ -355,8 +369,19 @@ int best_split(const ForceVariant& v, int64_t n_tgt, int64_t n_src, int sms) {
         chunk = std::max<int64_t>(chunk, (n_src / wide + v.jt / 2) / v.jt * v.jt);  // in whole passes
         most = (n_src + chunk - 1) / chunk;
     }
-    most = std::max<int64_t>(1, std::min(most, kMaxPartBytes / (24 * n_tgt)));
-    return (int)std::max<int64_t>(1, std::min(most, (n_src + chunk - 1) / chunk));
+    most = std::min(most, limit);
+    auto chunks = [&](int64_t c) { return (int)std::max<int64_t>(1, std::min(most, (n_src + c - 1) / c)); };
+    int best = chunks(chunk);
+    if (v.precision == kMixed) {
+        double bc = rounds(best, 60.0, 96.0, 6);
+        for (int64_t c : {256, 512, 768, 1024, 1536}) {
+            const double t = rounds(chunks(c), 60.0, 96.0, 6);
+            if (t >= 0.94 * bc) continue;
+            bc = t;
+            best = chunks(c);
+        }
+    }
+    return best;
 }
 
 // What the choice of a mixed variant weighs (heuristic_choice): a whole j tile of fixed work per
@@ -408,11 +433,11 @@ bool f64_shape(const ForceVariant& v, int64_t n_tgt, int64_t n_src, bool eps0) {
 }
 
 // Where a mixed twin is the faster one.  256 x 1 for 64 x 4: small systems, whose 64-thread blocks
-// leave each SM a few warps (N = 3000 15.7 against 21.4 us, N = 8192 47.0 / 47.4, N = 16,384 138 /
-// 134).  512 x 2 for 256 x 4: large ones (N = 262,144 26.7 against 27.0 ms, N = 65,536 1.71 / 1.72,
+// leave each SM a few warps (N = 3000 15.7 against 21.4 us, N = 9000 51.9 / 56.0, N = 11,200 77.0 / 78.1,
+// N = 12,000 82.2 / 80.5, N = 16,384 134.6 / 131.8).  512 x 2 for 256 x 4: large ones (N = 262,144 26.7 against 27.0 ms, N = 65,536 1.71 / 1.72,
 // N = 32,768 470 / 454 us).
 bool twin_faster(const ForceVariant& v, int64_t n_tgt, int64_t n_src) {
-    return v.block == 256 ? n_src <= 7000 : n_tgt >= 150000;
+    return v.block == 256 ? n_src < 11500 : n_tgt >= 150000;
 }
 
 // Untuned choice.  FP64: by n_tgt.  Mixed: the wave model over all variants, weighted by each

@@ -65,3 +65,41 @@ def test_fp64_without_softening(n):
         block, ipt, js = chosen(s, F64)
         assert block == (64 if n < 20000 else 256)
         assert -(-n // (block * ipt)) * js >= 2 * 148
+
+
+@pytest.mark.parametrize("n", [4999, 5000, 7001, 7199, 7200, 9000, 11499, 11500, 15001, 25000, 33000])
+@pytest.mark.parametrize("eps", [0.02, 0.0])
+def test_mixed_small_tiles(n, eps):
+    """Both sides of the lines of the 256-target tiles, and sizes at which one chunk length for all
+    left the SMs' last round nearly empty.  The rounds of an SM stay within a quarter of the work."""
+    p = gx.ics.two_disk_encounter(n - n // 2, n // 2, n, 0.02)
+    with gx.Session(n, gx.PhysicsParams(1.0, eps)) as s:
+        s.set_particles(p)
+        check(p, s, MIX, eps, 0, n)
+        block, ipt, js = chosen(s, MIX)
+        if block * ipt == 256 and eps > 0.0:
+            assert block == (256 if n < 11500 else 64)
+            blocks = -(-n // 256) * js
+            chunk = -(-(-(-n // js)) // 256) * 256
+            assert -(-blocks // 148) * chunk * 256 <= 1.3 * n * n / 148
+
+
+def test_twins_agree_on_both_sides_of_the_large_line():
+    """The variant chosen from 150,000 targets on gives the bits of the one chosen below."""
+    n = 150000
+    p = gx.ics.two_disk_encounter(n // 2, n // 2, 9, 0.02)
+    got = []
+    with gx.Session(n, gx.PhysicsParams(1.0, 0.02)) as s:
+        s.set_particles(p)
+        picked = s.get_config(MIX)
+        assert chosen(s, MIX)[:2] == (512, 2)
+        twin = next(v for v in range(64) if v != picked[0] and
+                    gx.describe_variant(MIX, v) == "mixed block=256 ipt=4 jt=512 f32x2-targets")
+        for v in (picked[0], twin):
+            s.set_config(MIX, v, picked[1])
+            s.compute_accelerations(MIX)
+            st = s.get_state()
+            got.append(np.stack([st[f] for f in ("ax", "ay", "az")]))
+    assert np.array_equal(got[0], got[1])
+    with gx.Session(n - 1, gx.PhysicsParams(1.0, 0.02)) as s:
+        assert chosen(s, MIX)[:2] != (512, 2)
