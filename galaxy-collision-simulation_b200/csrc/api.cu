@@ -310,6 +310,7 @@ int least_split(int64_t n_src, int jt, Cost cost) {
         int64_t chunk;
         int nse;
         split_layout(n_src, jt, ns, &chunk, &nse);
+        if (chunk == jt && nse < ns) break;  // no shorter chunks (small systems: a few us of every call)
         if (nse != ns) continue;
         const double c = cost(ns);
         if (c < bc * 0.995) {
@@ -470,16 +471,15 @@ Choice heuristic_choice(int dev, int precision, bool eps0, int64_t n_tgt, int64_
         if (cost < bc) {
             bc = cost;
             best.variant = ids[k];
-            best.nsplit = best_split(v, n_tgt, n_src, sms);
         }
     }
     for (int k = 0; k < c && precision == kMixed; ++k) {  // a twin in place of the chosen variant
         const ForceVariant& v = all[ids[k]];
         if (v.twin_of < 0 || v.twin_of != best.variant || !twin_faster(v, n_tgt, n_src)) continue;
         best.variant = ids[k];
-        best.nsplit = best_split(v, n_tgt, n_src, sms);
         break;
     }
+    best.nsplit = best_split(all[best.variant], n_tgt, n_src, sms);
     return best;
 }
 
