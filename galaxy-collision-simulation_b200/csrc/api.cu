@@ -2913,6 +2913,24 @@ void batch_free_items(gx_batch* b) {
 // 355 us and 810 / 814 / 765 us; whole tiles 5.49 and 14.0 ms, 1.34 and 1.73 ms.
 constexpr double kBatchItemsPerCta = 16.0;
 
+// Instances of one size whose whole tiles already fill the SMs evenly only lose by chunks: each
+// costs some 50 sources of fixed work.  True when, in mixed precision, the SMs' rounds of whole tiles
+// cost 3 % less than those of nsplit chunks (148 x 1536: 158 us whole, 168 in three chunks; 148 x
+// 3072 584, 633; 1000 x 1536 986, 1057; but 16 x 2000 74, 49 in four; 100 x 2000 202, 197).
+bool batch_tiles_whole(const gx_batch* b, const BatchVariant& v, int nsplit) {
+    const int64_t nb = b->off_h[1] - b->off_h[0], sms = sm_count(b->device), occ = batch_occupancy(v);
+    for (int i = 1; i < b->ni; ++i)
+        if (b->off_h[(size_t)i + 1] - b->off_h[(size_t)i] != nb) return false;
+    if (v.precision != kMixed || nsplit < 2) return false;
+    const int64_t tile = (int64_t)v.block * v.ipt, tiles = b->ni * ((nb + tile - 1) / tile);
+    auto cost = [&](int ns) {
+        const int64_t L = (tiles * ns + sms - 1) / sms, rem = L % occ;
+        auto slow = [&](int64_t c) { return 1.0 + 32.0 / (double)(c * v.block); };
+        return ((double)nb / ns + kCtaFixed) * ((double)(L - rem) * slow(occ) + (rem ? (double)rem * slow(rem) : 0.0));
+    };
+    return cost(1) < 0.97 * cost(nsplit);
+}
+
 int batch_build_items(gx_batch* b, int vid, int64_t part_limit = kMaxPartBytes) {
     if (b->items_variant == vid && b->items_d) return GX_OK;
     int cnt;
@@ -2938,6 +2956,10 @@ int batch_build_items(gx_batch* b, int vid, int64_t part_limit = kMaxPartBytes) 
             tickets += (nb + tile - 1) / tile;
         }
         if (part * (int64_t)sizeof(double) <= part_limit || want > b->n) break;
+    }
+    if (batch_tiles_whole(b, v, split[0].nsplit)) {
+        part = 0;
+        for (BatchSplit& s : split) split_layout(bodies(0), v.jt, 1, &s.j_chunk, &s.nsplit);
     }
     struct Item {
         int4 w;
