@@ -9,8 +9,9 @@
 namespace gx {
 
 // ---------------------------------------------------------------------------------------
-// FP64 reciprocal square root.  Seed: the hardware approximation rsqrt.approx.ftz.f64
-// (relative error below 2^-20 measured on B200).  One Householder step of order 2 on the
+// FP64 reciprocal square root.  Seed: the hardware approximation rsqrt.approx.ftz.f64 (relative
+// error below 2^-20: on B200 at most 2^-20.03 over every high word of two octaves, with all-zero and
+// all-one low words, and over 4096 mantissas of every exponent from -894 to 896).  One Householder step of order 2 on the
 // series (1 - e)^(-1/2) = 1 + e/2 + 3e^2/8 + O(e^3) with e = 1 - s*y^2 leaves a relative
 // error of about (5/16) e^3 < 2^-57, i.e. at the level of the final rounding.
 // 5 FP64 pipe operations after the MUFU seed.  s == 0 gives a non-finite result; callers
