@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(BLOCK) force_exact_serial_kernel(const ForceAr
      (const void*)&force_exact_kernel<T, W, U>, T}
 
 const ForceVariant kVariants[] = {
-    // mixed, targets packed (fastest at N = 2^20; the first entry is the untuned default)
+    // mixed, targets packed
     MIXTPU(256, 6, 512, 1, 8),
     MIXTPU(128, 8, 512, 1, 8),
     MIXTPU(128, 6, 512, 2, 16),

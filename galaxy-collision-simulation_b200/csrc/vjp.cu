@@ -7,7 +7,8 @@
 //     dL/dm_k = -G sum_j s^-3/2 (l_j . d),
 // which is a gather over j with the forward kernel's tiling: the sources stage
 // (x_j, m_j, l_j) -- 7 words -- in shared memory and each thread keeps IPT targets.
-// A self pair has d = 0 and A = 0, so it adds exactly zero when eps > 0.
+// A self pair has d = 0, and its A is zero up to the rounding of one product (m_k l_k - m_k l_k by a
+// fused multiply-add), so with eps > 0 it adds at most 2^-53 (mixed: 2^-24) of m_k |l_k| eps^-3.
 // Forms: FP64 (refined rsqrt) and mixed (FP32 pair arithmetic on offsets from a per-tile
 // FP64 origin, the sums of each source tile added up in FP64).  A j-split keeps systems of any
 // size spread over all SMs: grid and fused ordered reduction as in the forward kernels (force.cuh).
@@ -65,9 +66,9 @@ __device__ __forceinline__ void vjp_finish(const VjpArgs& a, int64_t tile) {
     }
 }
 
-// FP64: 34 FP64 operations per pair (3 differences, 3 FMA, 5 for the rsqrt, 3 for its powers, 3 for
+// FP64: 35 FP64 operations per pair (3 differences, 3 FMA, 5 for the rsqrt, 2 for its powers, 3 for
 // l_j . d, 6 for A, 3 for A . d, 3 for its factor, 7 FMA into the sums).  Bound by the FP64 pipe:
-// N = 16,384 632 us = 85% of the measured rate, against 720 us
+// N = 16,384 632 us = 87% of the measured rate, against 720 us
 // with 42 operations (l_k . d, products not fused into the sums).
 template <int BLOCK, int IPT, int JT, bool EPS0>
 __global__ void __launch_bounds__(BLOCK) vjp_f64_kernel(const VjpArgs a) {
