@@ -1981,13 +1981,14 @@ int fmm_plan_device(FmmPlan& P, int64_t n, const double* dx, const double* dy, c
     void* list_temp;
     GX_TRY(dev_array(hs, (int64_t)list_bytes, (char**)&list_temp));
     // Pools for the lists: a guess from the number of leaves and theta (a leaf of a two-disk system
-    // has 300 to 600 far nodes and 80 to 150 near leaves at theta 0.6, growing as theta falls), at
-    // most kListPoolBytes each; when it is too small, the totals tell what is needed and the lists
+    // has 300 to 600 far nodes and 80 to 150 near leaves at theta 0.6, growing as theta falls; leaves of
+    // one body in a filled cube have several thousand, which the empty leaves' share covers), at most
+    // kListPoolBytes each; when it is too small, the totals tell what is needed and the lists
     // are made again.  So are they when the guess does not fit in memory: pools of one entry then
     // count what the lists really need.
     constexpr int64_t kListPoolBytes = 2ll << 30;
     const double wide = std::min(8.0, std::max(1.0, 0.36 / (la.theta * la.theta)));
-    const int64_t leaf_bound = std::min<int64_t>(P.n_nodes - P.n_nodes / 8 + 1, n);  // leaves with bodies
+    const int64_t leaf_bound = P.n_nodes - P.n_nodes / 8 + 1;  // empty leaves included
     la.far_cap = std::min<int64_t>((int64_t)(2.0 * wide * (double)leaf_bound) + 64,
                                    kListPoolBytes / (int64_t)(kM2PChunk * sizeof(int32_t)));
     la.near_cap = std::min<int64_t>((int64_t)(256.0 * wide * (double)leaf_bound) + 4096,
