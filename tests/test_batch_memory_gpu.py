@@ -30,6 +30,7 @@ def evaluate(sizes):
 def test_the_next_batch_reuses_the_memory():
     sizes = [1024 + 512 * (k % 20) for k in range(100)]
     first, acc = evaluate(sizes)
+    first.diagnostics()
     first.close()
     left = free_bytes()
     for _ in range(3):
